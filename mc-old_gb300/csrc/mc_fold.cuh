@@ -1,0 +1,215 @@
+// mc_fold.cuh -- the ordered history fold of FP64 replay, many histories at once.
+//
+// Estimator::end_history (Estimator.cpp:339-346) adds one history after the
+// other to a running FP64 sum, and replay must give that sum's bits.  Taken
+// literally it is one serial chain per bin: every addition waits for the one
+// before it (64 cycles on this chip, and the load in front of it), while all
+// but one thread per bin idle.  It is not serial arithmetic, though.  While
+// the running sum s keeps its binade, s = k u with u its unit in the last
+// place and 2^52 <= |k| < 2^53, and adding v rounds v / u to the nearest
+// integer independently of s, except that a tie goes to the side that leaves
+// k even.  So in a fixed binade one addition is the map
+//     k -> k + inc[k & 1]
+// given by two integers (equal unless v is a tie), and such maps compose
+// associatively: (f then g)[p] = f[p] + g[(p + f[p]) & 1].  A block scans
+// them over kFoldThreads x kFoldValues histories at a time in integer
+// arithmetic.  Where the sum could leave its binade (about once per doubling
+// of a sum of positive terms), or where it is zero, subnormal or not finite,
+// the values are added one by one in FP64 (one thread's, or a longer run of
+// them where a signed sum keeps wandering about zero), and the scan goes on
+// behind them.  Every result bit is the serial chain's.
+//
+// Bound and measure (GB300, 500,000 histories x 19 bins, replay of the
+// 16-layer one-group slab): the serial chain, one thread per bin, took
+// 61.5 ms (123 ns per history: one addition's latency for each of sum and
+// sum of squares plus one load round trip per 8 histories); this kernel
+// 1.13 ms (the column reads bound it).
+#pragma once
+
+#include <cstdint>
+
+#include "mc_math.cuh"
+
+namespace mc {
+
+constexpr int kFoldThreads = 512;
+constexpr int kFoldValues = 8;    // consecutive histories per thread and step
+// after kFoldStreak failing steps in a row, the values of kFoldRun threads
+// are added serially at once: a step that places 8 histories costs about as
+// much as 40 serial additions
+constexpr int kFoldStreak = 8;
+constexpr int kFoldRun = 64;
+
+// inc[0], inc[1]: what the histories so far add to k if it starts even / odd
+struct FoldMap {
+    long long a0, a1;
+};
+
+__device__ __forceinline__ FoldMap fold_then(const FoldMap &f, const FoldMap &g)
+{
+    FoldMap r;
+    r.a0 = f.a0 + ((f.a0 & 1) ? g.a1 : g.a0);
+    r.a1 = f.a1 + ((f.a1 & 1) ? g.a0 : g.a1);
+    return r;
+}
+
+// One chain: block (bin, which), which = 0 the sum of the column's values,
+// 1 the sum of their squares.  hist is [n][nb].
+__global__ void __launch_bounds__(kFoldThreads) k_fold_ordered(const double *__restrict__ hist, uint32_t n,
+                                                               long long nb, double *__restrict__ sum,
+                                                               double *__restrict__ sq)
+{
+    __shared__ FoldMap s_warp[kFoldThreads / 32];
+    __shared__ double s_run;      // the running sum before the current step
+    __shared__ int s_fail;        // first thread whose histories need the serial chain
+    __shared__ FoldMap s_total;
+    __shared__ double s_v[kFoldRun * kFoldValues];
+    const long long bin = blockIdx.x;
+    const bool squares = blockIdx.y != 0;
+    double *dst = (squares ? sq : sum) + bin;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    constexpr uint32_t kStep = (uint32_t)kFoldThreads * kFoldValues;
+    const double *col = hist + bin;
+    double nxt[kFoldValues];
+    auto fetch = [&](uint64_t pos) {
+#pragma unroll
+        for (int j = 0; j < kFoldValues; ++j) {
+            const uint64_t h = pos + (uint64_t)t * kFoldValues + j;
+            nxt[j] = h < n ? col[h * (uint64_t)nb] : 0.0;
+        }
+    };
+    if (t == 0) s_run = *dst;
+    uint64_t pos = 0;
+    int streak = 0;
+    fetch(0);
+    while (pos < n) {
+        double v[kFoldValues];
+        bool any = false;
+#pragma unroll
+        for (int j = 0; j < kFoldValues; ++j) {
+            v[j] = nxt[j];
+            any = any || (dbits(v[j]) << 1) != 0;   // integer test: an FP64 compare costs 19 SM cycles a warp
+        }
+        fetch(pos + kStep);       // the next step's histories, if this one goes through
+        if (!__syncthreads_or(any)) {   // adding zeros changes nothing
+            pos += kStep;
+            continue;
+        }
+        if (squares) {
+#pragma unroll
+            for (int j = 0; j < kFoldValues; ++j) v[j] = v[j] * v[j];
+        }
+        const uint64_t sb = dbits(s_run);
+        const int es = (int)((sb >> 52) & 0x7FF);
+        const bool scannable = es > 0 && es < 0x7FF;
+        const long long k = (long long)((sb & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull);
+        // this thread's map, and a bound on how far k moves within it
+        FoldMap f{0, 0};
+        unsigned long long reach = 0;
+        bool bad = false;
+        if (any) {
+#pragma unroll
+            for (int j = 0; j < kFoldValues; ++j) {
+                const uint64_t b = dbits(v[j]);
+                if ((b << 1) == 0) continue;
+                const int ev = (int)((b >> 52) & 0x7FF);
+                uint64_t m = b & 0x000FFFFFFFFFFFFFull;
+                if (ev) m |= 0x0010000000000000ull;
+                const int sh = es - (ev ? ev : 1);      // v / u = m 2^-sh
+                if (!scannable || ev == 0x7FF || sh < 0) { bad = true; continue; }
+                if (sh > 54) continue;                  // below a quarter unit
+                const uint64_t q = m >> sh;
+                const uint64_t rem = m - (q << sh);
+                const uint64_t half = sh > 0 ? 1ull << (sh - 1) : 1ull;
+                uint64_t u0 = rem > half ? 1u : 0u, u1 = u0;
+                if (rem == half) {                      // a tie: to even
+                    u0 = (uint64_t)(f.a0 + (long long)q) & 1u;
+                    u1 = (uint64_t)(f.a1 + (long long)q + 1) & 1u;
+                }
+                reach += q + 1;
+                if ((b ^ sb) >> 63) {
+                    f.a0 -= (long long)(q + u0);
+                    f.a1 -= (long long)(q + u1);
+                } else {
+                    f.a0 += (long long)(q + u0);
+                    f.a1 += (long long)(q + u1);
+                }
+            }
+        }
+        // exclusive scan of the maps over the block
+        FoldMap inc = f;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            FoldMap p;
+            p.a0 = __shfl_up_sync(0xffffffffu, inc.a0, o);
+            p.a1 = __shfl_up_sync(0xffffffffu, inc.a1, o);
+            if (lane >= o) inc = fold_then(p, inc);
+        }
+        FoldMap before;
+        before.a0 = __shfl_up_sync(0xffffffffu, inc.a0, 1);
+        before.a1 = __shfl_up_sync(0xffffffffu, inc.a1, 1);
+        if (lane == 0) before = FoldMap{0, 0};
+        if (lane == 31) s_warp[warp] = inc;
+        if (t == 0) s_fail = kFoldThreads;
+        __syncthreads();
+        if (warp == 0) {
+            FoldMap w = lane < kFoldThreads / 32 ? s_warp[lane] : FoldMap{0, 0};
+#pragma unroll
+            for (int o = 1; o < kFoldThreads / 32; o <<= 1) {
+                FoldMap p;
+                p.a0 = __shfl_up_sync(0xffffffffu, w.a0, o);
+                p.a1 = __shfl_up_sync(0xffffffffu, w.a1, o);
+                if (lane >= o) w = fold_then(p, w);
+            }
+            if (lane == kFoldThreads / 32 - 1) s_total = w;
+            FoldMap x;
+            x.a0 = __shfl_up_sync(0xffffffffu, w.a0, 1);
+            x.a1 = __shfl_up_sync(0xffffffffu, w.a1, 1);
+            if (lane == 0) x = FoldMap{0, 0};
+            if (lane < kFoldThreads / 32) s_warp[lane] = x;
+        }
+        __syncthreads();
+        before = fold_then(s_warp[warp], before);
+        // k before this thread's histories; it stays in the binade through
+        // them if it cannot reach either end.  (Threads behind the first
+        // failing one may see wrapped values; they are taken again.)
+        const long long k0 = k + ((k & 1) ? before.a1 : before.a0);
+        if (any && (bad || k0 <= (1ll << 52) || k0 >= (1ll << 53) || reach >= (1ull << 53) ||
+                    (unsigned long long)(k0 - (1ll << 52)) <= reach || (unsigned long long)((1ll << 53) - k0) <= reach))
+            atomicMin(&s_fail, t);
+        __syncthreads();
+        const int fail = s_fail;
+        const uint64_t keep = sb & 0xFFF0000000000000ull;   // sign and exponent of the running sum
+        if (fail == kFoldThreads) {
+            if (t == 0) {
+                const long long kn = k + ((k & 1) ? s_total.a1 : s_total.a0);
+                s_run = scannable ? dfrom(keep | ((uint64_t)kn & 0x000FFFFFFFFFFFFFull)) : s_run;
+            }
+            pos += kStep;
+            streak = 0;
+        } else {
+            const int run = min(++streak >= kFoldStreak ? kFoldRun : 1, kFoldThreads - fail);
+            if (t > fail && t < fail + run) {
+#pragma unroll
+                for (int j = 0; j < kFoldValues; ++j) s_v[(t - fail) * kFoldValues + j] = v[j];
+            }
+            if (run > 1) __syncthreads();
+            if (t == fail) {
+                double s = scannable ? dfrom(keep | ((uint64_t)k0 & 0x000FFFFFFFFFFFFFull)) : s_run;
+#pragma unroll
+                for (int j = 0; j < kFoldValues; ++j) s += v[j];
+                for (int j = kFoldValues; j < run * kFoldValues; ++j) {
+                    const double x = s_v[j];
+                    if ((dbits(x) << 1) != 0) s += x;
+                }
+                s_run = s;
+            }
+            pos += (uint64_t)(fail + run) * kFoldValues;
+            fetch(pos);
+        }
+        __syncthreads();
+    }
+    if (t == 0) *dst = s_run;
+}
+
+}  // namespace mc

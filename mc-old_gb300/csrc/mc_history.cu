@@ -21,6 +21,7 @@
 #include <cfloat>
 
 #include "mc_device.h"
+#include "mc_fold.cuh"
 #include "mc_math.cuh"
 
 namespace mc {
@@ -818,30 +819,6 @@ __global__ void __launch_bounds__(128) k_history_fp64(const DevTables T, const H
         if (C.cnt[i]) atomicAdd(A.counters + i, C.cnt[i]);
 }
 
-// one thread per bin, histories in order (Estimator.cpp:339-346)
-__global__ void k_fold_ordered(const double *__restrict__ hist, uint32_t n, long long nb,
-                               double *__restrict__ sum, double *__restrict__ sq)
-{
-    const long long b = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= nb) return;
-    double s = sum[b], q = sq[b];
-    uint32_t h = 0;
-    for (; h + 8 <= n; h += 8) {
-        double v[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) v[k] = hist[(size_t)(h + k) * nb + b];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) { s += v[k]; q += v[k] * v[k]; }
-    }
-    for (; h < n; ++h) {
-        const double v = hist[(size_t)h * nb + b];
-        s += v;
-        q += v * v;
-    }
-    sum[b] = s;
-    sq[b] = q;
-}
-
 // block-tree fold over a tile of histories per block, FP64 atomics per bin
 __global__ void k_fold_tree(const double *__restrict__ hist, uint32_t n, long long nb,
                             double *__restrict__ sum, double *__restrict__ sq, uint32_t rows_per_block)
@@ -897,9 +874,7 @@ cudaError_t launch_fold(const double *hist, uint32_t n, long long nb, double *su
 {
     if (nb <= 0 || n == 0) return cudaSuccess;
     if (ordered) {
-        const int block = 128;
-        const int grid = (int)((nb + block - 1) / block);
-        k_fold_ordered<<<grid, block, 0, st>>>(hist, n, nb, sum, sq);
+        k_fold_ordered<<<dim3((unsigned)nb, 2), kFoldThreads, 0, st>>>(hist, n, nb, sum, sq);
     } else {
         const int block = 128;
         const uint32_t rows = 512;
