@@ -52,15 +52,16 @@ struct HistoryArgs {
     uint64_t first;          // first history of the chunk
     uint32_t n;              // histories in the chunk
     uint64_t seed;
-    double *hist;            // [n][n_bins] per-history totals (scratch)
+    double *hist;            // [columns][hist_ld] per-history totals (scratch, zeroed by the launcher)
+    uint64_t hist_ld;        // histories a column has room for (hist_rows(n) or more)
     void *stack;             // [threads][stack_depth] split particles (scratch)
     uint32_t stack_depth;
     unsigned long long *counters;   // [kNumCounters]
     unsigned long long *digest;     // [n] or nullptr
     int *status;
     unsigned int *next;      // work counter (zeroed by the launcher)
-    // likelihood-ratio differentiation (n_params > 0): each history row is
-    // followed by n_bins x n_params derivative contributions; split copies
+    // likelihood-ratio differentiation (n_params > 0): the n_bins tally
+    // columns are followed by n_bins x n_cols derivative columns; split copies
     // keep their score-function weights in lr_stack
     int n_params = 0;
     double *lr_stack = nullptr;   // [threads][stack_depth][n_params]
@@ -79,19 +80,25 @@ constexpr int kMaxLrParams = 64;   // (Sigma_s, Sigma_a) for up to 32 materials
 cudaError_t launch_history_fp64(const DevTables &T, const HistoryArgs &A, bool replay,
                                 int grid, int block, cudaStream_t st);
 
-// Folds a chunk's per-history totals into sum / sq.  ordered = history order
-// (bit-exact with the reference's end_history loop); otherwise a parallel
-// tree fold.
-cudaError_t launch_fold(const double *hist, uint32_t n, long long n_bins, double *sum, double *sq,
-                        bool ordered, cudaStream_t st);
+// Per-history totals are kept column by column, [column][ld]: the folds read
+// a column's histories as contiguous vectors, and neighbouring histories that
+// score the same bin share sectors.  Room of n histories in a column:
+inline uint64_t hist_rows(uint64_t n) { return (n + 7) & ~(uint64_t)7; }
+
+// Folds a chunk's per-history totals into sum / sq in history order (the bits
+// of the reference's end_history loop).
+cudaError_t launch_fold_ordered(const double *hist, uint32_t n, uint64_t ld, long long n_cols, double *sum,
+                                double *sq, cudaStream_t st);
 
 // Exact per-bin sums (mc_exact.cu): kExactLimbs signed 64-bit limbs per
 // value, value = sum_j limb[j] * 2^(32 j - 1074); [n_bins][2][kExactLimbs]
 // (sum of history totals, sum of their squares).
 constexpr int kExactLimbs = 68;
 
-// Adds a chunk's per-history totals and their squares to ex exactly.
-cudaError_t launch_fold_exact(const double *hist, uint32_t n, long long n_bins, long long *ex, cudaStream_t st);
+// Adds a chunk's per-history totals and their squares to ex exactly, and to
+// sum / sq in a parallel tree's order where those are given (plain mode).
+cudaError_t launch_fold_exact(const double *hist, uint32_t n, uint64_t ld, long long n_bins, long long *ex,
+                              double *sum, double *sq, cudaStream_t st);
 
 // Propagates the carries of every exact value of ex (one representation per
 // value: limbs 0..kExactLimbs-2 in [0, 2^32), the last one signed).

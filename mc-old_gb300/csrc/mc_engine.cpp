@@ -263,7 +263,8 @@ mc_status run_fp64(const Tables &t, DeviceProblem &d, uint64_t first, uint64_t n
     chunk = std::max<uint64_t>(1, std::min<uint64_t>(chunk, 1u << 22));
     chunk = std::min<uint64_t>(chunk, n);
     const uint64_t threads = (uint64_t)grid * block;
-    if (!devbuf_reserve(d.hist, (size_t)chunk * nb * sizeof(double)) ||
+    const uint64_t ld = hist_rows(chunk);
+    if (!devbuf_reserve(d.hist, (size_t)ld * nb * sizeof(double)) ||
         !devbuf_reserve(d.stack, (size_t)threads * depth * fp64_particle_bytes()) ||
         !devbuf_reserve(d.misc, 256 + kNumCounters * sizeof(unsigned long long) + 64) ||
         (want_digest && !devbuf_reserve(d.digest, (size_t)chunk * sizeof(uint64_t)))) {
@@ -284,6 +285,7 @@ mc_status run_fp64(const Tables &t, DeviceProblem &d, uint64_t first, uint64_t n
 
     float t_transport = 0.f, t_fold = 0.f;
     uint32_t launches = 0;
+    uint64_t unnormalized = 0;   // histories added to the exact sums since their carries were propagated
     // the exact sums stay valid only if this run completes
     const bool exact_was_valid = d.exact_valid;
     d.exact_valid = false;
@@ -295,6 +297,7 @@ mc_status run_fp64(const Tables &t, DeviceProblem &d, uint64_t first, uint64_t n
         A.n = cn;
         A.seed = seed;
         A.hist = static_cast<double *>(d.hist.ptr);
+        A.hist_ld = ld;
         A.stack = d.stack.ptr;
         A.stack_depth = depth;
         if (tune && tune->max_events) A.max_events = tune->max_events;
@@ -309,13 +312,24 @@ mc_status run_fp64(const Tables &t, DeviceProblem &d, uint64_t first, uint64_t n
             return MC_ERR_CUDA;
         }
         cudaEventRecord(d.ev[2], d.stream);
-        if ((e = launch_fold(A.hist, cn, d.dt.n_bins, d.d_sum, d.d_sq, replay, d.stream)) != cudaSuccess ||
-            (e = launch_fold_exact(A.hist, cn, d.dt.n_bins, d.d_exact, d.stream)) != cudaSuccess) {
+        if ((replay && (e = launch_fold_ordered(A.hist, cn, ld, d.dt.n_bins, d.d_sum, d.d_sq, d.stream)) != cudaSuccess) ||
+            (e = launch_fold_exact(A.hist, cn, ld, d.dt.n_bins, d.d_exact, replay ? nullptr : d.d_sum,
+                                   replay ? nullptr : d.d_sq, d.stream)) != cudaSuccess) {
             err = cuda_msg(e, "fold kernel launch");
             return MC_ERR_CUDA;
         }
+        launches += replay ? 3 : 2;
+        // a limb absorbs 2^31 additions of 32-bit digits
+        unnormalized += cn;
+        if (unnormalized >= (1ull << 30)) {
+            if ((e = launch_exact_normalize(d.d_exact, d.dt.n_bins, d.stream)) != cudaSuccess) {
+                err = cuda_msg(e, "exact sums");
+                return MC_ERR_CUDA;
+            }
+            unnormalized = 0;
+            ++launches;
+        }
         cudaEventRecord(d.ev[3], d.stream);
-        launches += 3;
         if (want_digest) {
             cudaMemcpyAsync(d.digests.data() + c0, A.digest, cn * sizeof(uint64_t), cudaMemcpyDeviceToHost, d.stream);
         }

@@ -23,7 +23,8 @@
 // 16-layer one-group slab): the serial chain, one thread per bin, took
 // 61.5 ms (123 ns per history: one addition's latency for each of sum and
 // sum of squares plus one load round trip per 8 histories); this kernel
-// 1.13 ms (the column reads bound it).
+// 0.86 ms (barriers and shuffles of the scan between steps).  A column is
+// contiguous, so a thread's 8 histories are four 16-byte loads.
 #pragma once
 
 #include <cstdint>
@@ -53,10 +54,37 @@ __device__ __forceinline__ FoldMap fold_then(const FoldMap &f, const FoldMap &g)
     return r;
 }
 
+// A thread's map where some terms are ties (rare: the plain sum of rounded
+// terms serves otherwise).  es, sb: exponent field and bits of the sum.
+__device__ __noinline__ FoldMap fold_map(const double (&v)[kFoldValues], int es, uint64_t sb)
+{
+    FoldMap f{0, 0};
+    for (int j = 0; j < kFoldValues; ++j) {
+        const uint64_t b = dbits(v[j]);
+        if ((b << 1) == 0) continue;
+        const int ev = (int)((b >> 52) & 0x7FF);
+        const uint64_t m = (b & 0x000FFFFFFFFFFFFFull) | (ev ? 0x0010000000000000ull : 0ull);
+        const int sh = es - max(ev, 1);
+        if (sh < 0 || sh > 63) continue;
+        const uint64_t rem = sh > 0 ? m << (64 - sh) : 0ull;
+        const uint64_t q = m >> sh;
+        uint64_t u0 = rem >> 63, u1 = u0;
+        if (rem == 0x8000000000000000ull) {             // to even
+            u0 = (uint64_t)(f.a0 + (long long)q) & 1u;
+            u1 = (uint64_t)(f.a1 + (long long)q + 1) & 1u;
+        }
+        const bool neg = (b ^ sb) >> 63;
+        f.a0 += neg ? -(long long)(q + u0) : (long long)(q + u0);
+        f.a1 += neg ? -(long long)(q + u1) : (long long)(q + u1);
+    }
+    return f;
+}
+
 // One chain: block (bin, which), which = 0 the sum of the column's values,
-// 1 the sum of their squares.  hist is [n][nb].
+// 1 the sum of their squares.  hist is [bins][ld], ld a multiple of 8 and at
+// least n, zero from n on.
 __global__ void __launch_bounds__(kFoldThreads) k_fold_ordered(const double *__restrict__ hist, uint32_t n,
-                                                               long long nb, double *__restrict__ sum,
+                                                               uint64_t ld, double *__restrict__ sum,
                                                                double *__restrict__ sq)
 {
     __shared__ FoldMap s_warp[kFoldThreads / 32];
@@ -69,13 +97,16 @@ __global__ void __launch_bounds__(kFoldThreads) k_fold_ordered(const double *__r
     double *dst = (squares ? sq : sum) + bin;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     constexpr uint32_t kStep = (uint32_t)kFoldThreads * kFoldValues;
-    const double *col = hist + bin;
+    const double *col = hist + (uint64_t)bin * ld;
     double nxt[kFoldValues];
     auto fetch = [&](uint64_t pos) {
+        const uint64_t h = pos + (uint64_t)t * kFoldValues;   // a multiple of 8, as ld
+        const double2 *p = reinterpret_cast<const double2 *>(col + h);
 #pragma unroll
-        for (int j = 0; j < kFoldValues; ++j) {
-            const uint64_t h = pos + (uint64_t)t * kFoldValues + j;
-            nxt[j] = h < n ? col[h * (uint64_t)nb] : 0.0;
+        for (int j = 0; j < kFoldValues / 2; ++j) {
+            const double2 x = h < n ? p[j] : double2{0.0, 0.0};
+            nxt[2 * j] = x.x;
+            nxt[2 * j + 1] = x.y;
         }
     };
     if (t == 0) s_run = *dst;
@@ -103,77 +134,73 @@ __global__ void __launch_bounds__(kFoldThreads) k_fold_ordered(const double *__r
         const int es = (int)((sb >> 52) & 0x7FF);
         const bool scannable = es > 0 && es < 0x7FF;
         const long long k = (long long)((sb & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull);
-        // this thread's map, and a bound on how far k moves within it
-        FoldMap f{0, 0};
+        // this thread's map, and a bound on how far k moves within it: without
+        // ties both entries are the sum of the rounded terms
+        long long move = 0;
         unsigned long long reach = 0;
-        bool bad = false;
+        bool bad = false, tie = false;
         if (any) {
 #pragma unroll
             for (int j = 0; j < kFoldValues; ++j) {
                 const uint64_t b = dbits(v[j]);
-                if ((b << 1) == 0) continue;
                 const int ev = (int)((b >> 52) & 0x7FF);
-                uint64_t m = b & 0x000FFFFFFFFFFFFFull;
-                if (ev) m |= 0x0010000000000000ull;
-                const int sh = es - (ev ? ev : 1);      // v / u = m 2^-sh
-                if (!scannable || ev == 0x7FF || sh < 0) { bad = true; continue; }
-                if (sh > 54) continue;                  // below a quarter unit
-                const uint64_t q = m >> sh;
-                const uint64_t rem = m - (q << sh);
-                const uint64_t half = sh > 0 ? 1ull << (sh - 1) : 1ull;
-                uint64_t u0 = rem > half ? 1u : 0u, u1 = u0;
-                if (rem == half) {                      // a tie: to even
-                    u0 = (uint64_t)(f.a0 + (long long)q) & 1u;
-                    u1 = (uint64_t)(f.a1 + (long long)q + 1) & 1u;
-                }
+                const uint64_t m = (b & 0x000FFFFFFFFFFFFFull) | (ev ? 0x0010000000000000ull : 0ull);
+                const int sh = es - max(ev, 1);         // v / u = m 2^-sh
+                bad = bad || ((b << 1) != 0 && (ev == 0x7FF || sh < 0));
+                const uint64_t rem = (sh > 0 && sh < 64) ? m << (64 - sh) : 0ull;   // the bits below the unit
+                const uint64_t q = ((sh >= 0 && sh < 64) ? m >> sh : 0ull) + (rem >> 63);
+                tie = tie || rem == 0x8000000000000000ull;
                 reach += q + 1;
-                if ((b ^ sb) >> 63) {
-                    f.a0 -= (long long)(q + u0);
-                    f.a1 -= (long long)(q + u1);
-                } else {
-                    f.a0 += (long long)(q + u0);
-                    f.a1 += (long long)(q + u1);
-                }
+                move += ((b ^ sb) >> 63) ? -(long long)q : (long long)q;
             }
+            bad = bad || !scannable;
         }
-        // exclusive scan of the maps over the block
-        FoldMap inc = f;
+        // k before this thread's histories (k0), and the block's total
+        long long k0;
+        if (!__syncthreads_or(tie)) {
+            long long inc = move;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            FoldMap p;
-            p.a0 = __shfl_up_sync(0xffffffffu, inc.a0, o);
-            p.a1 = __shfl_up_sync(0xffffffffu, inc.a1, o);
-            if (lane >= o) inc = fold_then(p, inc);
-        }
-        FoldMap before;
-        before.a0 = __shfl_up_sync(0xffffffffu, inc.a0, 1);
-        before.a1 = __shfl_up_sync(0xffffffffu, inc.a1, 1);
-        if (lane == 0) before = FoldMap{0, 0};
-        if (lane == 31) s_warp[warp] = inc;
-        if (t == 0) s_fail = kFoldThreads;
-        __syncthreads();
-        if (warp == 0) {
-            FoldMap w = lane < kFoldThreads / 32 ? s_warp[lane] : FoldMap{0, 0};
+            for (int o = 1; o < 32; o <<= 1) {
+                const long long p = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o) inc += p;
+            }
+            if (lane == 31) s_warp[warp].a0 = inc;
+            if (t == 0) s_fail = kFoldThreads;
+            __syncthreads();
+            long long w = 0, total = 0;
 #pragma unroll
-            for (int o = 1; o < kFoldThreads / 32; o <<= 1) {
+            for (int i = 0; i < kFoldThreads / 32; ++i) {
+                const long long x = s_warp[i].a0;
+                if (i < warp) w += x;
+                total += x;
+            }
+            k0 = k + w + inc - move;
+            if (t == 0) s_total = FoldMap{total, total};
+        } else {
+            FoldMap inc = any && !bad ? fold_map(v, es, sb) : FoldMap{0, 0};
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
                 FoldMap p;
-                p.a0 = __shfl_up_sync(0xffffffffu, w.a0, o);
-                p.a1 = __shfl_up_sync(0xffffffffu, w.a1, o);
-                if (lane >= o) w = fold_then(p, w);
+                p.a0 = __shfl_up_sync(0xffffffffu, inc.a0, o);
+                p.a1 = __shfl_up_sync(0xffffffffu, inc.a1, o);
+                if (lane >= o) inc = fold_then(p, inc);
             }
-            if (lane == kFoldThreads / 32 - 1) s_total = w;
-            FoldMap x;
-            x.a0 = __shfl_up_sync(0xffffffffu, w.a0, 1);
-            x.a1 = __shfl_up_sync(0xffffffffu, w.a1, 1);
-            if (lane == 0) x = FoldMap{0, 0};
-            if (lane < kFoldThreads / 32) s_warp[lane] = x;
+            FoldMap before;
+            before.a0 = __shfl_up_sync(0xffffffffu, inc.a0, 1);
+            before.a1 = __shfl_up_sync(0xffffffffu, inc.a1, 1);
+            if (lane == 0) before = FoldMap{0, 0};
+            if (lane == 31) s_warp[warp] = inc;
+            if (t == 0) s_fail = kFoldThreads;
+            __syncthreads();
+            FoldMap w{0, 0};
+            for (int i = 0; i < warp; ++i) w = fold_then(w, s_warp[i]);
+            if (warp == kFoldThreads / 32 - 1 && lane == 0) s_total = fold_then(w, s_warp[warp]);
+            before = fold_then(w, before);
+            k0 = k + ((k & 1) ? before.a1 : before.a0);
         }
-        __syncthreads();
-        before = fold_then(s_warp[warp], before);
-        // k before this thread's histories; it stays in the binade through
-        // them if it cannot reach either end.  (Threads behind the first
-        // failing one may see wrapped values; they are taken again.)
-        const long long k0 = k + ((k & 1) ? before.a1 : before.a0);
+        // k stays in the binade through this thread's histories if it cannot
+        // reach either end.  (Threads behind the first failing one may see
+        // wrapped values; they are taken again.)
         if (any && (bad || k0 <= (1ll << 52) || k0 >= (1ll << 53) || reach >= (1ull << 53) ||
                     (unsigned long long)(k0 - (1ll << 52)) <= reach || (unsigned long long)((1ll << 53) - k0) <= reach))
             atomicMin(&s_fail, t);

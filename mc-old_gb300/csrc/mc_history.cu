@@ -64,7 +64,8 @@ template <> struct Fn<false> {
 struct Ctx {
     const DevTables *T;
     Stream rng;
-    double *hist;
+    double *hist;          // the history's place in the first column
+    size_t ld;             // histories per column
     unsigned long long cnt[kNumCounters];
     unsigned long long digest;
     PartD *stack;
@@ -391,7 +392,7 @@ __device__ void estimator_score(Ctx &C, int e, const PartD &p, double l_in)
     const int f0 = T.est_filt_off[e], nf = T.est_filt_off[e + 1] - f0;
     const int s0 = T.est_score_off[e], ns = T.est_score_off[e + 1] - s0;
     const double *fac = T.est_factor + T.est_factor_off[e];
-    double *hist = C.hist + T.est_bin_off[e];
+    double *hist = C.hist + (size_t)T.est_bin_off[e] * C.ld;
     if (!(fabs(l_in) <= DBL_MAX)) {   // non-finite track: the loop below would never advance
         C.status = DS_NAN;
         return;
@@ -417,23 +418,23 @@ __device__ void estimator_score(Ctx &C, int e, const PartD &p, double l_in)
         for (int i = 0; i < nf; ++i) idx1 += (int)(il[off[i] + idx[i]].bin * fac[i + 1]);
         for (int s = 0; s < ns; ++s) {
             const double v = score_value(C, s0 + s, p, l);
-            hist[idx1] += v;
+            hist[(size_t)idx1 * C.ld] += v;
             C.cnt[C_TALLY]++;
             if constexpr (L) {
                 // d(contribution)/d(param_k) = v S_k + direct dependence
-                double *dh = C.hist + C.nb + (size_t)(T.est_bin_off[e] + idx1) * C.Kc;
+                double *dh = C.hist + (C.nb + (size_t)(T.est_bin_off[e] + idx1) * C.Kc) * C.ld;
                 double ds, da;
                 direct_terms(C, s0 + s, T.cell_mat[p.cell], p, v, ds, da);
                 const int m = T.cell_mat[p.cell];
                 for (int mm = 0; mm < C.K / 2; ++mm) {
                     double d_s = v * C.S[2 * mm], d_a = v * C.S[2 * mm + 1];
                     if (mm == m) { d_s += ds; d_a += da; }
-                    dh[2 * mm] += d_s;
-                    dh[2 * mm + 1] += d_a;
+                    dh[(size_t)(2 * mm) * C.ld] += d_s;
+                    dh[(size_t)(2 * mm + 1) * C.ld] += d_a;
                     // rho d/drho = Sigma_s d/dSigma_s + Sigma_a d/dSigma_a, per history
                     if (C.Kc > C.K) {
                         const int i = mm * T.mg_groups;
-                        dh[C.K + mm] += T.mg_scat_tot[i] * d_s + T.mg_capture[i] * d_a;
+                        dh[(size_t)(C.K + mm) * C.ld] += T.mg_scat_tot[i] * d_s + T.mg_capture[i] * d_a;
                     }
                 }
             }
@@ -775,19 +776,17 @@ __global__ void __launch_bounds__(128) k_history_fp64(const DevTables T, const H
     C.stack = reinterpret_cast<PartD *>(A.stack) + tid * A.stack_depth;
     C.status = DS_OK;
     for (int i = 0; i < kNumCounters; ++i) C.cnt[i] = 0;
-    const long long nb = T.n_bins;
-    C.nb = nb;
+    C.nb = T.n_bins;
+    C.ld = A.hist_ld;
     C.K = L ? A.n_params : 0;
     C.Kc = L ? (A.n_cols > A.n_params ? A.n_cols : A.n_params) : 0;
     C.lr_stack = L ? A.lr_stack + tid * A.stack_depth * (size_t)A.n_params : nullptr;
-    const long long row = L ? nb * (1 + (long long)C.Kc) : nb;
     const bool digests = A.digest != nullptr;
     for (;;) {
         const unsigned hl = atomicAdd(A.next, 1u);
         if (hl >= A.n) break;
         const uint64_t h = A.first + hl;
-        C.hist = A.hist + (size_t)hl * row;
-        for (long long b = 0; b < row; ++b) C.hist[b] = 0.0;
+        C.hist = A.hist + hl;
         C.rng.init(A.seed, h);
         C.digest = 0xCBF29CE484222325ULL;
         PartD p;
@@ -819,27 +818,6 @@ __global__ void __launch_bounds__(128) k_history_fp64(const DevTables T, const H
         if (C.cnt[i]) atomicAdd(A.counters + i, C.cnt[i]);
 }
 
-// block-tree fold over a tile of histories per block, FP64 atomics per bin
-__global__ void k_fold_tree(const double *__restrict__ hist, uint32_t n, long long nb,
-                            double *__restrict__ sum, double *__restrict__ sq, uint32_t rows_per_block)
-{
-    const uint32_t h0 = blockIdx.y * rows_per_block;
-    const uint32_t h1 = min(n, h0 + rows_per_block);
-    for (long long b = (long long)blockIdx.x * blockDim.x + threadIdx.x; b < nb;
-         b += (long long)gridDim.x * blockDim.x) {
-        double s = 0.0, q = 0.0;
-        for (uint32_t h = h0; h < h1; ++h) {
-            const double v = hist[(size_t)h * nb + b];
-            s += v;
-            q += v * v;
-        }
-        if (s != 0.0 || q != 0.0) {
-            atomicAdd(sum + b, s);
-            atomicAdd(sq + b, q);
-        }
-    }
-}
-
 }  // namespace
 
 size_t fp64_particle_bytes() { return sizeof(PartD); }
@@ -858,8 +836,14 @@ int history_fp64_max_threads(bool replay, int block)
 cudaError_t launch_history_fp64(const DevTables &T, const HistoryArgs &A, bool replay, int grid, int block,
                                 cudaStream_t st)
 {
+    if (A.n_params > 0 && (!replay || A.n_params > kMaxParams)) return cudaErrorInvalidValue;
+    const long long cols = A.n_params > 0 ? T.n_bins * (1 + (long long)(A.n_cols > A.n_params ? A.n_cols : A.n_params))
+                                          : T.n_bins;
+    if (cols > 0) {
+        const cudaError_t e = cudaMemsetAsync(A.hist, 0, (size_t)cols * A.hist_ld * sizeof(double), st);
+        if (e != cudaSuccess) return e;
+    }
     if (A.n_params > 0) {
-        if (!replay || A.n_params > kMaxParams) return cudaErrorInvalidValue;
         k_history_fp64<true, true><<<grid, block, 0, st>>>(T, A);
     } else if (replay) {
         k_history_fp64<true, false><<<grid, block, 0, st>>>(T, A);
@@ -869,18 +853,11 @@ cudaError_t launch_history_fp64(const DevTables &T, const HistoryArgs &A, bool r
     return cudaGetLastError();
 }
 
-cudaError_t launch_fold(const double *hist, uint32_t n, long long nb, double *sum, double *sq, bool ordered,
-                        cudaStream_t st)
+cudaError_t launch_fold_ordered(const double *hist, uint32_t n, uint64_t ld, long long n_cols, double *sum,
+                                double *sq, cudaStream_t st)
 {
-    if (nb <= 0 || n == 0) return cudaSuccess;
-    if (ordered) {
-        k_fold_ordered<<<dim3((unsigned)nb, 2), kFoldThreads, 0, st>>>(hist, n, nb, sum, sq);
-    } else {
-        const int block = 128;
-        const uint32_t rows = 512;
-        dim3 grid((unsigned)((nb + block - 1) / block), (n + rows - 1) / rows);
-        k_fold_tree<<<grid, block, 0, st>>>(hist, n, nb, sum, sq, rows);
-    }
+    if (n_cols <= 0 || n == 0) return cudaSuccess;
+    k_fold_ordered<<<dim3((unsigned)n_cols, 2), kFoldThreads, 0, st>>>(hist, n, ld, sum, sq);
     return cudaGetLastError();
 }
 

@@ -96,7 +96,8 @@ mc_status run_params(mc_problem *p, const double *params, uint64_t n, uint64_t s
     const uint64_t threads = (uint64_t)grid * block;
     uint64_t chunk = (uint64_t)((1ull << 30) / (row * sizeof(double)));
     chunk = std::max<uint64_t>(1, std::min<uint64_t>({chunk, 1u << 22, n}));
-    if (!devbuf_reserve(S.rows, (size_t)chunk * row * sizeof(double)) ||
+    const uint64_t ld = hist_rows(chunk);
+    if (!devbuf_reserve(S.rows, (size_t)ld * row * sizeof(double)) ||
         !devbuf_reserve(S.stack, (size_t)threads * depth * fp64_particle_bytes()) ||
         (K && !devbuf_reserve(S.lrstack, (size_t)threads * depth * K * sizeof(double))) ||
         !devbuf_reserve(S.sums, 2 * (size_t)row * sizeof(double)) ||
@@ -120,6 +121,7 @@ mc_status run_params(mc_problem *p, const double *params, uint64_t n, uint64_t s
         A.n = cn;
         A.seed = seed;
         A.hist = static_cast<double *>(S.rows.ptr);
+        A.hist_ld = ld;
         A.stack = S.stack.ptr;
         A.stack_depth = depth;
         A.counters = cnt;
@@ -131,7 +133,7 @@ mc_status run_params(mc_problem *p, const double *params, uint64_t n, uint64_t s
         A.lr_stack = K ? static_cast<double *>(S.lrstack.ptr) : nullptr;
         if ((e = cudaMemsetAsync(next, 0, sizeof(unsigned int), d.stream)) != cudaSuccess ||
             (e = launch_history_fp64(T, A, true, grid, block, d.stream)) != cudaSuccess ||
-            (e = launch_fold(A.hist, cn, row, dsum, dsq, true, d.stream)) != cudaSuccess) {
+            (e = launch_fold_ordered(A.hist, cn, ld, row, dsum, dsq, d.stream)) != cudaSuccess) {
             p->err = cuda_msg(e, "derivative kernels");
             return MC_ERR_CUDA;
         }

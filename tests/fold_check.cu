@@ -38,17 +38,18 @@ int main()
         for (uint32_t n : {1u, 7u, 8u, 9u, 4095u, 4096u, 4097u, 8193u, 30011u}) {
             for (int start = 0; start < 2; ++start) {
                 std::mt19937_64 g(n + nb);
-                std::vector<double> h((size_t)n * nb), s0(nb), q0(nb);
+                const size_t ld = (n + 7) & ~7u;
+                std::vector<double> h(ld * nb, 0.0), s0(nb), q0(nb);
                 for (int b = 0; b < nb; ++b) {
                     s0[b] = start ? (b % 2 ? -3.25 : 1.0) : 0.0;
                     q0[b] = start ? 0.5 : 0.0;
                     const int kind = nb == 1 ? (int)(n % 12) : b;
-                    for (uint32_t i = 0; i < n; ++i) h[(size_t)i * nb + b] = column(kind, g, i);
+                    for (uint32_t i = 0; i < n; ++i) h[b * ld + i] = column(kind, g, i);
                 }
                 std::vector<double> s = s0, q = q0, rs(nb), rq(nb);
                 for (int b = 0; b < nb; ++b)
                     for (uint32_t i = 0; i < n; ++i) {
-                        const double v = h[(size_t)i * nb + b];
+                        const double v = h[b * ld + i];
                         s[b] += v;
                         const double w = v * v;
                         q[b] += w;
@@ -58,7 +59,7 @@ int main()
                 cudaMemcpy(dh, h.data(), h.size() * 8, cudaMemcpyHostToDevice);
                 cudaMemcpy(ds, s0.data(), nb * 8, cudaMemcpyHostToDevice);
                 cudaMemcpy(ds + nb, q0.data(), nb * 8, cudaMemcpyHostToDevice);
-                mc::k_fold_ordered<<<dim3(nb, 2), mc::kFoldThreads>>>(dh, n, nb, ds, ds + nb);
+                mc::k_fold_ordered<<<dim3(nb, 2), mc::kFoldThreads>>>(dh, n, ld, ds, ds + nb);
                 cudaMemcpy(rs.data(), ds, nb * 8, cudaMemcpyDeviceToHost);
                 cudaMemcpy(rq.data(), ds + nb, nb * 8, cudaMemcpyDeviceToHost);
                 if (cudaGetLastError() != cudaSuccess) { std::printf("CUDA error\n"); return 2; }
