@@ -41,6 +41,7 @@ SOURCES = [
     ("mc_api.cpp", "host"),
     ("mc_report.cpp", "host"),
     ("mc_evtables.cpp", "host"),
+    ("mc_fp64tables.cpp", "host"),
     ("mc_api_batch.cpp", "host"),
     ("mc_lr.cpp", "host"),
     ("mc_history.cu", "fp64"),

@@ -5,10 +5,13 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "mc_fp64tables.h"
+
 namespace mc {
 
 // Plain-pointer view of Tables (mc_problem.h) in device memory.  Every array
-// lives in one allocation; the layouts are those documented in mc_problem.h.
+// lives in one allocation; the layouts are those documented in mc_problem.h
+// and mc_fp64tables.h.
 struct DevTables {
     int n_surf, n_cell, n_mat, n_nuc, mg_groups, n_est, n_src;
     long long n_bins;
@@ -19,13 +22,19 @@ struct DevTables {
     const double *cell_imp;
     const int *cell_mat, *cell_surf_off, *cell_surf, *cell_sense;
     const int *cell_tl_off, *cell_tl, *cell_c_off, *cell_c, *surf_est_off, *surf_est;
+    const int *cell_tl_pre, *cell_c_pre, *surf_est_pre;
     const int *mat_off, *mat_nuc;
     const double *mat_dens;
-    const int *nuc_kind, *nuc_len;
-    const double *nuc_A, *nuc_const;
-    const long long *nuc_off;
-    const double *xs_E, *xs_S, *xs_C, *xs_T;
-    const double *mg_total, *mg_scatter, *mg_scat_tot, *mg_capture;
+    // mc_fp64tables.h
+    const Nuc64 *nuc;
+    const Grid64 *xs_grid;
+    const XsRow64 *xs_row;
+    const Recip64 *xs_inv;
+    const int *xs_bkt;
+    const Mg64 *mg;
+    const double *mg_cum;
+    const int *est_ifac, *est_time;
+    int any_time;
     const int *est_score_off, *score_kind, *score_kernel;
     const int *est_filt_off, *filt_kind, *filt_size, *filt_grid_len;
     const long long *filt_grid_off;
@@ -70,6 +79,7 @@ struct HistoryArgs {
     // both cross sections of the material)
     int n_cols = 0;
     uint32_t max_events = 1u << 22;   // events per particle before DS_TIMEOUT
+    int lanes = 32;                   // lanes of a warp that take histories
 };
 
 constexpr int kMaxLrParams = 64;   // (Sigma_s, Sigma_a) for up to 32 materials
@@ -107,7 +117,10 @@ cudaError_t launch_exact_normalize(long long *ex, long long n_bins, cudaStream_t
 // Bytes of one FP64 split-stack entry.
 size_t fp64_particle_bytes();
 
-// Resident-thread estimate for the FP64 history kernel.
-int history_fp64_max_threads(bool replay, int block);
+// Launch shape of the FP64 history kernel for n histories on this device.
+struct HistoryShape {
+    int grid, lanes;
+};
+HistoryShape history_fp64_shape(uint64_t n);
 
 }  // namespace mc

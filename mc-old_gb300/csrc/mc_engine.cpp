@@ -80,6 +80,32 @@ struct Packer {
 
 }  // namespace
 
+// Saved states are keyed by a fingerprint of the problem: FNV-1a over the
+// reader's tables in this order, each at the next multiple of 256 bytes.  The
+// order and padding are part of the file format.
+uint64_t table_fingerprint(const Tables &t)
+{
+    std::vector<char> buf;
+    auto add = [&](const auto &v) {
+        const size_t size = sizeof(v[0]), off = (buf.size() + 255) & ~(size_t)255;
+        buf.resize(off + std::max<size_t>(v.size() * size, 8), 0);
+        if (!v.empty()) std::memcpy(buf.data() + off, v.data(), v.size() * size);
+    };
+    add(t.surf_type); add(t.surf_bc); add(t.surf_coef); add(t.cell_imp); add(t.cell_mat);
+    add(t.cell_surf_off); add(t.cell_surf); add(t.cell_sense); add(t.cell_tl_off); add(t.cell_tl);
+    add(t.cell_c_off); add(t.cell_c); add(t.surf_est_off); add(t.surf_est); add(t.mat_off); add(t.mat_nuc);
+    add(t.mat_dens); add(t.nuc_kind); add(t.nuc_len); add(t.nuc_A); add(t.nuc_const); add(t.nuc_off);
+    add(t.xs_E); add(t.xs_S); add(t.xs_C); add(t.xs_T); add(t.mg_total); add(t.mg_scatter);
+    add(t.mg_scat_tot); add(t.mg_capture); add(t.est_score_off); add(t.score_kind); add(t.score_kernel);
+    add(t.est_filt_off); add(t.filt_kind); add(t.filt_size); add(t.filt_grid_len); add(t.filt_grid_off);
+    add(t.filt_grid); add(t.est_factor); add(t.est_factor_off); add(t.est_bin_off); add(t.src_pos);
+    add(t.src_dir_par); add(t.src_e_par); add(t.src_cdf); add(t.src_cell); add(t.src_dir_kind);
+    add(t.src_e_kind); add(t.src_group);
+    uint64_t h = 0xCBF29CE484222325ULL;
+    for (const char c : buf) h = (h ^ (unsigned char)c) * 0x100000001B3ULL;
+    return h;
+}
+
 mc_status device_problem_init(const Tables &t, DeviceProblem &d, std::string &err)
 {
     int ndev = 0;
@@ -103,6 +129,9 @@ mc_status device_problem_init(const Tables &t, DeviceProblem &d, std::string &er
     T.n_bins = t.n_bins();
     T.wr = t.wr; T.ws = t.ws;
     T.comb_bank_max = t.comb_bank_max; T.comb_teeth = t.comb_teeth;
+    Fp64Tables F;
+    build_fp64_tables(t, F);
+    T.any_time = F.any_time;
     Packer P;
     P.add(t.surf_type, &T.surf_type); P.add(t.surf_bc, &T.surf_bc); P.add(t.surf_coef, &T.surf_coef);
     P.add(t.cell_imp, &T.cell_imp); P.add(t.cell_mat, &T.cell_mat); P.add(t.cell_surf_off, &T.cell_surf_off);
@@ -110,20 +139,17 @@ mc_status device_problem_init(const Tables &t, DeviceProblem &d, std::string &er
     P.add(t.cell_tl_off, &T.cell_tl_off); P.add(t.cell_tl, &T.cell_tl);
     P.add(t.cell_c_off, &T.cell_c_off); P.add(t.cell_c, &T.cell_c);
     P.add(t.surf_est_off, &T.surf_est_off); P.add(t.surf_est, &T.surf_est);
+    P.add(F.tl_pre, &T.cell_tl_pre); P.add(F.c_pre, &T.cell_c_pre); P.add(F.s_pre, &T.surf_est_pre);
     P.add(t.mat_off, &T.mat_off); P.add(t.mat_nuc, &T.mat_nuc); P.add(t.mat_dens, &T.mat_dens);
-    P.add(t.nuc_kind, &T.nuc_kind); P.add(t.nuc_len, &T.nuc_len); P.add(t.nuc_A, &T.nuc_A);
-    P.add(t.nuc_const, &T.nuc_const);
-    std::vector<long long> nuc_off(t.nuc_off.begin(), t.nuc_off.end());
-    P.add(nuc_off, &T.nuc_off);
-    P.add(t.xs_E, &T.xs_E); P.add(t.xs_S, &T.xs_S); P.add(t.xs_C, &T.xs_C); P.add(t.xs_T, &T.xs_T);
-    P.add(t.mg_total, &T.mg_total); P.add(t.mg_scatter, &T.mg_scatter);
-    P.add(t.mg_scat_tot, &T.mg_scat_tot); P.add(t.mg_capture, &T.mg_capture);
+    P.add(F.nuc, &T.nuc); P.add(F.grid, &T.xs_grid); P.add(F.row, &T.xs_row); P.add(F.inv, &T.xs_inv);
+    P.add(F.bkt, &T.xs_bkt); P.add(F.mg, &T.mg); P.add(F.mg_cum, &T.mg_cum);
     P.add(t.est_score_off, &T.est_score_off); P.add(t.score_kind, &T.score_kind);
     P.add(t.score_kernel, &T.score_kernel); P.add(t.est_filt_off, &T.est_filt_off);
     P.add(t.filt_kind, &T.filt_kind); P.add(t.filt_size, &T.filt_size); P.add(t.filt_grid_len, &T.filt_grid_len);
     std::vector<long long> fgo(t.filt_grid_off.begin(), t.filt_grid_off.end());
     P.add(fgo, &T.filt_grid_off);
-    P.add(t.filt_grid, &T.filt_grid); P.add(t.est_factor, &T.est_factor);
+    P.add(t.filt_grid, &T.filt_grid); P.add(t.est_factor, &T.est_factor); P.add(F.est_ifac, &T.est_ifac);
+    P.add(F.est_time, &T.est_time);
     P.add(t.est_factor_off, &T.est_factor_off);
     std::vector<long long> ebo(t.est_bin_off.begin(), t.est_bin_off.end());
     P.add(ebo, &T.est_bin_off);
@@ -253,9 +279,9 @@ mc_status run_fp64(const Tables &t, DeviceProblem &d, uint64_t first, uint64_t n
     // a combed bank holds `teeth` particles plus the split copies of one walk
     if (t.comb_teeth > 0 && !(tune && tune->stack_depth)) depth = std::max<uint32_t>(depth, (uint32_t)t.comb_teeth + 32);
     const bool want_digest = tune && tune->record_digests;
-    int max_threads = history_fp64_max_threads(replay, block);
-    int grid = (tune && tune->grid_blocks) ? (int)tune->grid_blocks : max_threads / block;
-    if (grid < 1) grid = 1;
+    HistoryShape shape = history_fp64_shape(n);
+    if (tune && tune->grid_blocks) shape = {(int)tune->grid_blocks, 32};
+    const int grid = shape.grid;
     const long long nb = std::max<long long>(d.dt.n_bins, 1);
     // chunk: histories whose per-history rows are kept before the fold;
     // bounded to ~1 GiB of rows
@@ -305,6 +331,7 @@ mc_status run_fp64(const Tables &t, DeviceProblem &d, uint64_t first, uint64_t n
         A.digest = want_digest ? static_cast<unsigned long long *>(d.digest.ptr) : nullptr;
         A.status = d_status;
         A.next = d_next;
+        A.lanes = shape.lanes;
         cudaMemsetAsync(d_next, 0, sizeof(unsigned int), d.stream);
         cudaEventRecord(d.ev[1], d.stream);
         if ((e = launch_history_fp64(d.dt, A, replay, grid, block, d.stream)) != cudaSuccess) {

@@ -51,6 +51,9 @@ struct DeviceProblem {
     void *lr = nullptr;            // forward / backward scratch (mc_lr.cpp)
 };
 
+// key of a problem's saved states (mc_state_save)
+uint64_t table_fingerprint(const Tables &t);
+
 mc_status device_problem_init(const Tables &t, DeviceProblem &d, std::string &err);
 void device_problem_free(DeviceProblem &d);
 mc_status reset_tallies(DeviceProblem &d, std::string &err);

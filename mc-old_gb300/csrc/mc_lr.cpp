@@ -76,23 +76,22 @@ mc_status run_params(mc_problem *p, const double *params, uint64_t n, uint64_t s
         stot[m] = 0.0 + ss;
         cap[m] = tot[m] - stot[m];
     }
-    const size_t tb = 4 * (size_t)nm * sizeof(double) + 4 * 256;
-    if (!devbuf_reserve(S.tab, tb)) { p->err = "cannot allocate parameter tables"; return MC_ERR_NOMEM; }
+    std::vector<Mg64> mg;
+    std::vector<double> cum;
+    build_mg64(nm, 1, tot.data(), sca.data(), stot.data(), cap.data(), mg, cum);
+    const size_t mg_bytes = mg.size() * sizeof(Mg64);
+    if (!devbuf_reserve(S.tab, mg_bytes + cum.size() * sizeof(double) + 256)) { p->err = "cannot allocate parameter tables"; return MC_ERR_NOMEM; }
     char *tp = static_cast<char *>(S.tab.ptr);
     DevTables T = d.dt;
-    const size_t step = ((size_t)nm * sizeof(double) + 255) & ~(size_t)255;
-    cudaMemcpyAsync(tp, tot.data(), nm * sizeof(double), cudaMemcpyHostToDevice, d.stream);
-    cudaMemcpyAsync(tp + step, sca.data(), nm * sizeof(double), cudaMemcpyHostToDevice, d.stream);
-    cudaMemcpyAsync(tp + 2 * step, stot.data(), nm * sizeof(double), cudaMemcpyHostToDevice, d.stream);
-    cudaMemcpyAsync(tp + 3 * step, cap.data(), nm * sizeof(double), cudaMemcpyHostToDevice, d.stream);
-    T.mg_total = reinterpret_cast<const double *>(tp);
-    T.mg_scatter = reinterpret_cast<const double *>(tp + step);
-    T.mg_scat_tot = reinterpret_cast<const double *>(tp + 2 * step);
-    T.mg_capture = reinterpret_cast<const double *>(tp + 3 * step);
+    cudaMemcpyAsync(tp, mg.data(), mg_bytes, cudaMemcpyHostToDevice, d.stream);
+    cudaMemcpyAsync(tp + mg_bytes, cum.data(), cum.size() * sizeof(double), cudaMemcpyHostToDevice, d.stream);
+    T.mg = reinterpret_cast<const Mg64 *>(tp);
+    T.mg_cum = reinterpret_cast<const double *>(tp + mg_bytes);
 
     const int block = 128;
     const uint32_t depth = 32;
-    const int grid = std::max(1, history_fp64_max_threads(true, block) / block);
+    const HistoryShape shape = history_fp64_shape(n);
+    const int grid = shape.grid;
     const uint64_t threads = (uint64_t)grid * block;
     uint64_t chunk = (uint64_t)((1ull << 30) / (row * sizeof(double)));
     chunk = std::max<uint64_t>(1, std::min<uint64_t>({chunk, 1u << 22, n}));
@@ -128,6 +127,7 @@ mc_status run_params(mc_problem *p, const double *params, uint64_t n, uint64_t s
         A.digest = nullptr;
         A.status = status;
         A.next = next;
+        A.lanes = shape.lanes;
         A.n_params = K;
         A.n_cols = Kc;
         A.lr_stack = K ? static_cast<double *>(S.lrstack.ptr) : nullptr;

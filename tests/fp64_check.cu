@@ -1,0 +1,152 @@
+// fp64_check.cu -- the FP64 kernels' helpers against what they stand for, on
+// the GPU over random and edge inputs: the bit-assembled uniforms, the
+// comparisons, the reciprocal division and the portable functions must give
+// the same bits as the plain FP64 expressions; the FP32 bounds must hold the
+// FP64 values, and the FP32 decisions must be the FP64 ones.  Prints "ok" or
+// what differs.
+#include <cstdio>
+#include <vector>
+
+#include "mc_history.cu"
+
+using namespace mc;
+
+enum { E_U01, E_MU, E_DIV, E_LOG, E_SINCOS, E_QUARTER, E_DLT, E_NEGLOG, E_BRANCH, E_CAND, E_DIST, E_OUT, E_UNSURE, E_CASES, E_N };
+
+__device__ __forceinline__ bool same(double a, double b) { return dbits(a) == dbits(b) || (a != a && b != b); }
+
+__global__ void k_check(DevTables T, int n_surf, uint64_t n, unsigned long long *err)
+{
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+        const U4 a = philox((uint32_t)i, (uint32_t)(i >> 32), 1, 2, 3, 4), e = philox((uint32_t)i, (uint32_t)(i >> 32), 2, 2, 3, 4);
+        const U4 c = philox((uint32_t)i, (uint32_t)(i >> 32), 3, 2, 3, 4);
+        auto pick = [&](uint32_t lo, uint32_t hi) {
+            uint64_t v = (((uint64_t)hi << 32) | lo) >> 12;
+            // the ends of the range, quadrant limits and their neighbours
+            if ((i & 15) == 0) {
+                const uint64_t at[8] = {0, (1ull << 52) - 1, 1ull << 49, 3ull << 49, 5ull << 49, 7ull << 49, 1ull << 51, 1ull << 50};
+                v = (at[v & 7] + ((v >> 3) % 5) - 2) & ((1ull << 52) - 1);
+            }
+            return v;
+        };
+        const uint64_t v1 = pick(a.x, a.y), v2 = pick(a.z, a.w), v3 = pick(e.x, e.y), v4 = pick(e.z, e.w), v5 = pick(c.x, c.y);
+        const double u1 = ((double)v1 + 0.5) * 0x1p-52, u2 = ((double)v2 + 0.5) * 0x1p-52, u3 = ((double)v3 + 0.5) * 0x1p-52;
+        if (!same(u01_bits(v1), u1)) atomicAdd(err + E_U01, 1ull);
+        if (!same(mu_bits(v1), 2.0 * u1 - 1.0)) atomicAdd(err + E_MU, 1ull);
+        // divisions: random significands, exponents of the tables' range
+        {
+            const double d = dfrom((dbits(u2) & 0x000FFFFFFFFFFFFFull) | ((uint64_t)(1023 - 150 + c.z % 300) << 52));
+            double x = dfrom((dbits(u1) & 0x800FFFFFFFFFFFFFull) | ((uint64_t)(1023 - 250 + c.w % 500) << 52) | ((uint64_t)(c.z & 1) << 63));
+            if ((i & 63) == 0) x = 0.0;
+            if ((i & 63) == 1) x = -0.0;
+            if ((i & 63) == 2) x = dfrom(dbits(x) & 0x800FFFFFFFFFFFFFull);
+            const double hi = 1.0 / d;
+            const Recip64 r{hi, __fma_rn(-d, hi, 1.0) * hi};
+            if (!same(div_by(x, d, r), x / d) || !same(div_by(x, d, Recip64{0.0, 0.0}), x / d)) atomicAdd(err + E_DIV, 1ull);
+        }
+        if (!same(plog_unit(u1, d_ln), plog(u1)) || !same(plog_unit(u1 * u2, d_ln), plog(u1 * u2))) atomicAdd(err + E_LOG, 1ull);
+        {
+            double s, k;
+            psincos_azi(kPi2 * u1, v1, s, k);
+            if (!same(s, psin(kPi2 * u1)) || !same(k, pcos(kPi2 * u1))) atomicAdd(err + E_SINCOS, 1ull);
+            if (!same(pcos_quarter(kPiHalf * u1, v1), pcos(kPiHalf * u1))) atomicAdd(err + E_QUARTER, 1ull);
+        }
+        {
+            const double odd[8] = {0.0, -0.0, 1.0, -1.0, 1e308 * 10.0, -1e308 * 10.0, 0.0 / 0.0, 4.9e-324};
+            const double x = (c.z & 8) ? odd[c.z & 7] : u1 - u2, y = (c.z & 128) ? odd[(c.z >> 4) & 7] : u1 - u3;
+            if (dlt(x, y) != (x < y)) atomicAdd(err + E_DLT, 1ull);
+        }
+        if (!(fabs((double)neglog_bits(v1) / -plog(u1) - 1.0) < 2e-6)) atomicAdd(err + E_NEGLOG, 1ull);
+        // free-gas candidates from y = 1e-3 (far below thermal) to 1e5
+        {
+            const double beta = 1.0, speed = exp(-7.0 + 18.5 * ((double)v5 * 0x1p-52));
+            const float y32 = f32_of(beta * speed);
+            int is = branch_test(v4, y32);
+            const bool w2 = u01_bits(v4) < 2.0 / (2.0 + kPiSqrt * (beta * speed));
+            if (is >= 0 && (is != 0) != w2) atomicAdd(err + E_BRANCH, 1ull);
+            // the acceptance draw near its limit half of the time
+            uint64_t va = ((uint64_t)c.w << 20) ^ e.x;
+            for (int w = 0; w < 2; ++w) {
+                double x;
+                if (w) x = dsqrt(-plog(u1 * u2));
+                else { const double k = pcos(kPiHalf * u1); x = dsqrt(-plog(u2) - plog(u3) * k * k); }
+                const double mu = mu_bits(v4);
+                const double acc = dsqrt(speed * speed + x * x - 2.0 * speed * x * mu) / (speed + x);
+                if (i & 1) {
+                    const double near = acc * (1.0 + ((double)c.z * 0x1p-32 - 0.5) * 4e-4);
+                    va = (uint64_t)fmin(fmax(near * 0x1p52, 0.0), 0x1p52 - 1.0);
+                }
+                is = candidate_test(w != 0, v1, v2, v3, v4, va, y32);
+                const bool take = !(u01_bits(va) > acc);
+                if (is >= 0 && (is != 0) != take) atomicAdd(err + E_CAND, 1ull);
+                if (!(i & 1)) { atomicAdd(err + E_CASES, 1ull); if (is < 0) atomicAdd(err + E_UNSURE, 1ull); }
+            }
+        }
+        // surfaces: points near to and far from them, unit directions and others
+        {
+            const int s = (int)(c.w % (uint32_t)n_surf);
+            Lane P;
+            const double far = (i & 2) ? 100.0 : 12.0;
+            P.x = far * (2.0 * u1 - 1.0); P.y = far * (2.0 * u2 - 1.0); P.z = far * (2.0 * u3 - 1.0);
+            double uu = mu_bits(v4), vv = mu_bits(v5), ww = mu_bits(v1);
+            const double len = sqrt(uu * uu + vv * vv + ww * ww);
+            if (i & 4) { uu /= len; vv /= len; ww /= len; }
+            P.u = uu; P.v = vv; P.w = ww;
+            if (i & 8) {           // onto the surface, then off it by a nudge
+                const double d = surface_distance(T, s, P.x, P.y, P.z, P.u, P.v, P.w);
+                if (d < 1e6) {
+                    const double e = d + ((i & 16) ? kEpsF : -kEpsF) * ((i & 32) ? 1.0 : 1e3);
+                    P.x += P.u * e; P.y += P.v * e; P.z += P.w * e;
+                }
+            }
+            const float reach = (float)exp(-14.0 + 20.0 * ((double)(c.x >> 8) * 0x1p-24));
+            const float2 b = distance_bounds(T, s, P.x, P.y, P.z, P.u, P.v, P.w, reach);
+            const float lo = b.x, hi = b.y;
+            const double d = surface_distance(T, s, P.x, P.y, P.z, P.u, P.v, P.w);
+            const double dd = d >= kMaxF ? (double)kInfF : d;
+            const bool good = lo == kInfF ? (dd == (double)kInfF || d > (double)reach) : ((double)lo <= dd && dd <= (double)hi);
+            if (!good) atomicAdd(err + E_DIST, 1ull);
+            for (int sense = -1; sense <= 1; ++sense)
+                if (outside(T, s, sense, P.x, P.y, P.z) != (surface_eval(T, s, P.x, P.y, P.z) * sense < 0)) atomicAdd(err + E_OUT, 1ull);
+        }
+    }
+}
+
+int main()
+{
+    // planes, general planes, spheres and cylinders, centred and not
+    std::vector<int> type;
+    std::vector<double> k;
+    auto add = [&](int t, std::vector<double> c) { type.push_back(t); c.resize(8, 0.0); k.insert(k.end(), c.begin(), c.end()); };
+    for (int t = 0; t < 3; ++t) { add(t, {0.0}); add(t, {7.25}); add(t, {-90.0}); add(t, {1e-9}); }
+    add(3, {1.0, 0.5, -0.25, 6.0}); add(3, {-1.0, 0.2, 0.1, 6.0});
+    for (double r : {0.5, 10.0, 30.0, 70.0}) {
+        add(4, {0.0, 0.0, 0.0, r, r * r}); add(4, {3.0, -40.0, 0.1, r, r * r});
+        add(5, {0.0, 0.0, r, r * r}); add(5, {5.0, -1.0, r, r * r});
+        add(6, {0.5, 0.0, r, r * r});
+        add(7, {0.0, 0.0, r, r * r}); add(7, {0.5, -20.0, r, r * r});
+    }
+    DevTables T{};
+    int *dt;
+    double *dk;
+    unsigned long long *de, e[E_N] = {};
+    if (cudaMalloc(&dt, type.size() * 4) != cudaSuccess || cudaMalloc(&dk, k.size() * 8) != cudaSuccess ||
+        cudaMalloc(&de, sizeof(e)) != cudaSuccess) return 2;
+    cudaMemcpy(dt, type.data(), type.size() * 4, cudaMemcpyHostToDevice);
+    cudaMemcpy(dk, k.data(), k.size() * 8, cudaMemcpyHostToDevice);
+    cudaMemset(de, 0, sizeof(e));
+    T.surf_type = dt;
+    T.surf_coef = dk;
+    k_check<<<608, 128>>>(T, (int)type.size(), 40000000ull, de);
+    if (cudaMemcpy(e, de, sizeof(e), cudaMemcpyDeviceToHost) != cudaSuccess) { std::printf("CUDA error\n"); return 2; }
+    const char *what[] = {"uniform", "mu", "division", "log", "sincos", "cos quarter", "compare", "neglog", "branch",
+                          "candidate", "distance bounds", "outside"};
+    bool bad = false;
+    for (int i = 0; i <= E_OUT; ++i)
+        if (e[i]) { std::printf("%s: %llu wrong\n", what[i], e[i]); bad = true; }
+    // the FP32 test is of use only if it almost always tells
+    std::fprintf(stderr, "candidates left to FP64: %.2e\n", (double)e[E_UNSURE] / (double)e[E_CASES]);
+    if (e[E_UNSURE] * 200 > e[E_CASES]) { std::printf("too many candidates undecided\n"); bad = true; }
+    if (!bad) std::printf("ok\n");
+    return bad;
+}
