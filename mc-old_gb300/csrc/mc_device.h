@@ -121,6 +121,6 @@ size_t fp64_particle_bytes();
 struct HistoryShape {
     int grid, lanes;
 };
-HistoryShape history_fp64_shape(uint64_t n);
+HistoryShape history_fp64_shape(uint64_t n, bool multigroup);
 
 }  // namespace mc

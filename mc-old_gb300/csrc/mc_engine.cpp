@@ -279,7 +279,7 @@ mc_status run_fp64(const Tables &t, DeviceProblem &d, uint64_t first, uint64_t n
     // a combed bank holds `teeth` particles plus the split copies of one walk
     if (t.comb_teeth > 0 && !(tune && tune->stack_depth)) depth = std::max<uint32_t>(depth, (uint32_t)t.comb_teeth + 32);
     const bool want_digest = tune && tune->record_digests;
-    HistoryShape shape = history_fp64_shape(n);
+    HistoryShape shape = history_fp64_shape(n, t.mg_groups > 0);
     if (tune && tune->grid_blocks) shape = {(int)tune->grid_blocks, 32};
     const int grid = shape.grid;
     const long long nb = std::max<long long>(d.dt.n_bins, 1);

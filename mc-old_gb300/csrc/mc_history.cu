@@ -1172,8 +1172,14 @@ constexpr int kCollideQuarters = 3;
 // idle lanes that take new histories together, while others have work
 constexpr int kRefillLanes = 4;
 
+// CTAs per SM: registers allow 3 for continuous energy (168 a thread; at 128
+// the spills cost more than a fourth CTA gives while histories run out: 13.8
+// against 12.1 ms on 50,000 shields) and 4 for the multigroup flavours (deep
+// slab 6.0 / 5.1 / 4.9 ms at 2 / 3 / 4).
+constexpr int ctas_per_sm(int flavour) { return flavour == F_CE ? 3 : 4; }
+
 template <bool R, int F>
-__global__ void __launch_bounds__(kBlock, 2) k_history_fp64(const __grid_constant__ DevTables T,
+__global__ void __launch_bounds__(kBlock, ctas_per_sm(F)) k_history_fp64(const __grid_constant__ DevTables T,
                                                             const __grid_constant__ HistoryArgs A)
 {
     const size_t tid = (size_t)blockIdx.x * kBlock + threadIdx.x;
@@ -1380,18 +1386,21 @@ __global__ void __launch_bounds__(kBlock, 2) k_history_fp64(const __grid_constan
 size_t fp64_particle_bytes() { return sizeof(PartD); }
 
 // One FP64 instruction takes a scheduler's pipe 64 cycles and more, for one
-// lane as for 32, so a single warp per scheduler (one CTA per SM) nearly
-// fills it.  Few histories are spread over all schedulers with as few lanes
-// of a warp each.
-HistoryShape history_fp64_shape(uint64_t n)
+// lane as for 32.  Few histories are therefore spread over all schedulers with
+// as few lanes of a warp each (3,001 duct histories: 4.8 ms, in full warps 5.6
+// ms); beyond one full warp per scheduler, CTAs are added until every history
+// has a lane or the registers run out.
+HistoryShape history_fp64_shape(uint64_t n, bool multigroup)
 {
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const uint64_t warps = (uint64_t)std::max(sms, 1) * (kBlock / 32);
+    sms = std::max(sms, 1);
+    const uint64_t warps = (uint64_t)sms * (kBlock / 32);
     if (n <= warps) return {(int)std::max<uint64_t>(1, (n + 3) / 4), 1};
     if (n <= warps * 32) return {sms, (int)((n + warps - 1) / warps)};
-    return {2 * sms, 32};
+    const uint64_t per_sm = (n + warps * 32 - 1) / (warps * 32);
+    return {sms * (int)std::min<uint64_t>(per_sm, (uint64_t)ctas_per_sm(multigroup ? F_MG : F_CE)), 32};
 }
 
 cudaError_t launch_history_fp64(const DevTables &T, const HistoryArgs &A, bool replay, int grid, int block,

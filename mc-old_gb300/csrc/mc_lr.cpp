@@ -90,7 +90,7 @@ mc_status run_params(mc_problem *p, const double *params, uint64_t n, uint64_t s
 
     const int block = 128;
     const uint32_t depth = 32;
-    const HistoryShape shape = history_fp64_shape(n);
+    const HistoryShape shape = history_fp64_shape(n, true);
     const int grid = shape.grid;
     const uint64_t threads = (uint64_t)grid * block;
     uint64_t chunk = (uint64_t)((1ull << 30) / (row * sizeof(double)));
