@@ -1189,6 +1189,11 @@ __device__ __forceinline__ int event_collide_begin(Ctx &C, const EvTables &V, Rn
     C.cnt[C_COLL]++;
     const int m = V.cell_mat[p.cell];
     if (m < 0) return 0;
+    // in a material the flight took draw 0 and the stream holds its block:
+    // said with constants, so that the collision's draws (1 to 4, all in that
+    // block) need no block test, no word selection and no refill code
+    R.draw = 1u;
+    R.cached = 1u;
     for (int i = V.cell_c_off[p.cell]; i < V.cell_c_off[p.cell + 1]; ++i)
         estimator_score<kFl>(C, V.cell_c[i], p, p.t, V.has_time ? speed_of(p.E) : 0.f, 0.f,
                                        V.cell_c_pre[i], 1);
@@ -1825,8 +1830,12 @@ __global__ void __launch_bounds__(kTrackBlock, MinB) k_track(const EvTables V0, 
         }
     }
     if (threadIdx.x == 0 && s_status != 0) atomicCAS(A.status, 0, s_status);
-    for (int i = 0; i < kNumCounters; ++i) {
-        unsigned long long v = C.cnt[i];
+    // the CTA's counters: a warp adds the 128 columns of every fourth one (all
+    // CTAs' additions meet at the same nine addresses; one per warp and
+    // counter queued up there at the end of short runs)
+    for (int i = threadIdx.x / 32; i < kNumCounters; i += kTrackBlock / 32) {
+        unsigned long long v = 0;
+        for (int t = lane; t < kTrackBlock; t += 32) v += s_cnt[i * kCntStride + t];
         for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
         if (lane == 0 && v) atomicAdd(A.counters + i, v);
     }
