@@ -47,7 +47,7 @@ struct EvArgs {
     double *const *psum;          // [n_prob] per-problem tallies
     double *const *psq;
     int n_prob;
-    // batches, and single problems whose sums do not fit in shared memory,
+    // batches, and single problems whose sums do not live in shared memory,
     // fold histories into n_rep > 0 replicas of their bins ([n_rep]
     // [rep_stride], problem p's bins from rep_off[p] on), each CTA into
     // replica blockIdx % n_rep; k_batch_reduce adds them to psum / psq
@@ -595,8 +595,10 @@ __device__ __forceinline__ void tally_add(Ctx &C, int hslot, int bin, double val
 {
     if constexpr (kFl == FL_MG) {
         if (C.cbin == bin || C.cbin < 0) {
+            // most histories score once: no FP64 addition (19 SM cycles a warp)
+            if (C.cbin < 0) C.cval = val;
+            else C.cval += val;
             C.cbin = bin;
-            C.cval += val;
             C.cnt[C_TALLY]++;
             return;
         }
@@ -1065,9 +1067,16 @@ __device__ __forceinline__ void weight_roulette(Ctx &C, Rng32 &R, PState &p, boo
     }
 }
 
-// SourceBank / SourcePoint (Source.cpp:20-24, 42-45), FP32
-__device__ void sample_source(const EvTables &V, uint64_t seed, uint64_t hist, PState &p)
+// SourceBank / SourcePoint (Source.cpp:20-24, 42-45), FP32: the source point
+// and the sampled direction and energy
+struct SrcDraw {
+    float u, v, w, E;
+    int s;
+};
+
+__device__ __forceinline__ SrcDraw draw_source(const EvTables &V, uint64_t seed, uint64_t hist)
 {
+    SrcDraw d;
     Rng32 R;
     R.init(seed, hist, 0u, 0u, 0u);
     R.prime();
@@ -1075,35 +1084,45 @@ __device__ void sample_source(const EvTables &V, uint64_t seed, uint64_t hist, P
     int s = bsearch_f(xi, V.src_cdf, V.n_src + 1);
     s = s < 0 ? 0 : (s >= V.n_src ? V.n_src - 1 : s);
     const float *ep = V.src_e_par + 2 * s;
-    const float E = (V.src_e_kind[s] == 1) ? ep[0] + R.next() * ep[1] : ep[0];
+    d.s = s;
+    d.E = (V.src_e_kind[s] == 1) ? ep[0] + R.next() * ep[1] : ep[0];
     const float *dp = V.src_dir_par + 9 * s;
     const int dk = V.src_dir_kind[s];
-    float d0, d1, d2;
     if (dk == 0) {
-        d0 = dp[0]; d1 = dp[1]; d2 = dp[2];
+        d.u = dp[0]; d.v = dp[1]; d.w = dp[2];
     } else if (dk == 1 || dk == 3) {
         const float mu = (dk == 1) ? 2.f * R.next() - 1.f : R.next();
         float sa, ca;
         __sincosf(k2PiF * R.next(), &sa, &ca);
         const float c = sqrtf(fmaxf(1.f - mu * mu, 0.f));
-        d0 = mu; d1 = ca * c; d2 = sa * c;
+        d.u = mu; d.v = ca * c; d.w = sa * c;
     } else {
-        float d[3];
+        float x[3];
         for (int k = 2; k >= 0; --k) {
             const float *q = dp + 3 * k;
-            d[k] = ((int)q[0] == 1) ? q[1] + R.next() * q[2] : q[1];
+            x[k] = ((int)q[0] == 1) ? q[1] + R.next() * q[2] : q[1];
         }
-        d0 = d[0]; d1 = d[1]; d2 = d[2];
+        d.u = x[0]; d.v = x[1]; d.w = x[2];
     }
-    p.x = V.src_pos[3 * s]; p.y = V.src_pos[3 * s + 1]; p.z = V.src_pos[3 * s + 2];
-    p.u = d0; p.v = d1; p.w = d2;
-    p.E = E; p.wt = 1.f; p.t = 0.f;
-    p.cell = V.src_cell[s];
+    return d;
+}
+
+__device__ __forceinline__ void place_source(const EvTables &V, const SrcDraw &d, PState &p)
+{
+    p.x = V.src_pos[3 * d.s]; p.y = V.src_pos[3 * d.s + 1]; p.z = V.src_pos[3 * d.s + 2];
+    p.u = d.u; p.v = d.v; p.w = d.w;
+    p.E = d.E; p.wt = 1.f; p.t = 0.f;
+    p.cell = V.src_cell[d.s];
     p.surf = -1;
-    p.g = V.src_group[s];
+    p.g = V.src_group[d.s];
     p.id = 0u;
     p.ev = 0u;
     p.prob = 0;
+}
+
+__device__ __forceinline__ void sample_source(const EvTables &V, uint64_t seed, uint64_t hist, PState &p)
+{
+    place_source(V, draw_source(V, seed, hist), p);
 }
 
 // ---------------------------------------------------------------------------
@@ -1637,8 +1656,67 @@ __device__ __noinline__ int comb_stack(OvfP *stk, int sp, int teeth, uint64_t se
 // holds only the CTA's tally sums.  A history's row is the thread's own, so
 // it is folded when the thread finishes the history.
 
+// Multigroup histories are short (a few events), so starting them is a large
+// part of the work, and at a lane's own time it runs for the few idle lanes
+// of its warp.  There a warp draws sources 32 at a time, all lanes together,
+// into a ring in shared memory, and an idle lane only reads one (30-group deep
+// slab, 10^8 histories: 15.88 -> 15.25 ms; 256 uneven shields: 24.1 -> 23.2 ms;
+// continuous-energy histories are long and gain nothing).
+// Towards the end of the histories a warp draws only what it needs, so that
+// none waits in a ring while another warp is idle.
+struct __align__(16) SrcSlot {
+    SrcDraw d;
+    int prob;
+    unsigned long long hist;
+};
+constexpr int kRing = 64;             // slots per warp: one refill of 32 on top of what is left
+struct SrcRing {
+    SrcSlot slot[kRing];
+    unsigned long long last;          // histories handed out when this warp last took some
+    uint32_t pos;                     // next slot to read
+    int left;
+};
+
+template <bool kBatch>
+__device__ __noinline__ void ring_draw(const EvTables &V0, const EvArgs &A, unsigned long long gi, SrcSlot &slot)
+{
+    int prob = 0;
+    unsigned long long hist = A.first + gi;
+    if (kBatch) {
+        prob = problem_of(A, gi);
+        hist = gi - A.prefix[prob];
+    }
+    slot.d = draw_source(kBatch ? A.tabs[prob] : V0, kBatch ? A.seeds[prob] : A.seed, hist);
+    slot.prob = prob;
+    slot.hist = hist;
+}
+
+// makes at least `want` sources available if the histories last; all lanes
+template <bool kBatch>
+__device__ __forceinline__ void ring_fill(const EvTables &V0, const EvArgs &A, SrcRing &Q, int want)
+{
+    const int lane = threadIdx.x & 31;
+    const int left = Q.left;
+    if (left >= want) return;
+    const uint32_t pos = Q.pos;
+    const unsigned long long guard = 4ull * gridDim.x * kTrackBlock;
+    const int take = Q.last + guard < A.n ? 32 : want - left;
+    unsigned long long base = 0;
+    if (lane == 0) base = atomicAdd(A.next, (unsigned long long)take);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    const int got = base >= A.n ? 0 : (int)min((unsigned long long)take, A.n - base);
+    if (lane < got) ring_draw<kBatch>(V0, A, base + lane, Q.slot[(pos + left + lane) % kRing]);
+    __syncwarp();
+    if (lane == 0) {
+        Q.last = base;
+        Q.left = left + got;
+    }
+    __syncwarp();
+}
+
 template <int MinB, bool kBatch, int kFl>
-__global__ void __launch_bounds__(kTrackBlock, MinB) k_track(const EvTables V0, const EvArgs A)
+__global__ void __launch_bounds__(kTrackBlock, MinB) k_track(const __grid_constant__ EvTables V0,
+                                                             const __grid_constant__ EvArgs A)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int s_status;
@@ -1665,6 +1743,14 @@ __global__ void __launch_bounds__(kTrackBlock, MinB) k_track(const EvTables V0, 
     if (A.smem_sums) {
         for (int b = threadIdx.x; b < 2 * V0.n_bins; b += blockDim.x) C.T.ssum()[b] = 0.0;
         if constexpr (kFl == FL_MG) C.T.lane_bin()[threadIdx.x] = -1;
+    }
+    constexpr bool kRinged = kFl == FL_MG;
+    __shared__ SrcRing s_ring[kRinged ? kTrackBlock / 32 : 1];
+    SrcRing &Q = s_ring[kRinged ? threadIdx.x / 32 : 0];
+    if (kRinged && threadIdx.x % 32 == 0) {
+        Q.last = 0;
+        Q.pos = 0;
+        Q.left = 0;
     }
     if (threadIdx.x == 0) s_status = 0;
     __syncthreads();
@@ -1719,7 +1805,8 @@ __global__ void __launch_bounds__(kTrackBlock, MinB) k_track(const EvTables V0, 
         const bool idle = !have && !exhausted;
         const unsigned im = __ballot_sync(0xffffffffu, idle);
         const bool refill = __popc(im) >= A.refill_min || __ballot_sync(0xffffffffu, have) == 0u;
-        if (refill && !have && open) {
+        const bool ends = refill && !have && open;
+        if (ends) {
             history_fold<kFl, !kBatch>(C, hslot, prob);
             open = false;
         }
@@ -1732,7 +1819,36 @@ __global__ void __launch_bounds__(kTrackBlock, MinB) k_track(const EvTables V0, 
         // slower: 8 at a time ran a batch of 4096 uneven shields in 498 ms
         // against 378 ms.)
         const unsigned m = __ballot_sync(0xffffffffu, need);
-        if (m) {
+        if constexpr (kRinged) {
+            if (m) {
+                const int want = __popc(m), r = __popc(m & ((1u << lane) - 1u));
+                ring_fill<kBatch>(V0, A, Q, want);
+                const int left = Q.left;
+                const uint32_t pos = Q.pos;
+                if (need) {
+                    if (r >= left) {
+                        exhausted = true;
+                    } else {
+                        const SrcSlot &q = Q.slot[(pos + r) % kRing];
+                        hist = q.hist;
+                        prob = kBatch ? q.prob : 0;
+                        place_source(tab(prob), q.d, p);
+                        p.hslot = hslot;
+                        p.prob = prob;
+                        have = true;
+                        open = true;
+                        walks = 1;
+                        C.cnt[C_PART]++;
+                    }
+                }
+                __syncwarp();
+                if (lane == 0) {
+                    Q.pos = (pos + min(want, left)) % kRing;
+                    Q.left = left - min(want, left);
+                }
+                __syncwarp();
+            }
+        } else if (m) {
             const int leader = __ffs(m) - 1;
             unsigned long long base = 0;
             if (lane == leader) base = atomicAdd(A.next, (unsigned long long)__popc(m));
