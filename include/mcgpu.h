@@ -85,7 +85,8 @@ typedef struct {
     uint32_t blocks_per_sm;  /* event mode: resident CTAs per SM, which sets the
                                 register budget: 2, 3 or 4 for the tile kernel
                                 (256 threads), 4, 6, 7 or 8 for the per-thread
-                                kernel (128 threads); 0 = tuned / 4 / 8 */
+                                kernel (128 threads); 0 = tuned / 4 / by the
+                                history count */
     uint32_t kernel;         /* event mode: 1 = particle tile with event queues,
                                 2 = one particle per thread, 3 = event kernels
                                 over an HBM particle bank, 0 = tuned / 2; the
@@ -98,8 +99,7 @@ typedef struct {
     uint32_t refill;         /* per-thread event kernel: a lane that finished its
                                 history waits until this many lanes of its warp
                                 are idle, so that they fold and start histories
-                                together (1..32; 0 = 8 for multigroup problems,
-                                4 otherwise) */
+                                together (1..32; 0 = 4) */
 } mc_tune;
 
 /* Event counters and timing of the last mc_run.  The counts follow the
@@ -120,9 +120,10 @@ typedef struct {
     double   fold_ms;         /* device time of the history fold */
     double   total_ms;        /* device time of the whole mc_run */
     uint32_t launches;        /* kernels launched by the last mc_run (mixed
-                                 mode: 2 where a second kernel adds the
-                                 replicated sums of a problem of more than
-                                 4096 bins, or of a batch) */
+                                 mode: 2 where a second kernel adds
+                                 replicated sums: a batch, a problem of more
+                                 than 4096 bins, a long run that is not
+                                 multigroup) */
     uint32_t reserved;        /* 0 (pads the struct to 8 bytes) */
 } mc_counters;
 

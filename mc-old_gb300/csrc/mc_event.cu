@@ -60,7 +60,7 @@ struct EventState {
     int grid = 0, block = 0, tile = 0, ovf_cap = 0;
     size_t smem = 0;
     bool rows_dirty = true;
-    // a problem whose sums do not fit in shared memory: replicas of its
+    // a problem whose sums do not live in shared memory: replicas of its
     // sums ([2][n_rep][n_bins]) and what k_batch_reduce reads for one
     // problem (the sums' pointers, rep_off = {0, n_bins}, rep_prob = 0)
     DevBuf rep, rep_meta;
@@ -203,17 +203,30 @@ struct EvLaunch {
     int flavor = FL_ALL;    // per-thread kernel flavour (FL_ALL / FL_CE / FL_MG)
     uint32_t max_events = kMaxEvents;
     int refill = 1;         // k_track: idle lanes a warp gathers before it starts histories
+    bool smem_sums = false; // the CTA's tally sums live in shared memory (else in replicas, EvArgs::n_rep)
     size_t smem = 0;
 };
 
+// From this many histories on, the per-thread kernel of continuous-energy and
+// mixed problems folds into replicated sums in L2 instead of its CTA's shared
+// memory.  A shared-memory FP64 addition is a compare-and-swap loop: k lanes
+// that end histories with the same bin make k rounds of 19 SM cycles each
+// (614 cycles for a full warp, measured), where a reduction to L2 takes the
+// SM 10 cycles and no round.  One-group slab, 1,000,000 histories: 3.29 ->
+// 2.72 ms; shield, 10,000,000: 78.7 -> 76.8 ms.  Below, the second kernel that
+// adds the replicas costs more (shield of 20,000: +0.01 ms); the multigroup
+// kernel keeps a running sum per thread instead, which is faster still (deep
+// slab 15.4 against 15.7 ms).
+constexpr uint64_t kReplicaHistories = 65536;
+
 static mc_status event_launch_shape(const DeviceProblem &d, const mc_tune *tune, const mc_tune &tuned,
-                                    long long nb_smem, bool batch, int flavor, int comb_teeth, EvLaunch &L,
+                                    long long nb, uint64_t n, bool batch, int flavor, int comb_teeth, EvLaunch &L,
                                     std::string &err)
 {
     L.flavor = flavor;
-    // measured: 4 idle lanes for continuous-energy histories (~115 events),
-    // 8 for the short multigroup ones
-    const int refill_default = flavor == FL_MG ? 8 : 4;
+    // measured at 2 / 4 / 8: shield 77.2 / 76.8 / 78.6 ms, deep slab 15.4 /
+    // 15.5 / 16.1 ms, 256 shields 22.6 / 22.3 / 23.7 ms
+    const int refill_default = 4;
     L.refill = (tune && tune->refill) ? (int)tune->refill : (tuned.refill ? (int)tuned.refill : refill_default);
     if (L.refill < 1 || L.refill > 32) { err = "refill must be 1..32"; return MC_ERR_ARG; }
     L.kernel = (tune && tune->kernel) ? (int)tune->kernel : (tuned.kernel ? (int)tuned.kernel : 2);
@@ -253,9 +266,17 @@ static mc_status event_launch_shape(const DeviceProblem &d, const mc_tune *tune,
         return MC_ERR_ARG;
     }
     const bool own_minb = tune && tune->blocks_per_sm;
+    // the per-thread kernel's CTAs per SM: no more than give every history a
+    // lane, as fewer CTAs leave a thread more registers (shield of 20,000
+    // histories: 0.87 ms at 4, 0.94 at 6, 1.05 at 8); a full GPU runs 8, or 7
+    // where the batch kernel spills at 8 (256 shields: 22.2 against 23.2 ms)
+    int minb_default = 4;
+    if (L.kernel == 2) {
+        const uint64_t lanes = (uint64_t)std::max(d.sms, 1) * kTrackBlock;
+        minb_default = n <= 4 * lanes ? 4 : (n <= 6 * lanes ? 6 : ((n <= 7 * lanes || batch) ? 7 : 8));
+    }
     L.minb = own_minb ? (int)tune->blocks_per_sm
-           : ((tuned.blocks_per_sm && tuned.kernel == (uint32_t)L.kernel) ? (int)tuned.blocks_per_sm
-                                                                          : (L.kernel == 2 ? 8 : 4));
+           : ((tuned.blocks_per_sm && tuned.kernel == (uint32_t)L.kernel) ? (int)tuned.blocks_per_sm : minb_default);
     if (L.kernel == 2 ? !(L.minb == 4 || L.minb == 6 || L.minb == 7 || L.minb == 8) : (L.minb < 2 || L.minb > 4)) {
         err = L.kernel == 2 ? "blocks_per_sm must be 4, 6, 7 or 8 for the per-thread kernel"
                             : "blocks_per_sm must be 2, 3 or 4 for the tile kernel";
@@ -275,8 +296,9 @@ static mc_status event_launch_shape(const DeviceProblem &d, const mc_tune *tune,
         L.ovf_cap = kTrackBlock * depth;
         // the per-CTA sums, then (multigroup, with them) every thread's
         // running sums of its register bin and that bin
-        L.smem = sizeof(double) * 2 * (size_t)nb_smem + 64;
-        if (nb_smem > 0 && flavor == FL_MG) L.smem += kTrackBlock * (2 * sizeof(double) + sizeof(int));
+        L.smem_sums = nb > 0 && nb <= 4096 && (flavor == FL_MG || n < kReplicaHistories);
+        L.smem = sizeof(double) * 2 * (size_t)(L.smem_sums ? nb : 0) + 64;
+        if (L.smem_sums && flavor == FL_MG) L.smem += kTrackBlock * (2 * sizeof(double) + sizeof(int));
     } else {
         L.tile = (tune && tune->bank_capacity) ? (int)tune->bank_capacity
                : (tuned.bank_capacity ? (int)tuned.bank_capacity : 512);
@@ -292,7 +314,8 @@ static mc_status event_launch_shape(const DeviceProblem &d, const mc_tune *tune,
             err = "stack_depth (the tile kernel's overflow bank) must be 1..2^20";
             return MC_ERR_ARG;
         }
-        L.smem = tile_smem_bytes(L.tile, nb_smem);
+        L.smem_sums = nb > 0 && nb <= 4096;
+        L.smem = tile_smem_bytes(L.tile, L.smem_sums ? nb : 0);
     }
     EvKernel k = pick_kernel(L.minb, batch, L.kernel, L.flavor);
     cudaError_t e;
@@ -345,8 +368,8 @@ static void fill_counters(mc_counters &L, const unsigned long long *cnt)
     L.nuc_lookups = cnt[8];
 }
 
-// Replicas of a single problem's sums when they do not fit in shared
-// memory (see EvArgs::n_rep); fills A's replica fields.
+// Replicas of a single problem's sums where they do not live in shared
+// memory (see EvArgs::n_rep, kReplicaHistories); fills A's replica fields.
 static mc_status single_replicas(EventState &S, const DeviceProblem &d, long long nb, EvArgs &A,
                                  const int *&rep_prob, std::string &err)
 {
@@ -363,11 +386,11 @@ static mc_status single_replicas(EventState &S, const DeviceProblem &d, long lon
         S.rep_stride = nb;
         S.rep_dirty = true;
     }
-    // the sums' pointers and rep_off = {0, nb} in the first 256 bytes, then rep_prob = 0
-    struct { double *ps, *pq; long long off[2]; } h{d.d_sum, d.d_sq, {0, nb}};
     char *m = static_cast<char *>(S.rep_meta.ptr);
-    cudaMemcpyAsync(m, &h, sizeof(h), cudaMemcpyHostToDevice, d.stream);
     if (S.rep_dirty) {
+        // the sums' pointers and rep_off = {0, nb} in the first 256 bytes, then rep_prob = 0
+        struct { double *ps, *pq; long long off[2]; } h{d.d_sum, d.d_sq, {0, nb}};
+        cudaMemcpyAsync(m, &h, sizeof(h), cudaMemcpyHostToDevice, d.stream);
         cudaMemsetAsync(m + 256, 0, (size_t)nb * sizeof(int), d.stream);
         cudaMemsetAsync(S.rep.ptr, 0, rep_bytes, d.stream);
         S.rep_dirty = false;
@@ -390,11 +413,10 @@ mc_status run_event(const Tables &t, DeviceProblem &d, uint64_t first, uint64_t 
     EventState &S = *d.ev_state;
     const EvTables &V = S.dv;
     const long long nb = std::max<long long>(V.n_bins, 1);
-    const bool smem_sums = nb <= 4096;
     EvLaunch L;
     const int comb = t.comb_teeth > 0 ? t.comb_teeth : 0;
     const int flavor = (V.has_time || comb) ? FL_ALL : (V.G > 0 ? FL_MG : FL_CE);
-    mc_status st = event_launch_shape(d, tune, d.tuned, smem_sums ? nb : 0, false, flavor, comb, L, err);
+    mc_status st = event_launch_shape(d, tune, d.tuned, nb, n, false, flavor, comb, L, err);
     if (st != MC_OK) return st;
     if (L.kernel == 3) {
         mc_tune bt = tune ? *tune : mc_tune{};
@@ -430,11 +452,11 @@ mc_status run_event(const Tables &t, DeviceProblem &d, uint64_t first, uint64_t 
     A.sum = d.d_sum;
     A.sq = d.d_sq;
     A.tile = L.tile;
-    A.smem_sums = smem_sums ? 1 : 0;
+    A.smem_sums = L.smem_sums ? 1 : 0;
     A.refill_min = L.refill;
     A.n_prob = 0;
     const int *d_rep_prob = nullptr;
-    if (!smem_sums && (st = single_replicas(S, d, nb, A, d_rep_prob, err)) != MC_OK) return st;
+    if (!L.smem_sums && (st = single_replicas(S, d, nb, A, d_rep_prob, err)) != MC_OK) return st;
     cudaEventRecord(d.ev[0], d.stream);
     pick_kernel(L.minb, false, L.kernel, L.flavor)<<<L.grid, L.block, L.smem, d.stream>>>(V, A);
     cudaError_t e;
@@ -614,7 +636,7 @@ mc_status batch_run(BatchState *b, int device_sms, uint64_t seed, const mc_tune 
     DeviceProblem shape_dev;
     shape_dev.sms = device_sms;
     EvLaunch L;
-    mc_status st = event_launch_shape(shape_dev, tune, tuned, 0, true, b->flavor, b->comb_teeth, L, err);
+    mc_status st = event_launch_shape(shape_dev, tune, tuned, 0, b->total, true, b->flavor, b->comb_teeth, L, err);
     if (st != MC_OK) return st;
     if ((st = event_scratch(b->scratch, b->stream, L.grid, L.tile, L.ovf_cap, b->row_nb, err)) != MC_OK) return st;
     L.max_events = (tune && tune->max_events) ? tune->max_events : kMaxEvents;
