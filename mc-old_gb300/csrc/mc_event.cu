@@ -67,6 +67,7 @@ struct EventState {
     int n_rep = 0;
     long long rep_stride = 0;
     bool rep_dirty = false;
+    const double *rep_sum = nullptr, *rep_sq = nullptr;   // the sums rep_meta points to
 };
 
 void event_state_free(EventState *s)
@@ -387,10 +388,14 @@ static mc_status single_replicas(EventState &S, const DeviceProblem &d, long lon
         S.rep_dirty = true;
     }
     char *m = static_cast<char *>(S.rep_meta.ptr);
-    if (S.rep_dirty) {
+    if (S.rep_dirty || S.rep_sum != d.d_sum || S.rep_sq != d.d_sq) {   // (autotuning folds into scratch sums)
         // the sums' pointers and rep_off = {0, nb} in the first 256 bytes, then rep_prob = 0
         struct { double *ps, *pq; long long off[2]; } h{d.d_sum, d.d_sq, {0, nb}};
         cudaMemcpyAsync(m, &h, sizeof(h), cudaMemcpyHostToDevice, d.stream);
+        S.rep_sum = d.d_sum;
+        S.rep_sq = d.d_sq;
+    }
+    if (S.rep_dirty) {
         cudaMemsetAsync(m + 256, 0, (size_t)nb * sizeof(int), d.stream);
         cudaMemsetAsync(S.rep.ptr, 0, rep_bytes, d.stream);
         S.rep_dirty = false;
