@@ -238,15 +238,15 @@ mc_status mc_tally_read(const mc_problem *p, uint32_t est, double *mean, double 
     const int64_t b0 = p->t.est_bin_off[est], b1 = p->t.est_bin_off[est + 1];
     const uint64_t nb = (uint64_t)(b1 - b0);
     if (cap < nb && (mean || sigma || sum || sumsq)) return MC_ERR_ARG;
-    std::vector<double> s, q;
     std::string err;
-    mc_status st = read_sums(p->dev, s, q, err);
+    mc_status st = read_bins(p->dev, (size_t)b0, (size_t)nb, err);
     if (st != MC_OK) { const_cast<mc_problem *>(p)->err = err; return st; }
+    const double *s = reinterpret_cast<const double *>(p->dev.h_stage + kCtlBytes), *q = s + nb;
     // Estimator::end_cycle / end_simulation for one active cycle
     // (Estimator.cpp:347-367) with N = histories folded so far
     const double N = (double)p->dev.histories;
     for (uint64_t j = 0; j < nb; ++j) {
-        const double sv = s[b0 + j], qv = q[b0 + j];
+        const double sv = s[j], qv = q[j];
         const double m = sv / N;
         const double us = (qv / N - m * m) / (N - 1.0);
         if (mean) mean[j] = (0.0 + m) / 1.0;

@@ -249,9 +249,7 @@ mc_status mc_batch_reset(mc_batch *b)
     mc_status st = batch_quiesce(b);
     if (st != MC_OK) return st;
     const cudaStream_t s = batch_stream(b->state);
-    cudaError_t e = cudaSuccess;
-    for (mc_problem *p : b->probs)
-        if ((e = reset_tallies_async(p->dev, s)) != cudaSuccess) break;
+    cudaError_t e = batch_clear(b->state);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) { b->err = cuda_msg(e, "batch reset"); return MC_ERR_CUDA; }
     return MC_OK;
@@ -270,41 +268,29 @@ mc_status mc_batch_tally_read(mc_batch *b, double *mean, double *sigma, double *
     }
     mc_status st = batch_quiesce(b);
     if (st != MC_OK) return st;
-    if (b->stage_doubles < 2 * total) {
+    const uint64_t stride = std::max<uint64_t>(total, 1);
+    if (b->stage_doubles < 2 * stride) {
         if (b->h_stage) cudaFreeHost(b->h_stage);
         b->h_stage = nullptr;
         b->stage_doubles = 0;
-        if (cudaHostAlloc(&b->h_stage, std::max<size_t>(2 * total, 1) * sizeof(double), cudaHostAllocDefault) !=
-            cudaSuccess) {
+        if (cudaHostAlloc(&b->h_stage, 2 * stride * sizeof(double), cudaHostAllocDefault) != cudaSuccess) {
             cudaGetLastError();
             b->err = "cannot allocate the batch's read-back buffer";
             return MC_ERR_NOMEM;
         }
-        b->stage_doubles = 2 * total;
+        b->stage_doubles = 2 * stride;
     }
-    const cudaStream_t s = batch_stream(b->state);
-    cudaError_t e = cudaSuccess;
-    uint64_t off = 0;
-    for (mc_problem *p : b->probs) {
-        const size_t nb = (size_t)std::max<long long>(p->dev.dt.n_bins, 0);
-        if (nb == 0) continue;
-        if ((e = cudaMemcpyAsync(b->h_stage + off, p->dev.d_sum, nb * sizeof(double), cudaMemcpyDeviceToHost, s)) !=
-                cudaSuccess ||
-            (e = cudaMemcpyAsync(b->h_stage + total + off, p->dev.d_sq, nb * sizeof(double),
-                                 cudaMemcpyDeviceToHost, s)) != cudaSuccess)
-            break;
-        off += nb;
-    }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    cudaError_t e = batch_gather(b->state, b->h_stage);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(batch_stream(b->state));
     if (e != cudaSuccess) { b->err = cuda_msg(e, "batch tally read"); return MC_ERR_CUDA; }
+    uint64_t off = 0;
     // per problem, the statistics of mc_tally_read (Estimator.cpp:347-367)
     // over that problem's histories
-    off = 0;
     for (mc_problem *p : b->probs) {
         const uint64_t nb = (uint64_t)std::max<long long>(p->dev.dt.n_bins, 0);
         const double N = (double)p->dev.histories;
         for (uint64_t j = 0; j < nb; ++j) {
-            const double sv = b->h_stage[off + j], qv = b->h_stage[total + off + j];
+            const double sv = b->h_stage[off + j], qv = b->h_stage[stride + off + j];
             const double m = sv / N;
             const double us = (qv / N - m * m) / (N - 1.0);
             if (mean) mean[off + j] = (0.0 + m) / 1.0;

@@ -122,6 +122,7 @@ mc_status device_problem_init(const Tables &t, DeviceProblem &d, std::string &er
         return MC_ERR_CUDA;
     }
     for (auto &ev : d.ev) cudaEventCreate(&ev);
+    cudaEventCreate(&d.ev_end);
 
     DevTables &T = d.dt;
     T.n_surf = t.n_surf(); T.n_cell = t.n_cell(); T.n_mat = t.n_mat(); T.n_nuc = t.n_nuc();
@@ -159,22 +160,26 @@ mc_status device_problem_init(const Tables &t, DeviceProblem &d, std::string &er
 
     d.blob_bytes = P.buf.size();
     if ((e = cudaMalloc(&d.blob, d.blob_bytes)) != cudaSuccess) { err = cuda_msg(e, "cudaMalloc(tables)"); return MC_ERR_NOMEM; }
-    if ((e = cudaHostAlloc(&d.h_blob, d.blob_bytes, cudaHostAllocDefault)) != cudaSuccess) {
+    const size_t nb = (size_t)std::max<int64_t>(t.n_bins(), 1);
+    const size_t stage = (d.blob_bytes + 255) & ~(size_t)255;
+    if ((e = cudaHostAlloc(&d.h_blob, stage + kCtlBytes + 2 * nb * sizeof(double), cudaHostAllocDefault)) != cudaSuccess) {
         err = cuda_msg(e, "cudaHostAlloc(tables)");
         return MC_ERR_NOMEM;
     }
+    d.h_stage = static_cast<char *>(d.h_blob) + stage;
     std::memcpy(d.h_blob, P.buf.data(), d.blob_bytes);
     for (auto &f : P.fix) *f.first = static_cast<const char *>(d.blob) + f.second;
     mc_status us = upload_tables(d, err);
     if (us != MC_OK) return us;
 
-    const size_t nb = (size_t)std::max<int64_t>(t.n_bins(), 1);
-    if ((e = cudaMalloc(&d.d_sum, nb * sizeof(double))) != cudaSuccess ||
-        (e = cudaMalloc(&d.d_sq, nb * sizeof(double))) != cudaSuccess ||
-        (e = cudaMalloc(&d.d_exact, nb * 2 * kExactLimbs * sizeof(long long))) != cudaSuccess) {
+    d.tally_bytes = nb * (2 * sizeof(double) + 2 * kExactLimbs * sizeof(long long));
+    if ((e = cudaMalloc(&d.tallies, d.tally_bytes)) != cudaSuccess) {
         err = cuda_msg(e, "cudaMalloc(tallies)");
         return MC_ERR_NOMEM;
     }
+    d.d_sum = static_cast<double *>(d.tallies);
+    d.d_sq = d.d_sum + nb;
+    d.d_exact = reinterpret_cast<long long *>(d.d_sq + nb);
     d.ready = true;
     return reset_tallies(d, err);
 }
@@ -191,10 +196,9 @@ void device_problem_free(DeviceProblem &d)
     devbuf_free(d.hist); devbuf_free(d.stack); devbuf_free(d.digest); devbuf_free(d.misc);
     if (d.blob) cudaFree(d.blob);
     if (d.h_blob) cudaFreeHost(d.h_blob);
-    if (d.d_sum) cudaFree(d.d_sum);
-    if (d.d_sq) cudaFree(d.d_sq);
-    if (d.d_exact) cudaFree(d.d_exact);
+    if (d.tallies) cudaFree(d.tallies);
     for (auto &ev : d.ev) if (ev) cudaEventDestroy(ev);
+    if (d.ev_end) cudaEventDestroy(d.ev_end);
     if (d.stream) cudaStreamDestroy(d.stream);
     d = DeviceProblem();
 }
@@ -217,47 +221,53 @@ cudaError_t upload_tables_async(DeviceProblem &d, cudaStream_t st)
 
 cudaError_t reset_tallies_async(DeviceProblem &d, cudaStream_t st)
 {
-    const size_t nb = (size_t)std::max<long long>(d.dt.n_bins, 1);
-    cudaError_t e;
-    if ((e = cudaMemsetAsync(d.d_sum, 0, nb * sizeof(double), st)) != cudaSuccess ||
-        (e = cudaMemsetAsync(d.d_sq, 0, nb * sizeof(double), st)) != cudaSuccess ||
-        (e = cudaMemsetAsync(d.d_exact, 0, nb * 2 * kExactLimbs * sizeof(long long), st)) != cudaSuccess)
-        return e;
+    const cudaError_t e = cudaMemsetAsync(d.tallies, 0, d.tally_bytes, st);
+    if (e != cudaSuccess) return e;
+    tallies_were_reset(d);
+    return cudaSuccess;
+}
+
+void tallies_were_reset(DeviceProblem &d)
+{
     d.exact_valid = true;
     d.histories = 0;
     d.ntrack = 0;
-    return cudaSuccess;
 }
 
 mc_status reset_tallies(DeviceProblem &d, std::string &err)
 {
-    const size_t nb = (size_t)std::max<long long>(d.dt.n_bins, 1);
-    cudaError_t e;
-    if ((e = cudaMemsetAsync(d.d_sum, 0, nb * sizeof(double), d.stream)) != cudaSuccess ||
-        (e = cudaMemsetAsync(d.d_sq, 0, nb * sizeof(double), d.stream)) != cudaSuccess ||
-        (e = cudaMemsetAsync(d.d_exact, 0, nb * 2 * kExactLimbs * sizeof(long long), d.stream)) != cudaSuccess ||
-        (e = cudaStreamSynchronize(d.stream)) != cudaSuccess) {
+    cudaError_t e = reset_tallies_async(d, d.stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(d.stream);
+    if (e != cudaSuccess) {
         err = cuda_msg(e, "reset tallies");
         return MC_ERR_CUDA;
     }
-    d.exact_valid = true;
-    d.histories = 0;
-    d.ntrack = 0;
+    return MC_OK;
+}
+
+mc_status read_bins(const DeviceProblem &d, size_t from, size_t count, std::string &err)
+{
+    if (count == 0) return MC_OK;
+    if (!d.tallies) { err = "read tallies: problem was not loaded"; return MC_ERR_CUDA; }
+    const size_t pitch = (size_t)((const char *)d.d_sq - (const char *)d.d_sum), width = count * sizeof(double);
+    cudaError_t e;
+    if ((e = cudaMemcpy2DAsync(d.h_stage + kCtlBytes, width, d.d_sum + from, pitch, width, 2, cudaMemcpyDeviceToHost,
+                               d.stream)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(d.stream)) != cudaSuccess) {
+        err = cuda_msg(e, "read tallies");
+        return MC_ERR_CUDA;
+    }
     return MC_OK;
 }
 
 mc_status read_sums(const DeviceProblem &d, std::vector<double> &sum, std::vector<double> &sq, std::string &err)
 {
     const size_t nb = (size_t)std::max<long long>(d.dt.n_bins, 1);
-    sum.assign(nb, 0.0);
-    sq.assign(nb, 0.0);
-    cudaError_t e;
-    if ((e = cudaStreamSynchronize(d.stream)) != cudaSuccess ||
-        (e = cudaMemcpy(sum.data(), d.d_sum, nb * sizeof(double), cudaMemcpyDeviceToHost)) != cudaSuccess ||
-        (e = cudaMemcpy(sq.data(), d.d_sq, nb * sizeof(double), cudaMemcpyDeviceToHost)) != cudaSuccess) {
-        err = cuda_msg(e, "read tallies");
-        return MC_ERR_CUDA;
-    }
+    const mc_status st = read_bins(d, 0, nb, err);
+    if (st != MC_OK) return st;
+    const double *h = reinterpret_cast<const double *>(d.h_stage + kCtlBytes);
+    sum.assign(h, h + nb);
+    sq.assign(h + nb, h + 2 * nb);
     return MC_OK;
 }
 
@@ -292,17 +302,17 @@ mc_status run_fp64(const Tables &t, DeviceProblem &d, uint64_t first, uint64_t n
     const uint64_t ld = hist_rows(chunk);
     if (!devbuf_reserve(d.hist, (size_t)ld * nb * sizeof(double)) ||
         !devbuf_reserve(d.stack, (size_t)threads * depth * fp64_particle_bytes()) ||
-        !devbuf_reserve(d.misc, 256 + kNumCounters * sizeof(unsigned long long) + 64) ||
+        !devbuf_reserve(d.misc, kCtlBytes) ||
         (want_digest && !devbuf_reserve(d.digest, (size_t)chunk * sizeof(uint64_t)))) {
         err = "cannot allocate FP64 scratch";
         return MC_ERR_NOMEM;
     }
     char *misc = static_cast<char *>(d.misc.ptr);
-    unsigned long long *d_cnt = reinterpret_cast<unsigned long long *>(misc);
-    int *d_status = reinterpret_cast<int *>(misc + kNumCounters * sizeof(unsigned long long));
-    unsigned int *d_next = reinterpret_cast<unsigned int *>(misc + kNumCounters * sizeof(unsigned long long) + 16);
+    unsigned long long *d_cnt = reinterpret_cast<unsigned long long *>(misc + kCtlCounters);
+    int *d_status = reinterpret_cast<int *>(misc + kCtlStatus);
+    unsigned int *d_next = reinterpret_cast<unsigned int *>(misc + kCtlNext);
     cudaError_t e;
-    if ((e = cudaMemsetAsync(misc, 0, 256 + kNumCounters * sizeof(unsigned long long), d.stream)) != cudaSuccess) {
+    if ((e = cudaMemsetAsync(misc, 0, kCtlBytes, d.stream)) != cudaSuccess) {
         err = cuda_msg(e, "memset");
         return MC_ERR_CUDA;
     }
@@ -332,7 +342,7 @@ mc_status run_fp64(const Tables &t, DeviceProblem &d, uint64_t first, uint64_t n
         A.status = d_status;
         A.next = d_next;
         A.lanes = shape.lanes;
-        cudaMemsetAsync(d_next, 0, sizeof(unsigned int), d.stream);
+        if (c0 > 0) cudaMemsetAsync(d_next, 0, sizeof(unsigned int), d.stream);
         cudaEventRecord(d.ev[1], d.stream);
         if ((e = launch_history_fp64(d.dt, A, replay, grid, block, d.stream)) != cudaSuccess) {
             err = cuda_msg(e, "history kernel launch");
@@ -360,8 +370,16 @@ mc_status run_fp64(const Tables &t, DeviceProblem &d, uint64_t first, uint64_t n
         if (want_digest) {
             cudaMemcpyAsync(d.digests.data() + c0, A.digest, cn * sizeof(uint64_t), cudaMemcpyDeviceToHost, d.stream);
         }
-        int hs = 0;
-        if ((e = cudaMemcpyAsync(&hs, d_status, sizeof(int), cudaMemcpyDeviceToHost, d.stream)) != cudaSuccess ||
+        const bool last = c0 + chunk >= n;
+        if (last) {
+            if ((e = launch_exact_normalize(d.d_exact, d.dt.n_bins, d.stream)) != cudaSuccess) {
+                err = cuda_msg(e, "exact sums");
+                return MC_ERR_CUDA;
+            }
+            ++launches;
+            cudaEventRecord(d.ev_end, d.stream);
+        }
+        if ((e = cudaMemcpyAsync(d.h_stage, misc, kCtlBytes, cudaMemcpyDeviceToHost, d.stream)) != cudaSuccess ||
             (e = cudaStreamSynchronize(d.stream)) != cudaSuccess) {
             err = cuda_msg(e, "history kernel");
             return MC_ERR_CUDA;
@@ -371,26 +389,18 @@ mc_status run_fp64(const Tables &t, DeviceProblem &d, uint64_t first, uint64_t n
         cudaEventElapsedTime(&b, d.ev[2], d.ev[3]);
         t_transport += a;
         t_fold += b;
+        int hs = 0;
+        std::memcpy(&hs, d.h_stage + kCtlStatus, sizeof(hs));
         if (hs != DS_OK) {
             err = device_status_text(hs);
             if (hs == DS_OVERFLOW) err += " (raise mc_tune.stack_depth)";
             return status_from_device(hs);
         }
     }
-    if ((e = launch_exact_normalize(d.d_exact, d.dt.n_bins, d.stream)) != cudaSuccess) {
-        err = cuda_msg(e, "exact sums");
-        return MC_ERR_CUDA;
-    }
-    ++launches;
     float total = 0.f;
-    cudaEventRecord(d.ev[3], d.stream);
-    cudaStreamSynchronize(d.stream);
-    cudaEventElapsedTime(&total, d.ev[0], d.ev[3]);
+    cudaEventElapsedTime(&total, d.ev[0], d.ev_end);
     unsigned long long cnt[kNumCounters];
-    if ((e = cudaMemcpy(cnt, d_cnt, sizeof(cnt), cudaMemcpyDeviceToHost)) != cudaSuccess) {
-        err = cuda_msg(e, "counters");
-        return MC_ERR_CUDA;
-    }
+    std::memcpy(cnt, d.h_stage + kCtlCounters, sizeof(cnt));
     mc_counters &L = d.last;
     L.flights = cnt[0]; L.collisions = cnt[1]; L.crossings = cnt[2]; L.tally_updates = cnt[3];
     L.particles = cnt[4]; L.splits = cnt[5]; L.xs_evals = cnt[6]; L.freegas_iters = cnt[7];

@@ -19,6 +19,10 @@ struct DevBuf {
     size_t bytes = 0;
 };
 
+// Control words of a run, read back as one copy: counters from kCtlCounters
+// on, the device status and the history counter.
+constexpr size_t kCtlBytes = 256, kCtlNext = 0, kCtlStatus = 8, kCtlCounters = 64;
+
 struct EventState;   // mixed-precision event engine (mc_event.cu)
 struct BankState;    // its event-split engine over an HBM particle bank (mc_bank.cu)
 struct EvTables;     // the mixed-precision engine's FP32 tables (mc_evtables.h)
@@ -29,13 +33,17 @@ struct DeviceProblem {
     int device = 0;
     int sms = 0;
     cudaStream_t stream = nullptr;
-    cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
+    cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr}, ev_end = nullptr;
     void *blob = nullptr;          // every problem table, one allocation
-    void *h_blob = nullptr;        // pinned host copy of blob
+    void *h_blob = nullptr;        // pinned host copy of blob, then h_stage
     size_t blob_bytes = 0;
     DevTables dt{};
+    // pinned: kCtlBytes for a run's control words, then [2][n_bins] for tallies
+    char *h_stage = nullptr;
+    void *tallies = nullptr;       // d_sum, d_sq and d_exact, one allocation (cleared as one)
+    size_t tally_bytes = 0;
     double *d_sum = nullptr;       // [n_bins] sum of history totals
-    double *d_sq = nullptr;        // [n_bins] sum of squared history totals
+    double *d_sq = nullptr;        // [n_bins] sum of squared history totals, right behind d_sum
     long long *d_exact = nullptr;  // [n_bins][2][kExactLimbs] exact sums of the FP64 runs
     bool exact_valid = true;       // every run since the last reset added to d_exact
     uint64_t histories = 0;        // histories folded into d_sum / d_sq
@@ -61,7 +69,11 @@ mc_status upload_tables(DeviceProblem &d, std::string &err);
 // the same on a caller's stream, without waiting (batches queue many problems)
 cudaError_t upload_tables_async(DeviceProblem &d, cudaStream_t st);
 cudaError_t reset_tallies_async(DeviceProblem &d, cudaStream_t st);
+void tallies_were_reset(DeviceProblem &d);   // the host's side of a reset
 cudaError_t event_tables_upload_async(DeviceProblem &d, cudaStream_t st);
+// bins [from, from + count) of d_sum and d_sq into the handle's pinned stage
+// (sums, then squares); one copy, one wait
+mc_status read_bins(const DeviceProblem &d, size_t from, size_t count, std::string &err);
 mc_status read_sums(const DeviceProblem &d, std::vector<double> &sum, std::vector<double> &sq, std::string &err);
 mc_status run_histories(const Tables &t, DeviceProblem &d, uint64_t first, uint64_t n, uint64_t seed,
                         mc_mode mode, const mc_tune *tune, std::string &err);
@@ -95,6 +107,10 @@ mc_status batch_create(const std::vector<const Tables *> &tabs, const std::vecto
                        const uint64_t *hist, const std::vector<double *> *sums_to, BatchState **out,
                        std::string &err);
 cudaStream_t batch_stream(const BatchState *b);
+// on the batch's stream, without waiting: every problem's tallies to zero;
+// every problem's sums, then squares, to host ([2][total bins, at least 1], pinned)
+cudaError_t batch_clear(BatchState *b);
+cudaError_t batch_gather(BatchState *b, double *host);
 mc_status batch_run(BatchState *b, int device_sms, uint64_t seed, const mc_tune *tune, const mc_tune &tuned,
                     std::string &err);
 void batch_state_free(BatchState *b);
