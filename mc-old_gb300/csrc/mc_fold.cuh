@@ -19,12 +19,12 @@
 // them where a signed sum keeps wandering about zero), and the scan goes on
 // behind them.  Every result bit is the serial chain's.
 //
-// Bound and measure (GB300, 500,000 histories x 19 bins, replay of the
-// 16-layer one-group slab): the serial chain, one thread per bin, took
-// 61.5 ms (123 ns per history: one addition's latency for each of sum and
-// sum of squares plus one load round trip per 8 histories); this kernel
-// 0.86 ms (barriers and shuffles of the scan between steps).  A column is
-// contiguous, so a thread's 8 histories are four 16-byte loads.
+// Bound and measure (GB300): the latency of the steps of the densest column
+// (barriers, shuffles, 64-bit shifts).  500,000 histories x 19 bins: 61.5 ms as
+// one serial chain per bin, 0.87 ms here; 50,000 x 931 derivative columns,
+// signed and mostly zero: 7.75 -> 0.9 ms; 3,001 x 180: 0.47 -> 0.12 ms.  (With
+// 512 threads, zeros left in and a step that fails redone from memory these
+// were 0.86, 2.9 and 0.40 ms.)
 #pragma once
 
 #include <cstdint>
@@ -33,13 +33,12 @@
 
 namespace mc {
 
-constexpr int kFoldThreads = 512;
+constexpr int kFoldThreads = 256;
 constexpr int kFoldValues = 8;    // consecutive histories per thread and step
-// after kFoldStreak failing steps in a row, the values of kFoldRun threads
-// are added serially at once: a step that places 8 histories costs about as
-// much as 40 serial additions
-constexpr int kFoldStreak = 8;
-constexpr int kFoldRun = 64;
+// Where a step fails, the values of this many threads are added serially: two
+// at first, more when steps fail one after the other (a sum that starts from
+// zero, or a signed one that wanders about it).
+__host__ __device__ constexpr int fold_run(int streak) { return streak < 3 ? 2 : (streak < 12 ? 16 : 64); }
 
 // inc[0], inc[1]: what the histories so far add to k if it starts even / odd
 struct FoldMap {
@@ -82,22 +81,30 @@ __device__ __noinline__ FoldMap fold_map(const double (&v)[kFoldValues], int es,
 
 // One chain: block (bin, which), which = 0 the sum of the column's values,
 // 1 the sum of their squares.  hist is [bins][ld], ld a multiple of 8 and at
-// least n, zero from n on.
+// least n, zero from n on.  Adding zero changes nothing, and most histories
+// score few bins, so the column's nonzero values go through a ring in shared
+// memory and every step scans kStep of them.
 __global__ void __launch_bounds__(kFoldThreads) k_fold_ordered(const double *__restrict__ hist, uint32_t n,
                                                                uint64_t ld, double *__restrict__ sum,
                                                                double *__restrict__ sq)
 {
-    __shared__ FoldMap s_warp[kFoldThreads / 32];
+    constexpr uint32_t kStep = (uint32_t)kFoldThreads * kFoldValues, kRing = 2 * kStep;
+    constexpr int kWarps = kFoldThreads / 32;
+    __shared__ double s_ring[kRing + kRing / 8];   // 9 doubles for 8: a thread's values miss its neighbours' banks
+    __shared__ FoldMap s_warp[kWarps];
+    __shared__ int s_count[kWarps];
     __shared__ double s_run;      // the running sum before the current step
-    __shared__ int s_fail;        // first thread whose histories need the serial chain
+    __shared__ int s_fail;        // first thread whose values need the serial chain
     __shared__ FoldMap s_total;
-    __shared__ double s_v[kFoldRun * kFoldValues];
     const long long bin = blockIdx.x;
     const bool squares = blockIdx.y != 0;
     double *dst = (squares ? sq : sum) + bin;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    constexpr uint32_t kStep = (uint32_t)kFoldThreads * kFoldValues;
     const double *col = hist + (uint64_t)bin * ld;
+    auto slot = [&](uint32_t i) -> double & {
+        i &= kRing - 1;
+        return s_ring[i + (i >> 3)];
+    };
     double nxt[kFoldValues];
     auto fetch = [&](uint64_t pos) {
         const uint64_t h = pos + (uint64_t)t * kFoldValues;   // a multiple of 8, as ld
@@ -111,22 +118,53 @@ __global__ void __launch_bounds__(kFoldThreads) k_fold_ordered(const double *__r
     };
     if (t == 0) s_run = *dst;
     uint64_t pos = 0;
+    uint32_t head = 0, count = 0;   // the ring's first value and how many it holds
     int streak = 0;
     fetch(0);
-    while (pos < n) {
+    for (;;) {
+        while (count < kStep && pos < n) {
+            double w[kFoldValues];
+            int nz = 0;
+#pragma unroll
+            for (int j = 0; j < kFoldValues; ++j) {
+                w[j] = nxt[j];
+                nz += (dbits(w[j]) << 1) != 0 ? 1 : 0;
+            }
+            pos += kStep;
+            fetch(pos);             // the next histories, while these are placed
+            int at = nz;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int p = __shfl_up_sync(0xffffffffu, at, o);
+                if (lane >= o) at += p;
+            }
+            if (lane == 31) s_count[warp] = at;
+            at -= nz;
+            __syncthreads();
+            int total = 0;
+#pragma unroll
+            for (int i = 0; i < kWarps; ++i) {
+                if (i < warp) at += s_count[i];
+                total += s_count[i];
+            }
+            uint32_t i = head + count + (uint32_t)at;
+#pragma unroll
+            for (int j = 0; j < kFoldValues; ++j)
+                if ((dbits(w[j]) << 1) != 0) slot(i++) = w[j];
+            count += (uint32_t)total;
+            __syncthreads();
+        }
+        if (count == 0) break;
+        const uint32_t have = min(count, kStep);
         double v[kFoldValues];
         bool any = false;
 #pragma unroll
         for (int j = 0; j < kFoldValues; ++j) {
-            v[j] = nxt[j];
-            any = any || (dbits(v[j]) << 1) != 0;   // integer test: an FP64 compare costs 19 SM cycles a warp
+            const uint32_t i = (uint32_t)t * kFoldValues + j;
+            v[j] = i < have ? slot(head + i) : 0.0;
+            any = any || i < have;
         }
-        fetch(pos + kStep);       // the next step's histories, if this one goes through
-        if (!__syncthreads_or(any)) {   // adding zeros changes nothing
-            pos += kStep;
-            continue;
-        }
-        if (squares) {
+        if (squares && any) {
 #pragma unroll
             for (int j = 0; j < kFoldValues; ++j) v[j] = v[j] * v[j];
         }
@@ -207,33 +245,28 @@ __global__ void __launch_bounds__(kFoldThreads) k_fold_ordered(const double *__r
         __syncthreads();
         const int fail = s_fail;
         const uint64_t keep = sb & 0xFFF0000000000000ull;   // sign and exponent of the running sum
+        uint32_t taken = have;
         if (fail == kFoldThreads) {
             if (t == 0) {
                 const long long kn = k + ((k & 1) ? s_total.a1 : s_total.a0);
                 s_run = scannable ? dfrom(keep | ((uint64_t)kn & 0x000FFFFFFFFFFFFFull)) : s_run;
             }
-            pos += kStep;
             streak = 0;
         } else {
-            const int run = min(++streak >= kFoldStreak ? kFoldRun : 1, kFoldThreads - fail);
-            if (t > fail && t < fail + run) {
-#pragma unroll
-                for (int j = 0; j < kFoldValues; ++j) s_v[(t - fail) * kFoldValues + j] = v[j];
-            }
-            if (run > 1) __syncthreads();
+            const uint32_t first = (uint32_t)fail * kFoldValues;
+            taken = min(have, first + (uint32_t)fold_run(++streak) * kFoldValues);
             if (t == fail) {
                 double s = scannable ? dfrom(keep | ((uint64_t)k0 & 0x000FFFFFFFFFFFFFull)) : s_run;
-#pragma unroll
-                for (int j = 0; j < kFoldValues; ++j) s += v[j];
-                for (int j = kFoldValues; j < run * kFoldValues; ++j) {
-                    const double x = s_v[j];
-                    if ((dbits(x) << 1) != 0) s += x;
+#pragma unroll 8
+                for (uint32_t i = first; i < taken; ++i) {
+                    const double x = slot(head + i);
+                    s += squares ? x * x : x;
                 }
                 s_run = s;
             }
-            pos += (uint64_t)(fail + run) * kFoldValues;
-            fetch(pos);
         }
+        head += taken;
+        count -= taken;
         __syncthreads();
     }
     if (t == 0) *dst = s_run;
