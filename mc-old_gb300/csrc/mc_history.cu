@@ -1067,47 +1067,109 @@ __device__ __noinline__ void particle_comb(const Ctx &C, Lane &P, uint32_t walke
     for (int k = 0; k < teeth; ++k) C.stack[k].id = child_id(walker, kCombEvent, (uint32_t)(k + 1));
 }
 
-// Source.cpp:20-24, 42-45 and Distribution.cpp:30-33, 78-96
+// Source.cpp:20-24, 42-45 and Distribution.cpp:30-33, 78-96: the source point
+// and the sampled direction and energy
+struct SrcDraw64 {
+    double u, v, w, E, speed;
+    int s;
+};
+
 template <bool R>
-__device__ __forceinline__ void sample_source(const DevTables &T, Lane &P)
+__device__ __forceinline__ SrcDraw64 draw_source(const DevTables &T, Draws &rng)
 {
-    const double xi = u01_bits(P.rng.next());
+    SrcDraw64 o;
+    const double xi = u01_bits(rng.next());
     int s = bsearch_d(xi, T.src_cdf, T.n_src + 1);
     s = s < 0 ? 0 : (s >= T.n_src ? T.n_src - 1 : s);
+    o.s = s;
     const double *ep = T.src_e_par + 2 * s;
     // the compiled reference samples the energy before the direction
-    const double E = (T.src_e_kind[s] == 1) ? ep[0] + u01_bits(P.rng.next()) * ep[1] : ep[0];
+    o.E = (T.src_e_kind[s] == 1) ? ep[0] + u01_bits(rng.next()) * ep[1] : ep[0];
     const double *dp = T.src_dir_par + 9 * s;
     const int dk = T.src_dir_kind[s];
     if (dk == 0) {
-        P.u = dp[0]; P.v = dp[1]; P.w = dp[2];
+        o.u = dp[0]; o.v = dp[1]; o.w = dp[2];
     } else if (dk == 1 || dk == 3) {
-        const uint64_t vm = P.rng.next();
+        const uint64_t vm = rng.next();
         const double mu = (dk == 1) ? mu_bits(vm) : u01_bits(vm);
-        const uint64_t va = P.rng.next();
+        const uint64_t va = rng.next();
         const double c = fsqrt(1.0 - mu * mu);
         double sn, cs;
         Fn<R>::sincos(kPi2 * u01_bits(va), va, sn, cs);
-        P.v = cs * c;
-        P.w = sn * c;
-        P.u = mu;
+        o.v = cs * c;
+        o.w = sn * c;
+        o.u = mu;
     } else {
         double d[3];
 #pragma unroll
         for (int k = 2; k >= 0; --k) {   // z component first, as compiled
             const double *q = dp + 3 * k;
-            d[k] = ((int)q[0] == 1) ? q[1] + u01_bits(P.rng.next()) * q[2] : q[1];
+            d[k] = ((int)q[0] == 1) ? q[1] + u01_bits(rng.next()) * q[2] : q[1];
         }
-        P.u = d[0]; P.v = d[1]; P.w = d[2];
+        o.u = d[0]; o.v = d[1]; o.w = d[2];
     }
-    P.x = T.src_pos[3 * s]; P.y = T.src_pos[3 * s + 1]; P.z = T.src_pos[3 * s + 2];
-    P.t = 0.0; P.t_old = 0.0; P.wgt = 1.0;
-    P.cell = T.src_cell[s];
-    P.surf_old = -1;
     // Particle::setEnergy (Particle.cpp:42-47)
-    P.E = E;
-    P.speed = 13831.5926439 * fsqrt(E) * 100.0;
-    P.g = T.src_group[s];
+    o.speed = 13831.5926439 * fsqrt(o.E) * 100.0;
+    return o;
+}
+
+__device__ __forceinline__ void place_source(const DevTables &T, const SrcDraw64 &o, Lane &P)
+{
+    P.x = T.src_pos[3 * o.s]; P.y = T.src_pos[3 * o.s + 1]; P.z = T.src_pos[3 * o.s + 2];
+    P.u = o.u; P.v = o.v; P.w = o.w;
+    P.t = 0.0; P.t_old = 0.0; P.wgt = 1.0;
+    P.cell = T.src_cell[o.s];
+    P.surf_old = -1;
+    P.E = o.E;
+    P.speed = o.speed;
+    P.g = T.src_group[o.s];
+}
+
+// Multigroup histories last a few events, and a source costs some 70 FP64
+// instructions: a warp draws 32 of them together into a ring in shared memory
+// and its idle lanes read one each (2,000,000 deep-slab histories: 4.89 -> 4.15
+// ms).  While histories run out
+// a warp draws only what it needs.
+struct SrcSlot64 {
+    SrcDraw64 o;
+    unsigned hl;               // history of the chunk
+};
+constexpr int kRing = 64;
+struct SrcRing64 {
+    SrcSlot64 slot[kRing];
+    unsigned last, pos;        // histories handed out when this warp last took some; next slot to read
+    int left;
+};
+
+template <bool R>
+__device__ __noinline__ void ring_draw(const DevTables &T, const HistoryArgs &A, unsigned hl, SrcSlot64 &slot)
+{
+    Draws rng;
+    rng.init(A.seed, A.first + hl);
+    slot.o = draw_source<R>(T, rng);
+    slot.hl = hl;
+}
+
+// makes `want` sources available if the histories last; all lanes
+template <bool R>
+__device__ __forceinline__ void ring_fill(const DevTables &T, const HistoryArgs &A, SrcRing64 &Q, int want)
+{
+    const int lane = threadIdx.x & 31, left = Q.left;
+    if (left >= want) return;
+    const unsigned pos = Q.pos;
+    const bool far = (uint64_t)Q.last + 4ull * gridDim.x * kBlock < A.n;
+    const int take = far ? 32 : want - left;
+    unsigned base = 0;
+    if (lane == 0) base = atomicAdd(A.next, (unsigned)take);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    const int got = base >= A.n ? 0 : (int)min((unsigned)take, A.n - base);
+    if (lane < got) ring_draw<R>(T, A, base + lane, Q.slot[(pos + left + lane) % kRing]);
+    __syncwarp();
+    if (lane == 0) {
+        Q.last = base;
+        Q.left = left + got;
+    }
+    __syncwarp();
 }
 
 // The advance (general.cpp:40-83, 177-200): collision or crossing?  The
@@ -1169,8 +1231,10 @@ __device__ __forceinline__ int next_surface(const DevTables &T, Lane &P, int m, 
 // a warp makes a collision step when this many quarters of its working lanes
 // stand before a collision, or none of them can advance
 constexpr int kCollideQuarters = 3;
-// idle lanes that take new histories together, while others have work
-constexpr int kRefillLanes = 4;
+// idle lanes that take new histories together, while others have work (deep
+// slab 4.17 / 4.16 / 4.19 / 4.15 ms at 1 / 2 / 4 / 8 from a ring, 16-layer slab
+// 3.89 / 3.79 / 3.64 / 3.64; shield 33.3 / 33.3 / 33.8 ms at 2 / 4 / 8)
+constexpr int kRefillLanes = 4, kRefillRinged = 8;
 
 // CTAs per SM: registers allow 3 for continuous energy (168 a thread; at 128
 // the spills cost more than a fourth CTA gives while histories run out: 13.8
@@ -1198,6 +1262,11 @@ __global__ void __launch_bounds__(kBlock, ctas_per_sm(F)) k_history_fp64(const _
     P.gi = 0;
     P.visited = 0;
     for (int i = 0; i < kNumCounters; ++i) P.cnt[i] = 0;
+    constexpr bool kRinged = F != F_CE;
+    __shared__ SrcRing64 s_ring[kRinged ? kBlock / 32 : 1];
+    SrcRing64 &Q = s_ring[kRinged ? threadIdx.x / 32 : 0];
+    if (kRinged && lane == 0) { Q.last = 0; Q.pos = 0; Q.left = 0; }
+    __syncwarp();
     const bool digests = A.digest != nullptr;
     bool have = false, open = false, exhausted = lane >= A.lanes;
     int at_collision = 0;                  // the particle stands before a collision
@@ -1250,31 +1319,56 @@ __global__ void __launch_bounds__(kBlock, ctas_per_sm(F)) k_history_fp64(const _
         const unsigned adv = __ballot_sync(0xffffffffu, have && !at_collision);
         const unsigned col = __ballot_sync(0xffffffffu, have && at_collision);
         if ((idle | adv | col) == 0u) break;
-        if (idle && (__popc(idle) >= kRefillLanes || (adv | col) == 0u)) {
-            unsigned base = 0;
-            const int leader = __ffs(idle) - 1;
-            if (lane == leader) base = atomicAdd(A.next, (unsigned)__popc(idle));
-            base = __shfl_sync(0xffffffffu, base, leader);
-            if ((idle >> lane) & 1u) {
-                hl = base + (unsigned)__popc(idle & ((1u << lane) - 1u));
-                if (hl >= A.n) {
-                    exhausted = true;
-                } else {
-                    P.hist = A.hist + hl;
+        if (idle && (__popc(idle) >= (kRinged ? kRefillRinged : kRefillLanes) || (adv | col) == 0u)) {
+            const bool need = (idle >> lane) & 1u;
+            const int r = __popc(idle & ((1u << lane) - 1u)), want = __popc(idle);
+            SrcDraw64 o;
+            bool got = false;
+            if constexpr (kRinged) {
+                ring_fill<R>(T, A, Q, want);
+                const int left = Q.left;
+                const unsigned pos = Q.pos;
+                got = need && r < left;
+                if (got) {
+                    const SrcSlot64 &q = Q.slot[(pos + r) % kRing];
+                    o = q.o;
+                    hl = q.hl;
                     P.rng.init(A.seed, A.first + hl);
-                    P.digest = 0xCBF29CE484222325ULL;
-                    sample_source<R>(T, P);
-                    P.sp = 0;
-                    P.visited = 0;
-                    P.xm = -2;
-                    P.gid = -1;
-                    P.rng.start(0);
-                    P.cnt[C_PART]++;
-                    if (digests) dig(P, 0xA5A5A5A5ULL);
-                    walks = 1;
-                    have = open = true;
-                    at_collision = 0;
                 }
+                __syncwarp();
+                if (lane == 0) {
+                    Q.pos = (pos + min(want, left)) % kRing;
+                    Q.left = left - min(want, left);
+                }
+                __syncwarp();
+            } else {
+                unsigned base = 0;
+                const int leader = __ffs(idle) - 1;
+                if (lane == leader) base = atomicAdd(A.next, (unsigned)want);
+                base = __shfl_sync(0xffffffffu, base, leader);
+                got = need && base + (unsigned)r < A.n;
+                if (got) {
+                    hl = base + (unsigned)r;
+                    P.rng.init(A.seed, A.first + hl);
+                    o = draw_source<R>(T, P.rng);
+                }
+            }
+            if (got) {
+                place_source(T, o, P);
+                P.hist = A.hist + hl;
+                P.digest = 0xCBF29CE484222325ULL;
+                P.sp = 0;
+                P.visited = 0;
+                P.xm = -2;
+                P.gid = -1;
+                P.rng.start(0);
+                P.cnt[C_PART]++;
+                if (digests) dig(P, 0xA5A5A5A5ULL);
+                walks = 1;
+                have = open = true;
+                at_collision = 0;
+            } else if (need) {
+                exhausted = true;
             }
             continue;
         }
