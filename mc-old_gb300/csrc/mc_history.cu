@@ -19,10 +19,9 @@
 //   * One flat loop instead of a walk per history: a lane whose particle died
 //     takes its next one while the others go on (nested loops ran with 11 of
 //     32 lanes active: a warp waited for its longest walk).
-//   * Two kinds of steps, chosen per warp: an advance (decide between
-//     collision and crossing, and cross), which is cheap, and a collision,
-//     which is most of the FP64 work.  Lanes at a collision wait until most
-//     of the warp's are, or no lane can advance.
+//   * Steps chosen per warp: an advance (decide between collision and
+//     crossing, almost without FP64), else the crossings or the collisions
+//     that wait, once enough lanes do.
 //   * What only decides something is bounded in FP32 first, and in FP64 where
 //     the bounds cannot tell: whether the particle reaches a surface before
 //     its collision, the sign of a surface's equation in the cell search, the
@@ -1173,12 +1172,12 @@ __device__ __forceinline__ void ring_fill(const DevTables &T, const HistoryArgs 
 }
 
 // The advance (general.cpp:40-83, 177-200): collision or crossing?  The
-// exponential distance and the surface distances are bounded in FP32; the one
-// that decides is computed in FP64 (the collision's by the collision step),
-// and all of them where the bounds overlap.  Returns the surface the particle
-// crosses, its distance in `dist`; -1 for a collision, -2 on an error.
+// exponential distance and the surface distances are bounded in FP32, and
+// computed in FP64 where the bounds overlap.  Returns the surface the particle
+// crosses, -1 for a collision, -2 on an error; the flight's length is computed
+// by the step that makes it.
 template <bool R, int F>
-__device__ __forceinline__ int next_surface(const DevTables &T, Lane &P, int m, double &dist)
+__device__ __forceinline__ int next_surface(const DevTables &T, Lane &P, int m)
 {
     float clo = 0.9f * FLT_MAX, chi = clo;
     if (m >= 0) {
@@ -1208,13 +1207,10 @@ __device__ __forceinline__ int next_surface(const DevTables &T, Lane &P, int m, 
             }
         }
         if (chi < fminf(near_lo, other_lo)) return -1;
-        if (minhi < clo && minhi < other_lo) {
-            dist = surface_distance(T, S, P.x, P.y, P.z, P.u, P.v, P.w);
-            return S;
-        }
+        if (minhi < clo && minhi < other_lo) return S;
     }
     // the reference's own order and comparisons
-    dist = kMaxF;
+    double dist = kMaxF;
     S = -1;
 #pragma unroll 1
     for (int i = i0; i < i1; ++i) {
@@ -1228,9 +1224,21 @@ __device__ __forceinline__ int next_surface(const DevTables &T, Lane &P, int m, 
     return S;
 }
 
-// a warp makes a collision step when this many quarters of its working lanes
-// stand before a collision, or none of them can advance
-constexpr int kCollideQuarters = 3;
+// What a particle does next.
+enum { AT_FLIGHT = 0, AT_COLLISION, AT_SURFACE };
+
+// When to make the crossings that wait.  A crossing step costs the warp X FP64
+// instructions for however many lanes, a collision step C; with a crossings
+// arriving per collision step, waiting for k of them costs a X / k for the
+// steps and (k - 1) / 64 C for the lanes that wait meanwhile, least at
+// k^2 = 64 a X / C; a is counted, and 64 X / C about 20 for multigroup
+// collisions and 8 for continuous energy.  Measured at a half / once / twice
+// that: 16-layer slab 3.25 / 3.31 / 3.56 ms, deep slab 3.66 / 3.64 / 3.75 ms,
+// 100,000 duct histories 14.9 / 15.2 / 15.6 ms (crossings with every advance:
+// 3.63, 4.15 and 15.1 ms).  A warp that was given few lanes is bound by its
+// longest history and waits for none.
+template <int F> constexpr uint32_t kCrossCost = F == F_CE ? 4u : 12u;
+
 // idle lanes that take new histories together, while others have work (deep
 // slab 4.17 / 4.16 / 4.19 / 4.15 ms at 1 / 2 / 4 / 8 from a ring, 16-layer slab
 // 3.89 / 3.79 / 3.64 / 3.64; shield 33.3 / 33.3 / 33.8 ms at 2 / 4 / 8)
@@ -1269,7 +1277,9 @@ __global__ void __launch_bounds__(kBlock, ctas_per_sm(F)) k_history_fp64(const _
     __syncwarp();
     const bool digests = A.digest != nullptr;
     bool have = false, open = false, exhausted = lane >= A.lanes;
-    int at_collision = 0;                  // the particle stands before a collision
+    int stage = AT_FLIGHT, sx = -1;        // what the particle does next; the surface it will cross
+    uint32_t n_cross = 0, n_collide = 1;   // the warp's crossings and collision steps of late
+    const uint32_t cross_cost = A.lanes == 32 ? kCrossCost<F> : 0u;
     uint32_t walks = 0;
     unsigned hl = 0;
     for (;;) {
@@ -1316,10 +1326,11 @@ __global__ void __launch_bounds__(kBlock, ctas_per_sm(F)) k_history_fp64(const _
             }
         }
         const unsigned idle = __ballot_sync(0xffffffffu, !have && !exhausted);
-        const unsigned adv = __ballot_sync(0xffffffffu, have && !at_collision);
-        const unsigned col = __ballot_sync(0xffffffffu, have && at_collision);
-        if ((idle | adv | col) == 0u) break;
-        if (idle && (__popc(idle) >= (kRinged ? kRefillRinged : kRefillLanes) || (adv | col) == 0u)) {
+        const unsigned adv = __ballot_sync(0xffffffffu, have && stage == AT_FLIGHT);
+        const unsigned col = __ballot_sync(0xffffffffu, have && stage == AT_COLLISION);
+        const unsigned crs = __ballot_sync(0xffffffffu, have && stage == AT_SURFACE);
+        if ((idle | adv | col | crs) == 0u) break;
+        if (idle && (__popc(idle) >= (kRinged ? kRefillRinged : kRefillLanes) || (adv | col | crs) == 0u)) {
             const bool need = (idle >> lane) & 1u;
             const int r = __popc(idle & ((1u << lane) - 1u)), want = __popc(idle);
             SrcDraw64 o;
@@ -1366,31 +1377,41 @@ __global__ void __launch_bounds__(kBlock, ctas_per_sm(F)) k_history_fp64(const _
                 if (digests) dig(P, 0xA5A5A5A5ULL);
                 walks = 1;
                 have = open = true;
-                at_collision = 0;
+                stage = AT_FLIGHT;
             } else if (need) {
                 exhausted = true;
             }
             continue;
         }
-        // one step of the warp: an advance, or a collision
-        const bool colliding = !(adv && 4 * __popc(col) < kCollideQuarters * __popc(adv | col));
-        const bool act = have && (at_collision != 0) == colliding;
-        const int m = act ? T.cell_mat[P.cell] : -1, cell_old = P.cell;
-        int s = -2;                        // the surface to cross, -1 for a collision
-        bool moves = false;
-        double dist = kMaxFLess;
-        if (!colliding) {
-            if (act) {
+        // one step of the warp: an advance, else a crossing or a collision
+        if (adv) {
+            if (have && stage == AT_FLIGHT) {
                 P.rng.start(P.rng.event + 1);
+                sx = -2;
                 if (P.rng.event > A.max_events) P.status = DS_TIMEOUT;   // bounded walk
-                else s = next_surface<R, F>(T, P, m, dist);
-                at_collision = s == -1;
-                moves = s >= 0;
+                else sx = next_surface<R, F>(T, P, T.cell_mat[P.cell]);
+                stage = sx == -1 ? AT_COLLISION : AT_SURFACE;
+                if (P.status != DS_OK) have = false;
             }
-        } else if (act) {
-            at_collision = 0;
-            moves = true;
-            if (m >= 0) {
+            __syncwarp();
+            continue;
+        }
+        const int nx = __popc(crs);
+        const bool colliding = nx == 0 || (col != 0u && (uint32_t)(nx * nx) * n_collide < cross_cost * n_cross);
+        if (colliding) ++n_collide;
+        else n_cross += (uint32_t)nx;
+        if (n_collide > 1024u || n_cross > 16384u) {
+            n_collide = (n_collide + 1u) / 2u;
+            n_cross /= 2u;
+        }
+        const bool moves = have && stage == (colliding ? AT_COLLISION : AT_SURFACE);
+        const int m = moves ? T.cell_mat[P.cell] : -1, cell_old = P.cell, s = sx;
+        double dist = kMaxFLess;
+        if (moves) {
+            stage = AT_FLIGHT;
+            if (!colliding) {
+                dist = surface_distance(T, s, P.x, P.y, P.z, P.u, P.v, P.w);
+            } else if (m >= 0) {
                 const double L0 = -Fn<R>::log(u01_bits(P.rng.first()));
                 if constexpr (F != F_CE) dist = div_by(L0, P.xT, T.mg[m * T.mg_groups + P.g].inv_T);
                 else dist = fdiv(L0, P.xT);
