@@ -325,15 +325,16 @@ struct XsAt { int m, i; float f; };   // material, global grid index, fraction
 // around it ({Sigma_t, Sigma_s, Sigma_c, E} each), and a bounded walk fixes
 // the rare bracket miss.  Below the grid the first row's values hold, above
 // it the last row's (the fraction is clamped), as XSTable::xs does.
-struct XsVal { XsAt at; float st, ss, sc; };
+struct XsVal { XsAt at; float st, ss, sc; int n_nuc; };   // n_nuc: nuclides of the material
 
 __device__ __forceinline__ XsVal xs_eval(const EvTables &V, int m, float E)
 {
-    const int off = V.mgrid_off[m], L = V.mgrid_len[m];
+    const int4 ra = __ldg(V.mat_rec + 2 * m), rb = __ldg(V.mat_rec + 2 * m + 1);
+    const int off = ra.x, L = ra.y;
     const float4 *row = V.xrow + off;
-    int b = (int)((__log2f(E) - V.bkt_lo[m]) * V.bkt_inv[m]);
-    b = b < 0 ? 0 : (b >= V.bkt_n[m] ? V.bkt_n[m] - 1 : b);
-    int i = __ldg(V.bkt + V.bkt_off[m] + b);
+    int b = (int)((__log2f(E) - __int_as_float(rb.x)) * __int_as_float(rb.y));
+    b = b < 0 ? 0 : (b >= ra.w ? ra.w - 1 : b);
+    int i = __ldg(V.bkt + ra.z + b);
     i = i > L - 2 ? L - 2 : i;
     float4 r0 = __ldg(row + i), r1 = __ldg(row + i + 1);
     while (i > 0 && r0.w > E) { --i; r1 = r0; r0 = __ldg(row + i); }
@@ -341,6 +342,7 @@ __device__ __forceinline__ XsVal xs_eval(const EvTables &V, int m, float E)
     float f = (E - r0.w) / (r1.w - r0.w);
     f = f < 0.f ? 0.f : (f > 1.f ? 1.f : f);
     XsVal x;
+    x.n_nuc = rb.w;
     x.at = XsAt{m, off + i, f};
     x.st = fmaf(f, r1.x - r0.x, r0.x);
     x.ss = fmaf(f, r1.y - r0.y, r0.y);
@@ -433,13 +435,13 @@ __device__ __forceinline__ float quad_root(float a, float h, float c, bool on)
     return fminf(t1, t2);
 }
 
-__device__ float surface_distance(const EvTables &V, int s, const PState &p, bool on)
+// (type and the first five coefficients from the cell's surface record)
+__device__ __forceinline__ float surface_distance(int type, const float (&k)[5], const PState &p, bool on)
 {
-    const float *k = V.surf_coef + 8 * s;
-    switch (V.surf_type[s]) {
+    switch (type) {
     case 0: case 1: case 2: {
         if (on) return kInf;
-        const int ax = V.surf_type[s];
+        const int ax = type;
         const float pos = ax == 0 ? p.x : (ax == 1 ? p.y : p.z);
         const float dir = ax == 0 ? p.u : (ax == 1 ? p.v : p.w);
         if (fabsf(dir) > kEpsF) {
@@ -502,9 +504,11 @@ __device__ void surface_reflect(const EvTables &V, int s, PState &p)
 
 __device__ __forceinline__ bool cell_contains(const EvTables &V, int c, const PState &p, int S, bool pos_side)
 {
-    for (int i = V.cell_surf_off[c]; i < V.cell_surf_off[c + 1]; ++i) {
-        const int s2 = V.cell_surf[i];
-        const int sense = V.cell_sense[i];
+    const int4 cr = __ldg(V.cell_rec + 2 * c);
+    for (int i = cr.y; i < cr.y + cr.z; ++i) {
+        const float4 sr = __ldg(V.surf_rec + 2 * i);
+        const int s2 = __float_as_int(sr.x);
+        const int sense = __float_as_int(sr.z);
         if (s2 == S) {
             if (sense != 0 && ((sense > 0) != pos_side)) return false;
             continue;
@@ -747,6 +751,36 @@ __device__ void estimator_score(Ctx &C, int e, const PState &p, float t_old, flo
             }
         }
         if (nf == 0) return;
+    }
+}
+
+// The estimators of one list of attachments; l_in and fixed as above.  Most
+// are one flux or current score in a bin that the record gives.
+template <int kFl>
+__device__ __forceinline__ void score_list(Ctx &C, const EvTables &V, const int4 *rec, int first, int count,
+                                           const PState &p, float t_old, float speed, float l_in, int fixed)
+{
+    if (count > 0 && !(fabsf(l_in) <= FLT_MAX)) {
+        atomicCAS(C.s_status, 0, DS_NAN);
+        return;
+    }
+    for (int i = first; i < first + count; ++i) {
+        const int4 r = __ldg(rec + i);
+        if (r.x < 0) continue;
+        const int code = r.y & ATT_CODES;
+        if (code == ATT_GENERAL) {
+            estimator_score<kFl>(C, r.z, p, t_old, speed, l_in, r.x, fixed);
+            continue;
+        }
+        int bin = r.x;
+        if (code == ATT_FLUX_ENERGY) {
+            const int b = bsearch_f(p.E, V.filt_grid + r.z, r.w);
+            if (b < 0 || b >= r.w - 1) continue;
+            bin += b;
+        } else if (code == ATT_FLUX_GROUP) {
+            bin += p.g;
+        }
+        tally_add<kFl>(C, p.hslot, bin, (double)((r.y & ATT_WEIGHT) ? p.wt : p.wt * l_in));
     }
 }
 
@@ -1145,7 +1179,8 @@ __device__ __forceinline__ int event_advance(Ctx &C, const EvTables &V, Rng32 &R
 #if MC_EV_RNG_OUTLINE
     R.prime();   // the event's first Philox block, inline: the event's later draws read it
 #endif
-    const int m = V.cell_mat[p.cell];
+    const int4 ca = __ldg(V.cell_rec + 2 * p.cell), cb = __ldg(V.cell_rec + 2 * p.cell + 1);
+    const int m = ca.x;
     float dcol;
     f.sig = 0.f;
     f.ss = 0.f;
@@ -1161,6 +1196,7 @@ __device__ __forceinline__ int event_advance(Ctx &C, const EvTables &V, Rng32 &R
             f.ss = x.ss;
             f.sc = x.sc;
             C.cnt[C_XS]++;
+            C.cnt[C_NUC] += (uint32_t)x.n_nuc;
         }
         dcol = -__logf(R.next()) / f.sig;
     } else {
@@ -1169,10 +1205,12 @@ __device__ __forceinline__ int event_advance(Ctx &C, const EvTables &V, Rng32 &R
     float dist = kInf;
     f.S = -1;
     f.sense = 0;
-    for (int i = V.cell_surf_off[p.cell]; i < V.cell_surf_off[p.cell + 1]; ++i) {
-        const int sf = V.cell_surf[i];
-        const float d = surface_distance(V, sf, p, sf == p.surf);
-        if (d < dist) { dist = d; f.S = sf; f.sense = V.cell_sense[i]; }
+    for (int i = ca.y; i < ca.y + ca.z; ++i) {
+        const float4 ra = __ldg(V.surf_rec + 2 * i), rb = __ldg(V.surf_rec + 2 * i + 1);
+        const int sf = __float_as_int(ra.x);
+        const float k[5] = {ra.w, rb.x, rb.y, rb.z, rb.w};
+        const float d = surface_distance(__float_as_int(ra.y), k, p, sf == p.surf);
+        if (d < dist) { dist = d; f.S = sf; f.sense = __float_as_int(ra.z); }
     }
     const bool cross = dcol > dist;
     if (cross && f.S < 0) {
@@ -1188,9 +1226,7 @@ __device__ __forceinline__ int event_advance(Ctx &C, const EvTables &V, Rng32 &R
         p.t = t_old + l / speed;
     }
     C.cnt[C_FLIGHTS]++;
-    if (m >= 0 && !is_mg<kFl>(V)) C.cnt[C_NUC] += (uint32_t)(V.mnuc_off[m + 1] - V.mnuc_off[m]);
-    for (int i = V.cell_tl_off[p.cell]; i < V.cell_tl_off[p.cell + 1]; ++i)
-        estimator_score<kFl>(C, V.cell_tl[i], p, t_old, speed, l, V.cell_tl_pre[i], 1);
+    score_list<kFl>(C, V, V.tl_rec, ca.w, cb.x, p, t_old, speed, l, 1);
     p.surf = -1;
     return cross ? 2 : 1;
 }
@@ -1213,9 +1249,8 @@ __device__ __forceinline__ int event_collide_begin(Ctx &C, const EvTables &V, Rn
     // block) need no block test, no word selection and no refill code
     R.draw = 1u;
     R.cached = 1u;
-    for (int i = V.cell_c_off[p.cell]; i < V.cell_c_off[p.cell + 1]; ++i)
-        estimator_score<kFl>(C, V.cell_c[i], p, p.t, V.has_time ? speed_of(p.E) : 0.f, 0.f,
-                                       V.cell_c_pre[i], 1);
+    const int4 cb = __ldg(V.cell_rec + 2 * p.cell + 1);
+    score_list<kFl>(C, V, V.c_rec, cb.y, cb.z, p, p.t, V.has_time ? speed_of(p.E) : 0.f, 0.f, 1);
     const float st = f.sig;
     if (is_mg<kFl>(V)) {
         const int row = m * V.G + p.g;
@@ -1248,8 +1283,10 @@ __device__ __forceinline__ int event_collide_begin(Ctx &C, const EvTables &V, Rn
     const float u = ss * R.next();
     float acc = 0.f;
     int nuc = -1;
-    for (int k = V.mnuc_off[m]; k < V.mnuc_off[m + 1]; ++k) {
-        acc += xs_at(V.nucS + V.mnuc_tab[k] - V.mgrid_off[m], a);
+    const int goff = __ldg(V.mat_rec + 2 * m).x;
+    const int4 rb = __ldg(V.mat_rec + 2 * m + 1);
+    for (int k = rb.z; k < rb.z + rb.w; ++k) {
+        acc += xs_at(V.nucS + V.mnuc_tab[k] - goff, a);
         if (acc > u) { nuc = V.mnuc_id[k]; break; }
     }
     if (nuc < 0) return 1;   // no scatter nuclide: the reference returns without scattering
@@ -1299,8 +1336,8 @@ __device__ __forceinline__ bool event_cross(Ctx &C, const EvTables &V, Rng32 &R,
     }
     if (p.wt != 0.f) {   // a vacuum boundary kills first and scores zero (general.cpp:98-111)
         const float speed = V.has_time ? speed_of(p.E) : 0.f;
-        for (int i = V.surf_est_off[S]; i < V.surf_est_off[S + 1]; ++i)
-            estimator_score<kFl>(C, V.surf_est[i], p, p.t, speed, 0.f, V.surf_est_pre[i], 0);
+        const int2 se = __ldg(V.surf_est_rec + S);
+        score_list<kFl>(C, V, V.s_rec, se.x, se.y, p, p.t, speed, 0.f, 0);
     }
     if (alive && p.cell != old_cell) {
         const float Iold = V.cell_imp[old_cell], Inew = V.cell_imp[p.cell];

@@ -66,9 +66,6 @@ bool build_event_tables(const Tables &t, EvHost &h, std::string &err)
     std::vector<float> cimp = cast<double, float>(t.cell_imp);
     P.add(cimp, &V.cell_imp);
     P.add(t.cell_mat, &V.cell_mat);
-    P.add(t.cell_surf_off, &V.cell_surf_off);
-    P.add(t.cell_surf, &V.cell_surf);
-    P.add(t.cell_sense, &V.cell_sense);
     std::vector<std::vector<int>> nb(2 * (size_t)t.n_surf());
     for (int c = 0; c < t.n_cell(); ++c)
         for (int i = t.cell_surf_off[c]; i < t.cell_surf_off[c + 1]; ++i) {
@@ -82,9 +79,6 @@ bool build_event_tables(const Tables &t, EvHost &h, std::string &err)
     }
     P.add(nb_off, &V.nb_off);
     P.add(nb_cell, &V.nb_cell);
-    P.add(t.cell_tl_off, &V.cell_tl_off); P.add(t.cell_tl, &V.cell_tl);
-    P.add(t.cell_c_off, &V.cell_c_off); P.add(t.cell_c, &V.cell_c);
-    P.add(t.surf_est_off, &V.surf_est_off); P.add(t.surf_est, &V.surf_est);
 
     // ---- estimators ----
     V.n_est = t.n_est();
@@ -137,9 +131,56 @@ bool build_event_tables(const Tables &t, EvHost &h, std::string &err)
     for (int sf = 0; sf < t.n_surf(); ++sf)
         for (int i = t.surf_est_off[sf]; i < t.surf_est_off[sf + 1]; ++i)
             s_pre[i] = fixed_part(t.surf_est[i], F_SURFACE, sf);
-    P.add(tl_pre, &V.cell_tl_pre);
-    P.add(c_pre, &V.cell_c_pre);
-    P.add(s_pre, &V.surf_est_pre);
+
+    // ---- records of cells, surfaces and attachments ----
+    auto bits = [](float x) { int i; std::memcpy(&i, &x, 4); return i; };
+    std::vector<int> cell_rec, surf_rec, surf_est_rec;
+    for (int c = 0; c < t.n_cell(); ++c) {
+        const int s0 = t.cell_surf_off[c], t0 = t.cell_tl_off[c], c0 = t.cell_c_off[c];
+        for (int x : {t.cell_mat[c], s0, t.cell_surf_off[c + 1] - s0, t0, t.cell_tl_off[c + 1] - t0, c0,
+                      t.cell_c_off[c + 1] - c0, 0})
+            cell_rec.push_back(x);
+    }
+    for (size_t i = 0; i < t.cell_surf.size(); ++i) {
+        const int sf = t.cell_surf[i];
+        const float *k = &surf_coef[8 * (size_t)sf];
+        for (int x : {sf, (int)t.surf_type[sf], (int)t.cell_sense[i], bits(k[0]), bits(k[1]), bits(k[2]), bits(k[3]),
+                      bits(k[4])})
+            surf_rec.push_back(x);
+    }
+    for (int sf = 0; sf < t.n_surf(); ++sf) {
+        surf_est_rec.push_back(t.surf_est_off[sf]);
+        surf_est_rec.push_back(t.surf_est_off[sf + 1] - t.surf_est_off[sf]);
+    }
+    auto attachments = [&](const std::vector<int32_t> &est, const std::vector<int> &pre) {
+        std::vector<int> rec;
+        for (size_t i = 0; i < est.size(); ++i) {
+            const int e = est[i], f0 = t.est_filt_off[e], nf = t.est_filt_off[e + 1] - f0, s0 = t.est_score_off[e];
+            int code = ATT_GENERAL, a = e, b = 0;
+            if (t.est_score_off[e + 1] - s0 == 1 && t.score_kind[s0] == SC_FLUX && t.score_kernel[s0] != K_C && nf <= 2) {
+                const int kind = nf == 2 ? t.filt_kind[f0 + 1] : -1;
+                if (nf == 1) code = ATT_FLUX;
+                else if (kind == F_GROUP) code = ATT_FLUX_GROUP;
+                else if (kind == F_ENERGY) code = ATT_FLUX_ENERGY;
+                if (code == ATT_FLUX_ENERGY) {
+                    a = fgo[f0 + 1];
+                    b = t.filt_grid_len[f0 + 1];
+                }
+                if (code != ATT_GENERAL && t.score_kernel[s0] == K_NEUTRON) code |= ATT_WEIGHT;
+            }
+            const bool simple = code != ATT_GENERAL;
+            for (int x : {pre[i] < 0 ? -1 : pre[i] + (simple ? ebo[e] : 0), code, a, b}) rec.push_back(x);
+        }
+        return rec;
+    };
+    const std::vector<int> tl_rec = attachments(t.cell_tl, tl_pre), c_rec = attachments(t.cell_c, c_pre),
+                           s_rec = attachments(t.surf_est, s_pre);
+    P.add(cell_rec, reinterpret_cast<const int **>(&V.cell_rec));
+    P.add(surf_rec, reinterpret_cast<const int **>(&V.surf_rec));
+    P.add(tl_rec, reinterpret_cast<const int **>(&V.tl_rec));
+    P.add(c_rec, reinterpret_cast<const int **>(&V.c_rec));
+    P.add(s_rec, reinterpret_cast<const int **>(&V.s_rec));
+    P.add(surf_est_rec, reinterpret_cast<const int **>(&V.surf_est_rec));
 
     // ---- continuous-energy materials ----
     V.n_mat = t.n_mat();
@@ -202,14 +243,18 @@ bool build_event_tables(const Tables &t, EvHost &h, std::string &err)
             }
         }
     }
-    P.add(mgrid_off, &V.mgrid_off); P.add(mgrid_len, &V.mgrid_len);
+    std::vector<int> mat_rec;
+    for (size_t m = 0; m < mgrid_off.size(); ++m)
+        for (int x : {mgrid_off[m], mgrid_len[m], bkt_off[m], bkt_n[m], bits(bkt_lo[m]), bits(bkt_inv[m]), mnuc_off[m],
+                      mnuc_off[m + 1] - mnuc_off[m]})
+            mat_rec.push_back(x);
+    P.add(mat_rec, reinterpret_cast<const int **>(&V.mat_rec));
     P.add(xrow, reinterpret_cast<const float **>(&V.xrow));
-    P.add(mnuc_off, &V.mnuc_off); P.add(mnuc_id, &V.mnuc_id); P.add(mnuc_tab, &V.mnuc_tab);
+    P.add(mnuc_id, &V.mnuc_id); P.add(mnuc_tab, &V.mnuc_tab);
     P.add(nucS, &V.nucS);
     std::vector<float> A = cast<double, float>(t.nuc_A);
     P.add(A, &V.nuc_A);
-    P.add(bkt_off, &V.bkt_off); P.add(bkt_lo, &V.bkt_lo); P.add(bkt_inv, &V.bkt_inv);
-    P.add(bkt_n, &V.bkt_n); P.add(bkt, &V.bkt);
+    P.add(bkt, &V.bkt);
 
     // ---- multigroup ----
     std::vector<float> mgT = cast<double, float>(t.mg_total), mgS = cast<double, float>(t.mg_scat_tot),

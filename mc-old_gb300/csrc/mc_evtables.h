@@ -13,11 +13,15 @@
 //    rounding.  N_k sigma_s,k per nuclide on the same grid serves the
 //    scatter-nuclide choice (Material.cpp:106-115).  A log-spaced bucket
 //    table maps log2(E) to a grid index, so no binary search is needed;
-//  * multigroup data in FP32 with cumulative scatter rows.
+//  * multigroup data in FP32 with cumulative scatter rows;
+//  * what an event reads about its cell, each of the cell's surfaces, each
+//    attached estimator and its material as records of one or two 16-byte
+//    vectors, instead of a value at a time from parallel arrays: fewer loads
+//    and address computations, and fewer of them one after the other.
 #pragma once
 
 #include <stdint.h>
-#include <vector_types.h>   // float4 (plain struct; host code builds the rows)
+#include <vector_types.h>   // float4, int4, int2 (plain structs; host code builds the rows)
 
 #include <vector>
 
@@ -25,19 +29,30 @@
 
 namespace mc {
 
+// Codes of an attachment record (AttRec::y, its low bits): the estimator takes
+// the general path, or it has one flux score and, besides the cell or surface
+// filter that the attachment fixes, no filter, an energy filter or a group
+// filter, whose index is added to the bin as it is.  ATT_WEIGHT: the score is
+// the particle's weight (a current), not weight times track length.
+enum AttCode : int { ATT_GENERAL = 0, ATT_FLUX, ATT_FLUX_ENERGY, ATT_FLUX_GROUP, ATT_CODES = 15, ATT_WEIGHT = 16 };
+
 struct EvTables {
+    // records (see above)
+    const int4 *cell_rec;             // [n_cell][2]: {material, first surface record, how many, first track-length
+                                      // record}, {how many, first collision record, how many, 0}
+    const float4 *surf_rec;           // [cell's surfaces][2]: {surface, type, sense, k0}, {k1, k2, k3, k4}
+    const int4 *tl_rec, *c_rec, *s_rec;   // per attachment: {bin or, in general, index part (-1: outside the
+                                      // filter), code, estimator or energy grid offset, grid length}
+    const int2 *surf_est_rec;         // per surface: first crossing record, how many
+    const int4 *mat_rec;              // [n_mat][2], continuous energy: {grid offset, length, bucket offset, buckets},
+                                      // {log2 E0, buckets per unit log2, first nuclide, how many}
     // geometry
     int n_surf, n_cell;
     const int *surf_type, *surf_bc;
     const float *surf_coef;           // 8 per surface
     const float *cell_imp;
-    const int *cell_mat, *cell_surf_off, *cell_surf, *cell_sense;
+    const int *cell_mat;
     const int *nb_off, *nb_cell;      // CSR over 2*n_surf lists: index 2*s + (sense > 0)
-    const int *cell_tl_off, *cell_tl, *cell_c_off, *cell_c, *surf_est_off, *surf_est;
-    // per attachment above: the part of the flattened tally index that the
-    // estimator's cell filter (track-length, collision) or surface filter
-    // (crossing) contributes, fixed by the attachment; -1 = outside the filter
-    const int *cell_tl_pre, *cell_c_pre, *surf_est_pre;
     // estimators
     int n_est;
     long long n_bins;
@@ -51,19 +66,14 @@ struct EvTables {
     int has_time;                     // a time filter exists (track time)
     // continuous-energy materials
     int n_mat;
-    const int *mgrid_off, *mgrid_len; // per material
     // union grid and macroscopic tables, one 16-byte row per grid point:
     // {Sigma_t, Sigma_s, Sigma_c, E}, so that the two rows bracketing E
     // (one 32-byte load) give the bracket check and all three values
     const float4 *xrow;
-    const int *mnuc_off;              // per material: first entry in the nuclide lists
     const int *mnuc_id;               // nuclide index (for the mass A)
     const int *mnuc_tab;              // offset of N_k sigma_s,k on the material grid
     const float *nucS;                // N_k sigma_s,k tables
     const float *nuc_A;
-    const int *bkt_off;               // per material
-    const float *bkt_lo, *bkt_inv;    // log2(E0) and buckets per unit log2
-    const int *bkt_n;
     const int *bkt;                   // grid index of the last point <= bucket start
     // multigroup
     int G;
