@@ -278,12 +278,13 @@ static mc_status event_launch_shape(const DeviceProblem &d, const mc_tune *tune,
     const bool own_minb = tune && tune->blocks_per_sm;
     // the per-thread kernel's CTAs per SM: no more than give every history a
     // lane, as fewer CTAs leave a thread more registers (shield of 20,000
-    // histories: 0.87 ms at 4, 0.94 at 6, 1.05 at 8); a full GPU runs 8, or 7
-    // where the batch kernel spills at 8 (256 shields: 22.2 against 23.2 ms)
+    // histories: 0.70 ms at 4, 0.75 at 6, 0.87 at 8); a full GPU runs 8, or 7
+    // for multigroup problems, whose kernels spill at 8 (deep slab 13.0 against
+    // 14.7 ms, a batch of 256 shields 19.5 against 23.3 ms)
     int minb_default = 4;
     if (L.kernel == 2) {
         const uint64_t lanes = (uint64_t)std::max(d.sms, 1) * kTrackBlock;
-        minb_default = n <= 4 * lanes ? 4 : (n <= 6 * lanes ? 6 : ((n <= 7 * lanes || batch) ? 7 : 8));
+        minb_default = n <= 4 * lanes ? 4 : (n <= 6 * lanes ? 6 : ((n <= 7 * lanes || flavor == FL_MG) ? 7 : 8));
     }
     L.minb = own_minb ? (int)tune->blocks_per_sm
            : ((tuned.blocks_per_sm && tuned.kernel == (uint32_t)L.kernel) ? (int)tuned.blocks_per_sm : minb_default);
