@@ -107,9 +107,9 @@ __device__ __forceinline__ void bank_ctx(Ctx &C, const EvTables &V, const EvArgs
     C.s_novf = nullptr;
     C.s_nlive = nullptr;
     C.s_nhfree = nullptr;
+    C.sectors = false;
     C.reg_mask = false;
     C.tmask = 0ull;
-    C.tmask1 = 0ull;
     C.cbin = -1;
     C.cval = 0.0;
     C.cnt.base = cnt_column(s_cnt, threadIdx.x);
@@ -184,7 +184,7 @@ __device__ __forceinline__ void bank_retire(Ctx &C, const BankArgs &B, bool dies
         if (B.may_split) __threadfence();
         if (atomicSub(&B.hlive[hslot], 1) == 1) {
             if (B.may_split) __threadfence();
-            history_fold<kFl, false>(C, hslot, 0);
+            history_fold<kFl>(C, hslot, 0);
         }
     }
 }

@@ -234,8 +234,8 @@ static mc_status event_launch_shape(const DeviceProblem &d, const mc_tune *tune,
                                     Residency &R, EvLaunch &L, std::string &err)
 {
     L.flavor = flavor;
-    // measured at 2 / 4 / 8: shield 77.2 / 76.8 / 78.6 ms, deep slab 15.4 /
-    // 15.5 / 16.1 ms, 256 shields 22.6 / 22.3 / 23.7 ms
+    // measured at 2 / 4 / 8: shield 69.3 / 67.3 / 67.9 ms, deep slab 11.7 /
+    // 11.7 / 11.9 ms, 256 shields 18.3 / 18.1 / 18.6 ms
     const int refill_default = 4;
     L.refill = (tune && tune->refill) ? (int)tune->refill : (tuned.refill ? (int)tuned.refill : refill_default);
     if (L.refill < 1 || L.refill > 32) { err = "refill must be 1..32"; return MC_ERR_ARG; }
@@ -278,13 +278,14 @@ static mc_status event_launch_shape(const DeviceProblem &d, const mc_tune *tune,
     const bool own_minb = tune && tune->blocks_per_sm;
     // the per-thread kernel's CTAs per SM: no more than give every history a
     // lane, as fewer CTAs leave a thread more registers (shield of 20,000
-    // histories: 0.70 ms at 4, 0.75 at 6, 0.87 at 8); a full GPU runs 8, or 7
-    // for multigroup problems, whose kernels spill at 8 (deep slab 13.0 against
-    // 14.7 ms, a batch of 256 shields 19.5 against 23.3 ms)
+    // histories: 0.70 ms at 4, 0.75 at 6, 0.87 at 8); a full GPU runs 8 for
+    // multigroup problems (deep slab 11.7 against 12.6 ms at 7, a batch of 256
+    // shields 18.1 against 18.6 ms), else 7, as those kernels spill at 8
+    // (shield 67.3 against 68.2 ms, one-group slab 1.67 against 1.77 ms)
     int minb_default = 4;
     if (L.kernel == 2) {
         const uint64_t lanes = (uint64_t)std::max(d.sms, 1) * kTrackBlock;
-        minb_default = n <= 4 * lanes ? 4 : (n <= 6 * lanes ? 6 : ((n <= 7 * lanes || flavor == FL_MG) ? 7 : 8));
+        minb_default = n <= 4 * lanes ? 4 : (n <= 6 * lanes ? 6 : ((n <= 7 * lanes || flavor != FL_MG) ? 7 : 8));
     }
     L.minb = own_minb ? (int)tune->blocks_per_sm
            : ((tuned.blocks_per_sm && tuned.kernel == (uint32_t)L.kernel) ? (int)tuned.blocks_per_sm : minb_default);
@@ -353,12 +354,15 @@ static mc_status event_launch_shape(const DeviceProblem &d, const mc_tune *tune,
     return MC_OK;
 }
 
+// bins of a history row: whole 32-byte sectors
+static long long row_bins(long long nb) { return (nb + 3) / 4 * 4; }
+
 static mc_status event_scratch(EventState &S, cudaStream_t st, int grid, int tile, int ovf_cap, long long row_nb,
                                std::string &err)
 {
     const int nw = (int)((row_nb + 63) / 64);
     const size_t rows = (size_t)grid * tile;
-    const size_t acc_bytes = rows * row_nb * sizeof(double);
+    const size_t acc_bytes = rows * row_bins(row_nb) * sizeof(double);
     const size_t mask_bytes = rows * nw * sizeof(unsigned long long);
     const bool grow = !S.acc.ptr || S.acc.bytes < acc_bytes || S.mask.bytes < mask_bytes;
     if (!devbuf_reserve(S.acc, acc_bytes) || !devbuf_reserve(S.mask, mask_bytes) ||
@@ -447,7 +451,7 @@ mc_status run_event(const Tables &t, DeviceProblem &d, uint64_t first, uint64_t 
     const long long nb = std::max<long long>(V.n_bins, 1);
     EvLaunch L;
     const int comb = t.comb_teeth > 0 ? t.comb_teeth : 0;
-    const int flavor = (V.has_time || comb) ? FL_ALL : (V.G > 0 ? FL_MG : FL_CE);
+    const int flavor = (V.has_time || V.general || comb) ? FL_ALL : (V.G > 0 ? FL_MG : FL_CE);
     mc_status st = event_launch_shape(d, tune, d.tuned, nb, n, false, flavor, comb, S.resident, L, err);
     if (st != MC_OK) return st;
     if (L.kernel == 3) {
@@ -478,7 +482,7 @@ mc_status run_event(const Tables &t, DeviceProblem &d, uint64_t first, uint64_t 
     A.acc = static_cast<double *>(S.acc.ptr);
     A.mask = static_cast<unsigned long long *>(S.mask.ptr);
     A.nw = (int)((nb + 63) / 64);
-    A.row_nb = (int)nb;
+    A.row_nb = (int)row_bins(nb);
     A.ovf = static_cast<OvfP *>(S.ovf.ptr);
     A.ovf_cap = L.ovf_cap;
     A.sum = d.d_sum;
@@ -608,7 +612,7 @@ mc_status batch_create(const std::vector<const Tables *> &tabs, const std::vecto
     for (uint32_t i = 0; i < n; ++i) {
         all_mg = all_mg && views[i].G > 0;
         all_ce = all_ce && views[i].G == 0;
-        any_time = any_time || views[i].has_time || views[i].comb_teeth > 0;
+        any_time = any_time || views[i].has_time || views[i].general || views[i].comb_teeth > 0;
         b->comb_teeth = std::max(b->comb_teeth, views[i].comb_teeth);
     }
     b->flavor = any_time ? FL_ALL : (all_mg ? FL_MG : (all_ce ? FL_CE : FL_ALL));
@@ -793,7 +797,7 @@ mc_status batch_run(BatchState *b, int device_sms, uint64_t seed, const mc_tune 
         A.acc = static_cast<double *>(b->scratch.acc.ptr);
         A.mask = static_cast<unsigned long long *>(b->scratch.mask.ptr);
         A.nw = (int)((b->row_nb + 63) / 64);
-        A.row_nb = (int)b->row_nb;
+        A.row_nb = (int)row_bins(b->row_nb);
         A.ovf = static_cast<OvfP *>(b->scratch.ovf.ptr);
         A.ovf_cap = L.ovf_cap;
         A.tile = L.tile;

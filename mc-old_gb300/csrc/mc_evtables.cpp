@@ -99,6 +99,7 @@ bool build_event_tables(const Tables &t, EvHost &h, std::string &err)
     std::vector<int> ebo = cast<int64_t, int>(t.est_bin_off);
     P.add(ebo, &V.est_bin_off);
     V.has_time = 0;
+    V.general = 0;
     for (int k : t.filt_kind) if (k == F_TIME) V.has_time = 1;
     // the index part of the filter an attachment fixes: the device searches
     // FP32 grids with the id converted to float, so the same search is done
@@ -134,11 +135,38 @@ bool build_event_tables(const Tables &t, EvHost &h, std::string &err)
 
     // ---- records of cells, surfaces and attachments ----
     auto bits = [](float x) { int i; std::memcpy(&i, &x, 4); return i; };
-    std::vector<int> cell_rec, surf_rec, surf_est_rec;
+    std::vector<int> cell_rec, surf_rec, surf_est_rec, tl_rec, c_rec, s_rec;
+    // the records of attachments [first, last) of one cell or surface; `xs`:
+    // the event has the cross sections at hand where it scores them
+    auto attach = [&](std::vector<int> &rec, const std::vector<int32_t> &est, const std::vector<int> &pre, int first,
+                      int last, bool xs) {
+        const int at = (int)rec.size() / 4;
+        for (int i = first; i < last; ++i) {
+            const int e = est[i], f0 = t.est_filt_off[e], nf = t.est_filt_off[e + 1] - f0;
+            const int s0 = t.est_score_off[e], ns = t.est_score_off[e + 1] - s0;
+            const int kind = nf == 2 ? t.filt_kind[f0 + 1] : -1;
+            int code = nf == 1 ? ATT_PLAIN : (kind == F_GROUP ? ATT_GROUP : (kind == F_ENERGY ? ATT_ENERGY : ATT_GENERAL));
+            for (int s = s0; s < s0 + ns; ++s)
+                if (!xs && (t.score_kind[s] != SC_FLUX || t.score_kernel[s] == K_C)) code = ATT_GENERAL;
+            if (code == ATT_GENERAL) {
+                V.general = 1;
+                for (int x : {pre[i], code, e, 0}) rec.push_back(x);
+                continue;
+            }
+            const int fac0 = (int)t.est_factor[t.est_factor_off[e]];
+            const int a = code == ATT_ENERGY ? fgo[f0 + 1] : 0, b = code == ATT_ENERGY ? t.filt_grid_len[f0 + 1] : 0;
+            for (int s = 0; s < ns; ++s)
+                for (int x : {pre[i] < 0 ? -1 : pre[i] + ebo[e] + s * fac0,
+                              code + ATT_KERNEL * t.score_kernel[s0 + s] + ATT_KIND * t.score_kind[s0 + s], a, b})
+                    rec.push_back(x);
+        }
+        return std::pair<int, int>(at, (int)rec.size() / 4 - at);
+    };
     for (int c = 0; c < t.n_cell(); ++c) {
-        const int s0 = t.cell_surf_off[c], t0 = t.cell_tl_off[c], c0 = t.cell_c_off[c];
-        for (int x : {t.cell_mat[c], s0, t.cell_surf_off[c + 1] - s0, t0, t.cell_tl_off[c + 1] - t0, c0,
-                      t.cell_c_off[c + 1] - c0, 0})
+        const int s0 = t.cell_surf_off[c];
+        const auto tl = attach(tl_rec, t.cell_tl, tl_pre, t.cell_tl_off[c], t.cell_tl_off[c + 1], true);
+        const auto cl = attach(c_rec, t.cell_c, c_pre, t.cell_c_off[c], t.cell_c_off[c + 1], true);
+        for (int x : {t.cell_mat[c], s0, t.cell_surf_off[c + 1] - s0, tl.first, tl.second, cl.first, cl.second, 0})
             cell_rec.push_back(x);
     }
     for (size_t i = 0; i < t.cell_surf.size(); ++i) {
@@ -149,32 +177,10 @@ bool build_event_tables(const Tables &t, EvHost &h, std::string &err)
             surf_rec.push_back(x);
     }
     for (int sf = 0; sf < t.n_surf(); ++sf) {
-        surf_est_rec.push_back(t.surf_est_off[sf]);
-        surf_est_rec.push_back(t.surf_est_off[sf + 1] - t.surf_est_off[sf]);
+        const auto sl = attach(s_rec, t.surf_est, s_pre, t.surf_est_off[sf], t.surf_est_off[sf + 1], false);
+        surf_est_rec.push_back(sl.first);
+        surf_est_rec.push_back(sl.second);
     }
-    auto attachments = [&](const std::vector<int32_t> &est, const std::vector<int> &pre) {
-        std::vector<int> rec;
-        for (size_t i = 0; i < est.size(); ++i) {
-            const int e = est[i], f0 = t.est_filt_off[e], nf = t.est_filt_off[e + 1] - f0, s0 = t.est_score_off[e];
-            int code = ATT_GENERAL, a = e, b = 0;
-            if (t.est_score_off[e + 1] - s0 == 1 && t.score_kind[s0] == SC_FLUX && t.score_kernel[s0] != K_C && nf <= 2) {
-                const int kind = nf == 2 ? t.filt_kind[f0 + 1] : -1;
-                if (nf == 1) code = ATT_FLUX;
-                else if (kind == F_GROUP) code = ATT_FLUX_GROUP;
-                else if (kind == F_ENERGY) code = ATT_FLUX_ENERGY;
-                if (code == ATT_FLUX_ENERGY) {
-                    a = fgo[f0 + 1];
-                    b = t.filt_grid_len[f0 + 1];
-                }
-                if (code != ATT_GENERAL && t.score_kernel[s0] == K_NEUTRON) code |= ATT_WEIGHT;
-            }
-            const bool simple = code != ATT_GENERAL;
-            for (int x : {pre[i] < 0 ? -1 : pre[i] + (simple ? ebo[e] : 0), code, a, b}) rec.push_back(x);
-        }
-        return rec;
-    };
-    const std::vector<int> tl_rec = attachments(t.cell_tl, tl_pre), c_rec = attachments(t.cell_c, c_pre),
-                           s_rec = attachments(t.surf_est, s_pre);
     P.add(cell_rec, reinterpret_cast<const int **>(&V.cell_rec));
     P.add(surf_rec, reinterpret_cast<const int **>(&V.surf_rec));
     P.add(tl_rec, reinterpret_cast<const int **>(&V.tl_rec));

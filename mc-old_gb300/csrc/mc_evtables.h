@@ -29,19 +29,24 @@
 
 namespace mc {
 
-// Codes of an attachment record (AttRec::y, its low bits): the estimator takes
-// the general path, or it has one flux score and, besides the cell or surface
-// filter that the attachment fixes, no filter, an energy filter or a group
-// filter, whose index is added to the bin as it is.  ATT_WEIGHT: the score is
-// the particle's weight (a current), not weight times track length.
-enum AttCode : int { ATT_GENERAL = 0, ATT_FLUX, ATT_FLUX_ENERGY, ATT_FLUX_GROUP, ATT_CODES = 15, ATT_WEIGHT = 16 };
+// Attachment records, one per score of an attached estimator.  The low bits of
+// a code: the estimator takes the general path (one record for all its
+// scores), or besides the cell or surface filter that the attachment fixes it
+// has no filter, an energy filter or a group filter, whose index is added to
+// the bin as it is.  ATT_KERNEL: what the score multiplies (Kernel), ATT_KIND:
+// the cross section it multiplies by (ScoreKind).
+enum AttCode : int {
+    ATT_GENERAL = 0, ATT_PLAIN, ATT_ENERGY, ATT_GROUP, ATT_CODES = 15,
+    ATT_KERNEL = 16,   // x Kernel (2 bits)
+    ATT_KIND = 64,     // x ScoreKind (3 bits)
+};
 
 struct EvTables {
     // records (see above)
     const int4 *cell_rec;             // [n_cell][2]: {material, first surface record, how many, first track-length
                                       // record}, {how many, first collision record, how many, 0}
     const float4 *surf_rec;           // [cell's surfaces][2]: {surface, type, sense, k0}, {k1, k2, k3, k4}
-    const int4 *tl_rec, *c_rec, *s_rec;   // per attachment: {bin or, in general, index part (-1: outside the
+    const int4 *tl_rec, *c_rec, *s_rec;   // per attached score: {bin or, in general, index part (-1: outside the
                                       // filter), code, estimator or energy grid offset, grid length}
     const int2 *surf_est_rec;         // per surface: first crossing record, how many
     const int4 *mat_rec;              // [n_mat][2], continuous energy: {grid offset, length, bucket offset, buckets},
@@ -64,6 +69,7 @@ struct EvTables {
     const int *est_factor_off;
     const int *est_bin_off;
     int has_time;                     // a time filter exists (track time)
+    int general;                      // an attached estimator takes the general path (ATT_GENERAL)
     // continuous-energy materials
     int n_mat;
     // union grid and macroscopic tables, one 16-byte row per grid point:
