@@ -444,6 +444,27 @@ __device__ __forceinline__ float quad_root(float a, float h, float c, bool on)
     return fminf(t1, t2);
 }
 
+// Whether a flight of length l ends before the sphere for certain, so that its
+// distance need not be computed: most flights collide far from any surface.
+// The distance's polynomial t^2 + 2 h t + c (c here without compensation) is
+// taken at T, a little beyond l; m bounds, several times over, the rounding of
+// c, of the value at T and of what the root's own rounding amounts to as a
+// change of c (a few 2^-24 (T^2 + |d|^2 + r^2), as |h| <= |d|).  Inside, the
+// sphere is farther if the polynomial is still negative at T; outside, if the
+// flight leads away, passes by, or ends while the polynomial is positive and
+// still falling.  NaN and infinities (a void's flight) answer no.  (Shield of
+// 10^7 histories: 67.4 -> 63.8 ms; the distance has an error-free sum of
+// squares, a square root and two divisions.)
+__device__ __forceinline__ bool sphere_beyond(const float (&k)[5], const PState &p, float l)
+{
+    const float dx = p.x - k[0], dy = p.y - k[1], dz = p.z - k[2];
+    const float h = dx * p.u + dy * p.v + dz * p.w;
+    const float s = dx * dx + dy * dy + dz * dz, c = s - k[4];
+    const float T = 1.00001f * l, f = fmaf(T, fmaf(2.f, h, T), c);
+    const float m = 4e-6f * (fmaf(T, T, s) + k[4]);
+    return (c < -m && f < -m) || (c > m && (h >= 0.f || c - h * h > m || (f > m && T < -h)));
+}
+
 // (type and the first five coefficients from the cell's surface record)
 __device__ __forceinline__ float surface_distance(int type, const float (&k)[5], const PState &p, bool on)
 {
@@ -1082,6 +1103,7 @@ __device__ __forceinline__ int nth_set_bit(unsigned m, int n)
 // accepted candidate in candidate order, which is the one the sequential loop
 // accepts; a warp needs about two rounds where the sequential loop needs the
 // longest rejection chain among its lanes.
+template <bool kBatch>
 __device__ __forceinline__ bool warp_free_gas(Ctx &C, bool pend, const Rng32 &R, const FgState &g, float &V,
                                               float &mu)
 {
@@ -1105,7 +1127,8 @@ __device__ __forceinline__ bool warp_free_gas(Ctx &C, bool pend, const Rng32 &R,
             s_speed = __shfl_sync(0xffffffffu, g.speed, src);
             s_beta = __shfl_sync(0xffffffffu, g.beta, src);
             s_pg2 = __shfl_sync(0xffffffffu, g.p_g2, src);
-            s_k0 = __shfl_sync(0xffffffffu, R.k0, src);
+            // one problem has one seed (a lane without a particle has none in R)
+            s_k0 = kBatch ? __shfl_sync(0xffffffffu, R.k0, src) : (uint32_t)C.A->seed;
             s_k1 = __shfl_sync(0xffffffffu, R.k1, src);
             s_hlo = __shfl_sync(0xffffffffu, R.hlo, src);
             s_id = __shfl_sync(0xffffffffu, R.id, src);
@@ -1282,7 +1305,10 @@ __device__ __forceinline__ int event_advance(Ctx &C, const EvTables &V, Rng32 &R
         const float4 ra = __ldg(V.surf_rec + 2 * i), rb = __ldg(V.surf_rec + 2 * i + 1);
         const int sf = __float_as_int(ra.x);
         const float k[5] = {ra.w, rb.x, rb.y, rb.z, rb.w};
-        const float d = surface_distance(__float_as_int(ra.y), k, p, sf == p.surf);
+        const int type = __float_as_int(ra.y);
+        const bool on = sf == p.surf;
+        if (type == 4 && !on && sphere_beyond(k, p, dcol)) continue;
+        const float d = surface_distance(type, k, p, on);
         if (d < dist) { dist = d; f.S = sf; f.sense = __float_as_int(ra.z); }
     }
     const bool cross = dcol > dist;
@@ -1355,15 +1381,18 @@ __device__ __forceinline__ int event_collide_begin(Ctx &C, const EvTables &V, Rn
     p.wt = p.wt * (st - sc) / st;
     const float u = ss * R.next();
     float acc = 0.f;
-    int nuc = -1;
-    const int goff = __ldg(V.mat_rec + 2 * m).x;
+    // (one record per nuclide, its mass with it: two dependent loads fewer; with
+    // the one seed of warp_free_gas 63.8 -> 62.5 ms)
     const int4 rb = __ldg(V.mat_rec + 2 * m + 1);
+    float A = 0.f;
+    bool found = false;
     for (int k = rb.z; k < rb.z + rb.w; ++k) {
-        acc += xs_at(V.nucS + V.mnuc_tab[k] - goff, a);
-        if (acc > u) { nuc = V.mnuc_id[k]; break; }
+        const int2 r = __ldg(V.mnuc_rec + k);
+        acc += xs_at(V.nucS + r.x, a);
+        if (acc > u) { A = __int_as_float(r.y); found = true; break; }
     }
-    if (nuc < 0) return 1;   // no scatter nuclide: the reference returns without scattering
-    free_gas_begin(R, p, __ldg(V.nuc_A + nuc), g);
+    if (!found) return 1;   // no scatter nuclide: the reference returns without scattering
+    free_gas_begin(R, p, A, g);
     return 2;
 }
 
@@ -1661,7 +1690,7 @@ __global__ void __launch_bounds__(256, MinB) k_event(const EvTables V0, const Ev
                 cst = event_collide_begin<FL_ALL>(C, V, R, p, f, g);
             }
             float Vt = 0.f, mu = 0.f;
-            if (!warp_free_gas(C, cst == 2, R, g, Vt, mu) && cst == 2) {
+            if (!warp_free_gas<kBatch>(C, cst == 2, R, g, Vt, mu) && cst == 2) {
                 atomicCAS(&s_status, 0, DS_TIMEOUT);
                 cst = 1;
             }
@@ -2022,7 +2051,7 @@ __global__ void __launch_bounds__(kTrackBlock, MinB) k_track(const __grid_consta
         // free-gas target velocities for the whole warp (every lane takes part)
         float Vt = 0.f, mu = 0.f;
         if constexpr (kFl != FL_MG) {   // multigroup scatters sample no target
-            if (!warp_free_gas(C, cst == 2, R, g, Vt, mu) && cst == 2) {
+            if (!warp_free_gas<kBatch>(C, cst == 2, R, g, Vt, mu) && cst == 2) {
                 atomicCAS(&s_status, 0, DS_TIMEOUT);
                 cst = 1;
             }

@@ -191,7 +191,7 @@ bool build_event_tables(const Tables &t, EvHost &h, std::string &err)
     // ---- continuous-energy materials ----
     V.n_mat = t.n_mat();
     V.G = t.mg_groups;
-    std::vector<int> mgrid_off, mgrid_len, mnuc_off(1, 0), mnuc_id, mnuc_tab, bkt_off, bkt_n, bkt;
+    std::vector<int> mgrid_off, mgrid_len, mnuc_off(1, 0), mnuc_rec, bkt_off, bkt_n, bkt;
     std::vector<float> xrow, nucS, bkt_lo, bkt_inv;
     if (t.mg_groups == 0) {
         for (int m = 0; m < t.n_mat(); ++m) {
@@ -228,11 +228,11 @@ bool build_event_tables(const Tables &t, EvHost &h, std::string &err)
             }
             for (int i = t.mat_off[m]; i < t.mat_off[m + 1]; ++i) {
                 const int n = t.mat_nuc[i];
-                mnuc_id.push_back(n);
-                mnuc_tab.push_back((int)nucS.size());
+                mnuc_rec.push_back((int)nucS.size() - mgrid_off.back());
+                mnuc_rec.push_back(bits((float)t.nuc_A[n]));
                 for (double e : grid) nucS.push_back((float)(nuc_xs(t, n, t.xs_S, e) * t.mat_dens[i]));
             }
-            mnuc_off.push_back((int)mnuc_id.size());
+            mnuc_off.push_back((int)mnuc_rec.size() / 2);
             // log-spaced buckets: about one grid point per bucket, at most 2^16
             const double lo = std::log2(grid.front()), hi = std::log2(grid.back());
             const int nbk = std::max(16, std::min(1 << 16, 2 * L));
@@ -256,10 +256,8 @@ bool build_event_tables(const Tables &t, EvHost &h, std::string &err)
             mat_rec.push_back(x);
     P.add(mat_rec, reinterpret_cast<const int **>(&V.mat_rec));
     P.add(xrow, reinterpret_cast<const float **>(&V.xrow));
-    P.add(mnuc_id, &V.mnuc_id); P.add(mnuc_tab, &V.mnuc_tab);
+    P.add(mnuc_rec, reinterpret_cast<const int **>(&V.mnuc_rec));
     P.add(nucS, &V.nucS);
-    std::vector<float> A = cast<double, float>(t.nuc_A);
-    P.add(A, &V.nuc_A);
     P.add(bkt, &V.bkt);
 
     // ---- multigroup ----

@@ -76,10 +76,9 @@ struct EvTables {
     // {Sigma_t, Sigma_s, Sigma_c, E}, so that the two rows bracketing E
     // (one 32-byte load) give the bracket check and all three values
     const float4 *xrow;
-    const int *mnuc_id;               // nuclide index (for the mass A)
-    const int *mnuc_tab;              // offset of N_k sigma_s,k on the material grid
+    const int2 *mnuc_rec;             // per nuclide of a material: {offset of its table in nucS less the material's
+                                      // grid offset, mass A (float bits)}
     const float *nucS;                // N_k sigma_s,k tables
-    const float *nuc_A;
     const int *bkt;                   // grid index of the last point <= bucket start
     // multigroup
     int G;
