@@ -5,8 +5,9 @@ shared library into mcgpu/libmcgpu.so.  Flags that matter for results:
 
   * host C++ uses -ffp-contract=off so that set-up arithmetic (plane
     coefficients, lethargy grids) gives the same bits on x86-64 and aarch64;
-  * mc_history.cu (FP64 replay / plain) uses -fmad=false so that no multiply
-    and add are fused and the replay matches the CPU oracle bit for bit;
+  * mc_history.cu (FP64 replay) uses -fmad=false so that no multiply and add
+    are fused and the replay matches the CPU oracle bit for bit; the plain
+    mode's kernels (mc_history_plain.cu) keep contraction;
   * the mixed-precision kernels keep FMA contraction and use approximate
     FP32 division and square root with denormals flushed to zero (they are
     not bit-exact by design; the statistical tests against FP64 replay and
@@ -33,7 +34,8 @@ CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 NVCC = os.path.join(CUDA, "bin", "nvcc")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
-# (source, kind): host = g++, fp64 = nvcc without FMA contraction, fast = nvcc
+# (source, kind): host = g++, fp64 = nvcc without FMA contraction, plain = nvcc
+# with it, fast = nvcc with approximate FP32
 SOURCES = [
     ("mc_xml.cpp", "host"),
     ("mc_problem.cpp", "host"),
@@ -45,6 +47,7 @@ SOURCES = [
     ("mc_api_batch.cpp", "host"),
     ("mc_lr.cpp", "host"),
     ("mc_history.cu", "fp64"),
+    ("mc_history_plain.cu", "plain"),
     ("mc_event.cu", "fast"),
     ("mc_event_ce.cu", "fast"),
     ("mc_event_mg.cu", "fast"),

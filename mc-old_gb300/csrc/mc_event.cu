@@ -35,7 +35,7 @@
 // in FP64: per history into L2-resident rows with a touched-bin mask, folded
 // into per-CTA shared sums when the history's last particle dies, and into
 // the global sums once per CTA.  Physics and tally semantics follow the
-// reference line by line as the FP64 path does (see mc_history.cu); only the
+// reference line by line as the FP64 path does (see mc_history_kernels.cuh); only the
 // precision and the crossing logic differ, so results agree statistically,
 // not bit for bit.
 #include <algorithm>

@@ -56,7 +56,7 @@ __device__ __forceinline__ float f32_of(double x)
 }
 
 // -log(u) in FP32, relative error below 2e-6 (measured: 4e-7)
-__device__ __noinline__ float neglog_bits(uint64_t v)
+static __device__ __noinline__ float neglog_bits(uint64_t v)
 {
     if (v >> 51) {                                   // u >= 1/2: from 1 - u = (2 (2^52 - 1 - v) + 1) 2^-53
         return -log1pf(-f32_of(u01_bits(((1ull << 52) - 1) - v)));
@@ -64,8 +64,8 @@ __device__ __noinline__ float neglog_bits(uint64_t v)
     return -__logf(f32_of(u01_bits(v)));
 }
 
-__device__ __noinline__ double fdiv(double a, double b) { return a / b; }
-__device__ __noinline__ double fsqrt(double x) { return dsqrt(x); }
+static __device__ __noinline__ double fdiv(double a, double b) { return a / b; }
+static __device__ __noinline__ double fsqrt(double x) { return dsqrt(x); }
 
 // a / d with 1/d given as hi + lo, for d in recip64's range.  q0 is within a
 // unit in the last place of a / d (hi + lo has 2^-104 relative error), so the

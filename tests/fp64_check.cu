@@ -7,7 +7,7 @@
 #include <cstdio>
 #include <vector>
 
-#include "mc_history.cu"
+#include "mc_history_kernels.cuh"
 
 using namespace mc;
 

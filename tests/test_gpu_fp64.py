@@ -1,5 +1,5 @@
 """The FP64 kernels' arithmetic helpers and FP32 decisions
-(csrc/mc_fp64.cuh, csrc/mc_history.cu) against the plain FP64 expressions
+(csrc/mc_fp64.cuh, csrc/mc_history_kernels.cuh) against the plain FP64 expressions
 they stand for (tests/fp64_check.cu)."""
 import os
 import subprocess
