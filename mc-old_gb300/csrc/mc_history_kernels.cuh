@@ -137,6 +137,7 @@ struct Lane {
     // macroscopic cross sections of material xm at the particle's energy
     // (xm < -1: none yet), and the grid place they came from
     double xT, xS, xC;
+    double xS0;            // the first nuclide's part of xS (continuous energy)
     int xm, gid, gi;
     double q1, q2;
     Draws rng;
@@ -487,6 +488,7 @@ __device__ __forceinline__ void material_xs(const DevTables &T, Lane &P, int m)
             sT += N.constant * dens;
             sS += 0.0 * dens;
             sC += N.constant * dens;
+            if (i == T.mat_off[m]) P.xS0 = sS;
             continue;
         }
         locate(T, P, N.grid);
@@ -504,6 +506,7 @@ __device__ __forceinline__ void material_xs(const DevTables &T, Lane &P, int m)
         sT += t * dens;
         sS += s * dens;
         sC += c * dens;
+        if (i == T.mat_off[m]) P.xS0 = sS;
     }
     P.xT = sT;
     P.xS = sS;
@@ -1000,14 +1003,16 @@ __device__ __forceinline__ int collision_begin(const Ctx &C, Lane &P, int m, Fre
     const double implicit = P.xC + 0.0;
     P.wgt = fdiv(P.wgt * (P.xT - implicit), P.xT);
     // Material::nuclide_scatter (Material.cpp:106-115): the sum over all
-    // nuclides is Sigma_s itself
+    // nuclides is Sigma_s itself, and the lookup left its first term (with two
+    // nuclides none is looked up again: 200,000 plain shields 31.3 -> 30.8 ms)
     const double u = P.xS * u01_bits(P.rng.next());
-    double s = 0.0;
+    double s = P.xS0;
     g.nuc = -1;
-    const int last = T.mat_off[m + 1] - 1;
+    const int first = T.mat_off[m], last = T.mat_off[m + 1] - 1;
 #pragma unroll 1
-    for (int i = T.mat_off[m]; i <= last && g.nuc < 0; ++i) {
-        s = i == last ? P.xS : s + nuclide_scatter(T, P, T.nuc[T.mat_nuc[i]]) * T.mat_dens[i];
+    for (int i = first; i <= last && g.nuc < 0; ++i) {
+        if (i == last) s = P.xS;
+        else if (i != first) s = s + nuclide_scatter(T, P, T.nuc[T.mat_nuc[i]]) * T.mat_dens[i];
         if (dlt(u, s)) g.nuc = T.mat_nuc[i];
     }
     if (g.nuc < 0) return COL_DONE;
