@@ -20,11 +20,13 @@
 // behind them.  Every result bit is the serial chain's.
 //
 // Bound and measure (GB300): the latency of the steps of the densest column
-// (barriers, shuffles, 64-bit shifts).  500,000 histories x 19 bins: 61.5 ms as
-// one serial chain per bin, 0.87 ms here; 50,000 x 931 derivative columns,
-// signed and mostly zero: 7.75 -> 0.9 ms; 3,001 x 180: 0.47 -> 0.12 ms.  (With
-// 512 threads, zeros left in and a step that fails redone from memory these
-// were 0.86, 2.9 and 0.40 ms.)
+// (barriers, shuffles, 64-bit shifts) and of its loads, three blocks of which
+// are in flight.  500,000 histories x 19 bins: 61.5 ms as one serial chain per
+// bin, 0.80 ms here; 50,000 x 931 derivative columns, signed and mostly zero:
+// 7.75 -> 0.45 ms, where the slowest column adds 6,700 values serially; 3,001 x
+// 180: 0.47 -> 0.08 ms.  (One block in flight, and squares multiplied in the
+// serial chain, whose every instruction takes the pipe 64 cycles: 0.87, 0.84
+// and 0.12 ms.)
 #pragma once
 
 #include <cstdint>
@@ -35,6 +37,7 @@ namespace mc {
 
 constexpr int kFoldThreads = 256;
 constexpr int kFoldValues = 8;    // consecutive histories per thread and step
+constexpr int kFoldAhead = 3;     // blocks of histories whose loads are in flight
 // Where a step fails, the values of this many threads are added serially: two
 // at first, more when steps fail one after the other (a sum that starts from
 // zero, or a signed one that wanders about it).
@@ -105,54 +108,65 @@ __global__ void __launch_bounds__(kFoldThreads) k_fold_ordered(const double *__r
         i &= kRing - 1;
         return s_ring[i + (i >> 3)];
     };
-    double nxt[kFoldValues];
-    auto fetch = [&](uint64_t pos) {
-        const uint64_t h = pos + (uint64_t)t * kFoldValues;   // a multiple of 8, as ld
+    // the column's next values, kFoldAhead blocks of kStep histories ahead
+    double nxt[kFoldAhead][kFoldValues];
+    auto fetch = [&](double (&to)[kFoldValues], uint64_t at) {
+        const uint64_t h = at + (uint64_t)t * kFoldValues;   // a multiple of 8, as ld
         const double2 *p = reinterpret_cast<const double2 *>(col + h);
 #pragma unroll
         for (int j = 0; j < kFoldValues / 2; ++j) {
             const double2 x = h < n ? p[j] : double2{0.0, 0.0};
-            nxt[2 * j] = x.x;
-            nxt[2 * j + 1] = x.y;
+            to[2 * j] = x.x;
+            to[2 * j + 1] = x.y;
         }
     };
     if (t == 0) s_run = *dst;
     uint64_t pos = 0;
     uint32_t head = 0, count = 0;   // the ring's first value and how many it holds
-    int streak = 0;
-    fetch(0);
+    // one block of histories: its nonzero values (or their squares) go behind
+    // the ring's last, and the buffer is filled again
+    auto place = [&](double (&buf)[kFoldValues]) {
+        double w[kFoldValues];
+        int nz = 0;
+#pragma unroll
+        for (int j = 0; j < kFoldValues; ++j) {
+            w[j] = buf[j];
+            nz += (dbits(w[j]) << 1) != 0 ? 1 : 0;
+        }
+        fetch(buf, pos + (uint64_t)kFoldAhead * kStep);
+        pos += kStep;
+        if (!__syncthreads_or(nz)) return;
+        int at = nz;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int p = __shfl_up_sync(0xffffffffu, at, o);
+            if (lane >= o) at += p;
+        }
+        if (lane == 31) s_count[warp] = at;
+        at -= nz;
+        __syncthreads();
+        int total = 0;
+#pragma unroll
+        for (int i = 0; i < kWarps; ++i) {
+            if (i < warp) at += s_count[i];
+            total += s_count[i];
+        }
+        uint32_t i = head + count + (uint32_t)at;
+#pragma unroll
+        for (int j = 0; j < kFoldValues; ++j)
+            if ((dbits(w[j]) << 1) != 0) slot(i++) = squares ? w[j] * w[j] : w[j];
+        count += (uint32_t)total;
+        __syncthreads();
+    };
+    int turn = 0, streak = 0;
+#pragma unroll
+    for (int a = 0; a < kFoldAhead; ++a) fetch(nxt[a], (uint64_t)a * kStep);
     for (;;) {
         while (count < kStep && pos < n) {
-            double w[kFoldValues];
-            int nz = 0;
 #pragma unroll
-            for (int j = 0; j < kFoldValues; ++j) {
-                w[j] = nxt[j];
-                nz += (dbits(w[j]) << 1) != 0 ? 1 : 0;
-            }
-            pos += kStep;
-            fetch(pos);             // the next histories, while these are placed
-            int at = nz;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int p = __shfl_up_sync(0xffffffffu, at, o);
-                if (lane >= o) at += p;
-            }
-            if (lane == 31) s_count[warp] = at;
-            at -= nz;
-            __syncthreads();
-            int total = 0;
-#pragma unroll
-            for (int i = 0; i < kWarps; ++i) {
-                if (i < warp) at += s_count[i];
-                total += s_count[i];
-            }
-            uint32_t i = head + count + (uint32_t)at;
-#pragma unroll
-            for (int j = 0; j < kFoldValues; ++j)
-                if ((dbits(w[j]) << 1) != 0) slot(i++) = w[j];
-            count += (uint32_t)total;
-            __syncthreads();
+            for (int a = 0; a < kFoldAhead; ++a)
+                if (turn == a) place(nxt[a]);
+            turn = turn + 1 == kFoldAhead ? 0 : turn + 1;
         }
         if (count == 0) break;
         const uint32_t have = min(count, kStep);
@@ -163,10 +177,6 @@ __global__ void __launch_bounds__(kFoldThreads) k_fold_ordered(const double *__r
             const uint32_t i = (uint32_t)t * kFoldValues + j;
             v[j] = i < have ? slot(head + i) : 0.0;
             any = any || i < have;
-        }
-        if (squares && any) {
-#pragma unroll
-            for (int j = 0; j < kFoldValues; ++j) v[j] = v[j] * v[j];
         }
         const uint64_t sb = dbits(s_run);
         const int es = (int)((sb >> 52) & 0x7FF);
@@ -258,10 +268,7 @@ __global__ void __launch_bounds__(kFoldThreads) k_fold_ordered(const double *__r
             if (t == fail) {
                 double s = scannable ? dfrom(keep | ((uint64_t)k0 & 0x000FFFFFFFFFFFFFull)) : s_run;
 #pragma unroll 8
-                for (uint32_t i = first; i < taken; ++i) {
-                    const double x = slot(head + i);
-                    s += squares ? x * x : x;
-                }
+                for (uint32_t i = first; i < taken; ++i) s += slot(head + i);
                 s_run = s;
             }
         }
