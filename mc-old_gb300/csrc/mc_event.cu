@@ -354,6 +354,21 @@ static mc_status event_launch_shape(const DeviceProblem &d, const mc_tune *tune,
     return MC_OK;
 }
 
+// Lanes of a warp of k_track that take histories.  A run too short to give
+// every lane one lasts as long as its longest history, and a warp of few lanes
+// gets through an event sooner: it splits less between paths, and its free-gas
+// rounds have more helpers to a candidate.  So few histories are spread over
+// all warps (rule / full warps: 10,000 shields 0.60 / 0.66 ms, 20,000 0.64 /
+// 0.66, 40,000 0.69 / 0.72; one-group slab of 10,000 0.30 / 0.35, 40,000 0.35 /
+// 0.37; layered slab of 10,000 0.092 / 0.125, 40,000 0.119 / 0.133).  From 20
+// lanes on the spread no longer pays for its warps (60,000 shields, 25 lanes:
+// 0.76 / 0.75 ms; 99,991 layered, 16 lanes against 32: 0.162 / 0.156 ms).
+static int track_lanes(int grid, uint64_t n)
+{
+    const uint64_t warps = (uint64_t)grid * (kTrackBlock / 32);
+    return n > 20 * warps ? 32 : (int)std::max<uint64_t>(1, (n + warps - 1) / warps);
+}
+
 // bins of a history row: whole 32-byte sectors
 static long long row_bins(long long nb) { return (nb + 3) / 4 * 4; }
 
@@ -490,6 +505,7 @@ mc_status run_event(const Tables &t, DeviceProblem &d, uint64_t first, uint64_t 
     A.tile = L.tile;
     A.smem_sums = L.smem_sums ? 1 : 0;
     A.refill_min = L.refill;
+    A.lanes = track_lanes(L.grid, n);
     A.n_prob = 0;
     const int *d_rep_prob = nullptr;
     if (!L.smem_sums && (st = single_replicas(S, d, nb, A, d_rep_prob, err)) != MC_OK) return st;
@@ -803,6 +819,7 @@ mc_status batch_run(BatchState *b, int device_sms, uint64_t seed, const mc_tune 
         A.tile = L.tile;
         A.smem_sums = 0;
         A.refill_min = L.refill;
+        A.lanes = track_lanes(L.grid, n);
         A.tabs = d_tabs;
         A.prefix = d_prefix;
         A.seeds = d_seeds;

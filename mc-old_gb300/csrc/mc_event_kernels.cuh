@@ -39,6 +39,7 @@ struct EvArgs {
     int tile;
     int smem_sums;                // per-CTA sums live in shared memory
     int refill_min;               // k_track: idle lanes a warp gathers before it starts histories
+    int lanes;                    // k_track: lanes of a warp that take histories
     // batch of problems (kBatch): history index space = concatenation of
     // every problem's histories
     const EvTables *tabs;         // [n_prob]
@@ -1905,7 +1906,7 @@ __global__ void __launch_bounds__(kTrackBlock, MinB) k_track(const __grid_consta
     const int depth = A.ovf_cap / kTrackBlock;
     OvfP *stk = A.ovf + (size_t)blockIdx.x * A.ovf_cap + (size_t)threadIdx.x * depth;
     int sp = 0;
-    bool have = false, open = false, exhausted = false;
+    bool have = false, open = false, exhausted = lane >= A.lanes;
     PState p;
     uint64_t hist = 0;
     int prob = 0;
