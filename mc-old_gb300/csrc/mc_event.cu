@@ -33,11 +33,11 @@
 // which FP32 positions cannot resolve: the new cell is searched among the
 // cells that list that surface with the opposite sense.  Tallies accumulate
 // in FP64: per history into L2-resident rows with a touched-bin mask, folded
-// into per-CTA shared sums when the history's last particle dies, and into
-// the global sums once per CTA.  Physics and tally semantics follow the
-// reference line by line as the FP64 path does (see mc_history_kernels.cuh); only the
-// precision and the crossing logic differ, so results agree statistically,
-// not bit for bit.
+// when the history's last particle dies into its CTA's shared sums or into
+// replicas of the sums in L2 (kReplicaHistories), and from there into the
+// global sums.  Physics and tally semantics follow the reference line by line
+// as the FP64 path does (see mc_history_kernels.cuh); only the precision and
+// the crossing logic differ, so results agree statistically, not bit for bit.
 #include <algorithm>
 #include <cfloat>
 #include <cstring>
@@ -505,7 +505,7 @@ mc_status run_event(const Tables &t, DeviceProblem &d, uint64_t first, uint64_t 
     A.tile = L.tile;
     A.smem_sums = L.smem_sums ? 1 : 0;
     A.refill_min = L.refill;
-    A.lanes = track_lanes(L.grid, n);
+    A.lanes = track_lanes(L.grid, A.n);
     A.n_prob = 0;
     const int *d_rep_prob = nullptr;
     if (!L.smem_sums && (st = single_replicas(S, d, nb, A, d_rep_prob, err)) != MC_OK) return st;
@@ -819,7 +819,7 @@ mc_status batch_run(BatchState *b, int device_sms, uint64_t seed, const mc_tune 
         A.tile = L.tile;
         A.smem_sums = 0;
         A.refill_min = L.refill;
-        A.lanes = track_lanes(L.grid, n);
+        A.lanes = track_lanes(L.grid, A.n);
         A.tabs = d_tabs;
         A.prefix = d_prefix;
         A.seeds = d_seeds;

@@ -70,12 +70,12 @@ enum TileArray {
 // for one kind of problem leaves out the rest, which would otherwise cost the
 // hot loop registers and instruction-cache room.
 //   FL_ALL  everything: continuous-energy and multigroup physics, the
-//           general scoring path for time filters (one flight may cover
-//           several bins, through a pair list in local memory) and the
-//           particle comb;
-//   FL_CE   continuous energy, no time filter;
-//   FL_MG   multigroup, no time filter;
-//   FL_MGB  multigroup, no time filter, every tally through the history row
+//           general scoring path (time filters, where one flight may cover
+//           several bins through a pair list in local memory, and whatever
+//           else has no record, EvTables::general) and the particle comb;
+//   FL_CE   continuous energy, records only;
+//   FL_MG   multigroup, records only;
+//   FL_MGB  multigroup, records only, every tally through the history row
 //           (the event-split kernels: nothing stays in a thread's registers
 //           from one event kernel to the next).
 enum Flavor { FL_ALL = 0, FL_CE = 1, FL_MG = 2, FL_MGB = 3 };
@@ -897,7 +897,7 @@ __device__ __forceinline__ void fold_first(Ctx &C, int prob)
 }
 
 // Folds a finished history's row into the sums (Estimator.cpp:339-346):
-// per-CTA shared sums for one problem, the problem's global sums in a batch.
+// the CTA's shared sums, a replica, or the problem's global sums.
 template <int kFl>
 __device__ void history_fold(Ctx &C, int hslot, int prob)
 {
