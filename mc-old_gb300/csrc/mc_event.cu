@@ -281,11 +281,15 @@ static mc_status event_launch_shape(const DeviceProblem &d, const mc_tune *tune,
     // histories: 0.70 ms at 4, 0.75 at 6, 0.87 at 8); a full GPU runs 8 for
     // multigroup problems (deep slab 11.7 against 12.6 ms at 7, a batch of 256
     // shields 18.1 against 18.6 ms), else 7, as those kernels spill at 8
-    // (shield 67.3 against 68.2 ms, one-group slab 1.67 against 1.77 ms)
+    // (shield 67.3 against 68.2 ms, one-group slab 1.67 against 1.77 ms).  The
+    // kernels that carry everything keep 4, their pair lists and spills in
+    // local memory (500,000 duct histories with a time filter 8.9 / 9.5 / 9.7 ms
+    // at 4 / 6 / 7, with the comb 3.3 / 4.1 / 4.5; a slab with two energy
+    // filters 4.9 / 5.3 / 5.9)
     int minb_default = 4;
     if (L.kernel == 2) {
         const uint64_t lanes = (uint64_t)std::max(d.sms, 1) * kTrackBlock;
-        minb_default = n <= 4 * lanes ? 4 : (n <= 6 * lanes ? 6 : ((n <= 7 * lanes || flavor != FL_MG) ? 7 : 8));
+        minb_default = n <= 4 * lanes || flavor == FL_ALL ? 4 : (n <= 6 * lanes ? 6 : ((n <= 7 * lanes || flavor != FL_MG) ? 7 : 8));
     }
     L.minb = own_minb ? (int)tune->blocks_per_sm
            : ((tuned.blocks_per_sm && tuned.kernel == (uint32_t)L.kernel) ? (int)tuned.blocks_per_sm : minb_default);
