@@ -923,11 +923,14 @@ __device__ void history_fold(Ctx &C, int hslot, int prob)
 // that ends here are listed in shared memory, and each lane takes one off the
 // list.  A lane that folds its own history waits one L2 round trip per bin
 // while the others idle: a third of the one-group slab's time (1,000,000
-// histories, 100 cells with two scores: 2.42 -> 1.67 ms with the records of
+// histories, 100 cells with two scores: 2.42 -> 1.58 ms with the records of
 // its reaction scores; deep slab 13.0 -> 12.1 ms).  Untouched bins of a sector
-// are zero and add nothing.  Half a sector or a bin per lane coalesces the
-// additions better but takes two or four times the round trips (slab 1.84 and
-// 1.90 ms).
+// are zero and add nothing.  The values are taken by exchanges, four in flight:
+// a plain load and store of a sector that reductions went to just before, and
+// go to again just after, waited some 10^4 cycles where rows outgrow a die's
+// half of L2 (deep slab with three scores by group and cell, 5,000,000
+// histories: 17.8 ms by loads and stores, 4.5 by exchanges; shield with 50,004
+// bins, 200,000 histories: 29.5 and 8.4 ms; one-group slab 1.70 and 1.58 ms).
 constexpr int kFoldList = 64;   // sectors listed at a time, per warp
 
 template <bool kBatch>
@@ -970,12 +973,9 @@ __device__ __forceinline__ void warp_fold(Ctx &C, bool ends, int prob, uint16_t 
                 const int pb = kBatch ? __shfl_sync(0xffffffffu, prob, (e >> 6) & 31) : 0;
                 if (e >= 0) {
                     const int bin = (wi * 64 + (e & 63)) * 4;
-                    double2 *at = reinterpret_cast<double2 *>(A.acc + (row0 + (e >> 6)) * A.row_nb + bin);
-                    const double2 v0 = __ldcg(at), v1 = __ldcg(at + 1);
-                    __stcg(at, make_double2(0.0, 0.0));
-                    __stcg(at + 1, make_double2(0.0, 0.0));
+                    double *at = A.acc + (row0 + (e >> 6)) * A.row_nb + bin;
+                    const double v[4] = {row_take(at), row_take(at + 1), row_take(at + 2), row_take(at + 3)};
                     const long long rep = replica_at(A, pb);
-                    const double v[4] = {v0.x, v0.y, v1.x, v1.y};
 #pragma unroll
                     for (int j = 0; j < 4; ++j)
                         if (v[j] != 0.0) fold_add(A, C.T.ssum(), C.T.nsum, rep, bin + j, v[j]);
