@@ -123,7 +123,7 @@ typedef struct {
                                  mode: 2 where a second kernel adds
                                  replicated sums: a batch, a problem of more
                                  than 4096 bins, a long run that is not
-                                 multigroup) */
+                                 multigroup or scores in cells) */
     uint32_t reserved;        /* 0 (pads the struct to 8 bytes) */
 } mc_counters;
 

@@ -566,7 +566,7 @@ mc_status run_bank(DeviceProblem &d, const EvTables &V, int flavor, bool may_spl
     // problem has at most 1024 bins; else straight into the global sums
     const bool smem_sums = V.n_bins > 0 && V.n_bins <= 1024;
     const size_t sum_smem = smem_sums ? 2 * (size_t)V.n_bins * sizeof(double) : 0;
-    A.smem_sums = smem_sums ? 1 : 0;
+    A.smem_sums = A.rows_shared = smem_sums ? 1 : 0;
     A.n_prob = 0;
 
     cudaError_t e;

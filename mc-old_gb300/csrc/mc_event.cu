@@ -101,20 +101,34 @@ size_t tile_smem_bytes(int P, long long nb_smem)
     return (size_t)P * (8 + 4 * TA_COUNT + 2 * sizeof(unsigned short)) + sizeof(double) * 2 * (size_t)nb_smem + 64;
 }
 
-// The replicas of a batch's sums into each problem's sums (fixed order over
-// the replicas), and the replicas back to zero for the next run.
+// The replicas of the sums into each problem's sums (fixed order over the
+// replicas), and the replicas back to zero for the next run.  Bound by the
+// latency of its loads: with 16 replicas' in flight a problem of 31 bins takes
+// 0.01 ms less than with one after the other.
 __global__ void k_batch_reduce(const EvArgs A, const int *rep_prob)
 {
+    constexpr int kAhead = 16;
     const long long stride = A.rep_stride;
     for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j < stride;
          j += (long long)gridDim.x * blockDim.x) {
         double s = 0.0, q = 0.0;
-        for (int k = 0; k < A.n_rep; ++k) {
-            const size_t at = (size_t)k * (size_t)stride + (size_t)j;
-            s += A.rsum[at];
-            q += A.rsq[at];
-            A.rsum[at] = 0.0;
-            A.rsq[at] = 0.0;
+        for (int k0 = 0; k0 < A.n_rep; k0 += kAhead) {
+            double vs[kAhead], vq[kAhead];
+#pragma unroll
+            for (int i = 0; i < kAhead; ++i) {
+                const size_t at = (size_t)(k0 + i) * (size_t)stride + (size_t)j;
+                vs[i] = k0 + i < A.n_rep ? A.rsum[at] : 0.0;
+                vq[i] = k0 + i < A.n_rep ? A.rsq[at] : 0.0;
+            }
+#pragma unroll
+            for (int i = 0; i < kAhead; ++i) {
+                if (k0 + i >= A.n_rep) break;
+                const size_t at = (size_t)(k0 + i) * (size_t)stride + (size_t)j;
+                s += vs[i];
+                q += vq[i];
+                A.rsum[at] = 0.0;
+                A.rsq[at] = 0.0;
+            }
         }
         if (s != 0.0 || q != 0.0) {
             const int p = rep_prob[j];
@@ -224,10 +238,17 @@ struct EvLaunch {
 // (614 cycles for a full warp, measured), where a reduction to L2 takes the
 // SM 10 cycles and no round.  One-group slab, 1,000,000 histories: 3.29 ->
 // 2.72 ms; shield, 10,000,000: 78.7 -> 76.8 ms.  Below, the second kernel that
-// adds the replicas costs more (shield of 20,000: +0.01 ms); the multigroup
-// kernel keeps a running sum per thread instead, which is faster still (deep
-// slab 15.4 against 15.7 ms).
-constexpr uint64_t kReplicaHistories = 65536;
+// adds the replicas costs more (shield of 20,000: +0.01 ms).  The multigroup
+// kernel keeps a running sum per thread of the bin that a history scores first,
+// which is faster still (deep slab 15.4 against 15.7 ms).  Where estimators on
+// cells have its histories score in their rows, those fold into replicas in
+// longer runs (flux by group in 5 cells of the deep slab, replicas / shared
+// memory: with 8 groups 5,000,000 histories 1.0 / 1.7 ms, 1,000,000 0.26 /
+// 0.40, 200,000 0.10 / 0.13; with 30 groups 1.19 / 1.67, 0.31 / 0.39 and 0.12 /
+// 0.12 ms).  Currents alone touch few bins, and gain little (deep slab by
+// groups on every plane, 5,000,000 histories 1.01 / 1.04 ms, 200,000 0.105 /
+// 0.096).
+constexpr uint64_t kReplicaHistories = 65536, kReplicaHistoriesMg = 1 << 18;
 
 static mc_status event_launch_shape(const DeviceProblem &d, const mc_tune *tune, const mc_tune &tuned,
                                     long long nb, uint64_t n, bool batch, int flavor, int comb_teeth,
@@ -508,11 +529,14 @@ mc_status run_event(const Tables &t, DeviceProblem &d, uint64_t first, uint64_t 
     A.sq = d.d_sq;
     A.tile = L.tile;
     A.smem_sums = L.smem_sums ? 1 : 0;
+    const bool row_replicas = L.kernel == 2 && L.flavor == FL_MG && n >= kReplicaHistoriesMg &&
+                              t.cell_tl.size() + t.cell_c.size() > 0;
+    A.rows_shared = L.smem_sums && !row_replicas ? 1 : 0;
     A.refill_min = L.refill;
     A.lanes = track_lanes(L.grid, A.n);
     A.n_prob = 0;
     const int *d_rep_prob = nullptr;
-    if (!L.smem_sums && (st = single_replicas(S, d, nb, A, d_rep_prob, err)) != MC_OK) return st;
+    if (!A.rows_shared && (st = single_replicas(S, d, nb, A, d_rep_prob, err)) != MC_OK) return st;
     cudaEventRecord(d.ev[0], d.stream);
     pick_kernel(L.minb, false, L.kernel, L.flavor)<<<L.grid, L.block, L.smem, d.stream>>>(V, A);
     cudaError_t e;
@@ -821,7 +845,7 @@ mc_status batch_run(BatchState *b, int device_sms, uint64_t seed, const mc_tune 
         A.ovf = static_cast<OvfP *>(b->scratch.ovf.ptr);
         A.ovf_cap = L.ovf_cap;
         A.tile = L.tile;
-        A.smem_sums = 0;
+        A.smem_sums = A.rows_shared = 0;
         A.refill_min = L.refill;
         A.lanes = track_lanes(L.grid, A.n);
         A.tabs = d_tabs;

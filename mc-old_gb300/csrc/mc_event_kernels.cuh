@@ -48,7 +48,7 @@ struct EvArgs {
     double *const *psum;          // [n_prob] per-problem tallies
     double *const *psq;
     int n_prob;
-    // batches, and single problems whose sums do not live in shared memory,
+    // batches, and single problems whose rows do not fold into shared memory,
     // fold histories into n_rep > 0 replicas of their bins ([n_rep]
     // [rep_stride], problem p's bins from rep_off[p] on), each CTA into
     // replica blockIdx % n_rep; k_batch_reduce adds them to psum / psq
@@ -56,6 +56,7 @@ struct EvArgs {
     const long long *rep_off;     // [n_prob + 1]
     long long rep_stride;
     int n_rep;
+    int rows_shared;              // history rows fold into shared memory too, not only a history's first bin
 };
 
 enum TileArray {
@@ -840,7 +841,7 @@ __device__ __forceinline__ void score_list(Ctx &C, const EvTables &V, const int4
 // ---------------------------------------------------------------------------
 // particle life cycle
 // ---------------------------------------------------------------------------
-// where a history's sums go when they do not live in shared memory: this
+// where a history's values go when they do not fold into shared memory: this
 // CTA's replica of the problem's bins, or the problem's own.  Histories of one
 // problem fold at the same time all over the GPU; into one set of sums their
 // FP64 additions to the same few addresses queue up at L2 (a batch: about 10^9
@@ -849,9 +850,12 @@ __device__ __forceinline__ long long replica_at(const EvArgs &A, int prob)
 {
     return A.n_rep > 0 ? (long long)(blockIdx.x % A.n_rep) * A.rep_stride + (A.n_prob > 0 ? A.rep_off[prob] : 0) : 0;
 }
+// (a batch's sums never live in shared memory, which both words say; one that
+// other code tests too costs it 1 % less)
+template <bool kBatch>
 __device__ __forceinline__ void fold_add(const EvArgs &A, double *ssum, int nsum, long long at, int bin, double v)
 {
-    if (A.smem_sums) {
+    if (kBatch ? A.smem_sums : A.rows_shared) {
         atomicAdd(ssum + bin, v);
         atomicAdd(ssum + nsum + bin, v * v);
     } else {
@@ -866,6 +870,7 @@ __device__ __forceinline__ double row_take(double *bin)
 }
 
 // the bin a multigroup history kept in registers
+template <bool kBatch>
 __device__ __forceinline__ void fold_first(Ctx &C, int prob)
 {
     if (C.cbin < 0) return;
@@ -890,7 +895,7 @@ __device__ __forceinline__ void fold_first(Ctx &C, int prob)
             la[1] = v * v;
         }
     } else {
-        fold_add(*C.A, C.T.ssum(), C.T.nsum, replica_at(*C.A, prob), C.cbin, v);
+        fold_add<kBatch>(*C.A, C.T.ssum(), C.T.nsum, replica_at(*C.A, prob), C.cbin, v);
     }
     C.cbin = -1;
     C.cval = 0.0;
@@ -905,14 +910,13 @@ __device__ void history_fold(Ctx &C, int hslot, int prob)
     double *acc = C.A->acc + row * C.A->row_nb;
     unsigned long long *mask = C.A->mask + row * C.A->nw;
     const long long at = replica_at(*C.A, prob);
-    if constexpr (kFl == FL_MG) fold_first(C, prob);
     for (int wi = 0; wi < C.A->nw; ++wi) {
         if (__ldcg(mask + wi) == 0ull) continue;
         unsigned long long m = atomicExch(mask + wi, 0ull);
         while (m) {
             const int b = wi * 64 + __ffsll((long long)m) - 1;
             m &= m - 1;
-            fold_add(*C.A, C.T.ssum(), C.T.nsum, at, b, row_take(acc + b));
+            fold_add<false>(*C.A, C.T.ssum(), C.T.nsum, at, b, row_take(acc + b));
         }
     }
     C.cbin = -1;
@@ -978,7 +982,7 @@ __device__ __forceinline__ void warp_fold(Ctx &C, bool ends, int prob, uint16_t 
                     const long long rep = replica_at(A, pb);
 #pragma unroll
                     for (int j = 0; j < 4; ++j)
-                        if (v[j] != 0.0) fold_add(A, C.T.ssum(), C.T.nsum, rep, bin + j, v[j]);
+                        if (v[j] != 0.0) fold_add<kBatch>(A, C.T.ssum(), C.T.nsum, rep, bin + j, v[j]);
                 }
             }
             __syncwarp();   // the rows are clear before their owners' next reductions
@@ -1954,7 +1958,7 @@ __global__ void __launch_bounds__(kTrackBlock, MinB) k_track(const __grid_consta
         const bool ends = refill && !have && open;
         if (__builtin_expect(refill, 0)) {
             if constexpr (kFl == FL_MG) {
-                if (ends) fold_first(C, prob);
+                if (ends) fold_first<kBatch>(C, prob);
             }
             if (!C.reg_mask || __any_sync(0xffffffffu, ends && C.tmask != 0ull))
                 warp_fold<kBatch>(C, ends, prob, s_fold[threadIdx.x / 32]);
