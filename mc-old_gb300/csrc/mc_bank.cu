@@ -331,7 +331,7 @@ __global__ void __launch_bounds__(kBankBlock) k_bank_collide(const EvTables V, c
             cst = event_collide_begin<kFl>(C, V, R, p, f, g);
         }
         float Vt = 0.f, mu = 0.f;
-        if constexpr (kFl != FL_MG && kFl != FL_MGB) {   // multigroup scatters sample no target
+        if constexpr (!fl_multigroup(kFl)) {   // multigroup scatters sample no target
             if (!warp_free_gas<false>(C, cst == 2, R, g, Vt, mu) && cst == 2) {
                 atomicCAS(&s_status, 0, DS_TIMEOUT);
                 cst = 1;

@@ -139,11 +139,21 @@ __global__ void k_batch_reduce(const EvArgs A, const int *rep_prob)
     }
 }
 
+// the per-thread kernel's flavour for problems that are all multigroup (mg), all
+// continuous energy (ce) or both; full: one has a time filter, an estimator
+// without records or the comb
+int flavor_of(bool mg, bool ce, bool full)
+{
+    if (mg) return full ? FL_MGX : FL_MG;
+    return ce && !full ? FL_CE : FL_ALL;
+}
+
 EvKernel pick_kernel(int minb, bool batch, int kernel, int flavor)
 {
     if (kernel == 2) {
         if (flavor == FL_CE) return pick_track_ce(minb, batch);
         if (flavor == FL_MG) return pick_track_mg(minb, batch);
+        if (flavor == FL_MGX) return pick_track_mgx(minb, batch);
         return pick_track_all(minb, batch);
     }
     if (batch) {
@@ -224,7 +234,7 @@ struct EvLaunch {
     int block = 256, tile = 512, minb = 4, grid = 0;
     int kernel = 1;         // 1: tile / event queues (k_event), 2: one particle per thread (k_track)
     int ovf_cap = 0;        // split-copy slots per CTA
-    int flavor = FL_ALL;    // per-thread kernel flavour (FL_ALL / FL_CE / FL_MG)
+    int flavor = FL_ALL;    // per-thread kernel flavour (FL_ALL / FL_CE / FL_MG / FL_MGX)
     uint32_t max_events = kMaxEvents;
     int refill = 1;         // k_track: idle lanes a warp gathers before it starts histories
     bool smem_sums = false; // the CTA's tally sums live in shared memory (else in replicas, EvArgs::n_rep)
@@ -310,7 +320,7 @@ static mc_status event_launch_shape(const DeviceProblem &d, const mc_tune *tune,
     int minb_default = 4;
     if (L.kernel == 2) {
         const uint64_t lanes = (uint64_t)std::max(d.sms, 1) * kTrackBlock;
-        minb_default = n <= 4 * lanes || flavor == FL_ALL ? 4 : (n <= 6 * lanes ? 6 : ((n <= 7 * lanes || flavor != FL_MG) ? 7 : 8));
+        minb_default = n <= 4 * lanes || flavor == FL_ALL ? 4 : (n <= 6 * lanes ? 6 : ((n <= 7 * lanes || !fl_lane_bin(flavor)) ? 7 : 8));
     }
     L.minb = own_minb ? (int)tune->blocks_per_sm
            : ((tuned.blocks_per_sm && tuned.kernel == (uint32_t)L.kernel) ? (int)tuned.blocks_per_sm : minb_default);
@@ -333,9 +343,9 @@ static mc_status event_launch_shape(const DeviceProblem &d, const mc_tune *tune,
         L.ovf_cap = kTrackBlock * depth;
         // the per-CTA sums, then (multigroup, with them) every thread's
         // running sums of its register bin and that bin
-        L.smem_sums = nb > 0 && nb <= 4096 && (flavor == FL_MG || n < kReplicaHistories);
+        L.smem_sums = nb > 0 && nb <= 4096 && (fl_lane_bin(flavor) || n < kReplicaHistories);
         L.smem = sizeof(double) * 2 * (size_t)(L.smem_sums ? nb : 0) + 64;
-        if (L.smem_sums && flavor == FL_MG) L.smem += kTrackBlock * (2 * sizeof(double) + sizeof(int));
+        if (L.smem_sums && fl_lane_bin(flavor)) L.smem += kTrackBlock * (2 * sizeof(double) + sizeof(int));
     } else {
         L.tile = (tune && tune->bank_capacity) ? (int)tune->bank_capacity
                : (tuned.bank_capacity ? (int)tuned.bank_capacity : 512);
@@ -491,7 +501,7 @@ mc_status run_event(const Tables &t, DeviceProblem &d, uint64_t first, uint64_t 
     const long long nb = std::max<long long>(V.n_bins, 1);
     EvLaunch L;
     const int comb = t.comb_teeth > 0 ? t.comb_teeth : 0;
-    const int flavor = (V.has_time || V.general || comb) ? FL_ALL : (V.G > 0 ? FL_MG : FL_CE);
+    const int flavor = flavor_of(V.G > 0, V.G == 0, V.has_time || V.general || comb);
     mc_status st = event_launch_shape(d, tune, d.tuned, nb, n, false, flavor, comb, S.resident, L, err);
     if (st != MC_OK) return st;
     if (L.kernel == 3) {
@@ -529,7 +539,7 @@ mc_status run_event(const Tables &t, DeviceProblem &d, uint64_t first, uint64_t 
     A.sq = d.d_sq;
     A.tile = L.tile;
     A.smem_sums = L.smem_sums ? 1 : 0;
-    const bool row_replicas = L.kernel == 2 && L.flavor == FL_MG && n >= kReplicaHistoriesMg &&
+    const bool row_replicas = L.kernel == 2 && fl_lane_bin(L.flavor) && n >= kReplicaHistoriesMg &&
                               t.cell_tl.size() + t.cell_c.size() > 0;
     A.rows_shared = L.smem_sums && !row_replicas ? 1 : 0;
     A.refill_min = L.refill;
@@ -649,17 +659,15 @@ mc_status batch_create(const std::vector<const Tables *> &tabs, const std::vecto
         psq[i] = sums_to ? (*sums_to)[2 * i + 1] : probs[i]->d_sq;
         b->row_nb = std::max<long long>(b->row_nb, views[i].n_bins);
     }
-    // one flavour for the launch: every problem multigroup (or every one
-    // continuous energy) and none with a time filter, else the full kernel
-    // (the particle comb, too, takes the full kernel)
-    bool all_mg = true, all_ce = true, any_time = false;
+    // one flavour for the launch
+    bool all_mg = true, all_ce = true, any_full = false;
     for (uint32_t i = 0; i < n; ++i) {
         all_mg = all_mg && views[i].G > 0;
         all_ce = all_ce && views[i].G == 0;
-        any_time = any_time || views[i].has_time || views[i].general || views[i].comb_teeth > 0;
+        any_full = any_full || views[i].has_time || views[i].general || views[i].comb_teeth > 0;
         b->comb_teeth = std::max(b->comb_teeth, views[i].comb_teeth);
     }
-    b->flavor = any_time ? FL_ALL : (all_mg ? FL_MG : (all_ce ? FL_CE : FL_ALL));
+    b->flavor = flavor_of(all_mg, all_ce, any_full);
     b->total = prefix[n];
     // replicas of every problem's bins: kBatchReplicas copies, fewer where
     // they would pass kBatchReplicaBytes

@@ -1,4 +1,5 @@
-// mc_event_all.cu -- the per-thread kernels (k_track) for problems with time filters, and batches that mix continuous-energy and multigroup problems.
+// mc_event_all.cu -- the per-thread kernels (k_track) for continuous-energy problems with time filters,
+// estimators without records or the particle comb, and for batches that mix them with multigroup problems.
 #include "mc_event_kernels.cuh"
 
 namespace mc {

@@ -1,4 +1,4 @@
-// mc_event_ce.cu -- the per-thread kernels (k_track) for continuous-energy problems without time filters.
+// mc_event_ce.cu -- the per-thread kernels (k_track) for continuous-energy problems whose estimators all have records.
 #include "mc_event_kernels.cuh"
 
 namespace mc {

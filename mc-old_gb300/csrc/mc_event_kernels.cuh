@@ -2,7 +2,7 @@
 // event functions shared by both kernels, the tile kernel (k_event) and the
 // per-thread kernel (k_track).  Included by mc_event.cu (host side and the
 // tile kernel) and by one translation unit per per-thread kernel flavour
-// (mc_event_ce.cu, mc_event_mg.cu, mc_event_all.cu), so that the flavours
+// (mc_event_ce.cu, mc_event_mg.cu, mc_event_mgx.cu, mc_event_all.cu), so that the flavours
 // compile in parallel.
 #pragma once
 
@@ -76,10 +76,21 @@ enum TileArray {
 //           else has no record, EvTables::general) and the particle comb;
 //   FL_CE   continuous energy, records only;
 //   FL_MG   multigroup, records only;
+//   FL_MGX  multigroup, with the general scoring path and the comb.  A
+//           multigroup problem loses most of its speed without its sources
+//           from a ring, its first bin in registers and 8 CTAs per SM (FL_ALL /
+//           FL_MGX: 10^7 deep-slab histories with the comb 2.84 / 1.42 ms, with
+//           a time filter 7.3 / 5.2, with two filters besides the cell 5.0 /
+//           3.6; 256 shields, one of them with a time filter, 39.1 / 20.8);
 //   FL_MGB  multigroup, records only, every tally through the history row
 //           (the event-split kernels: nothing stays in a thread's registers
 //           from one event kernel to the next).
-enum Flavor { FL_ALL = 0, FL_CE = 1, FL_MG = 2, FL_MGB = 3 };
+enum Flavor { FL_ALL = 0, FL_CE = 1, FL_MG = 2, FL_MGB = 3, FL_MGX = 4 };
+__host__ __device__ constexpr bool fl_multigroup(int fl) { return fl == FL_MG || fl == FL_MGB || fl == FL_MGX; }
+// time filters, estimators without records and the comb
+__host__ __device__ constexpr bool fl_full(int fl) { return fl == FL_ALL || fl == FL_MGX; }
+// sources from a ring, and the first bin of a history in registers
+__host__ __device__ constexpr bool fl_lane_bin(int fl) { return fl == FL_MG || fl == FL_MGX; }
 
 // 128 threads per CTA lets the register budget step through 128 / 80 / 72 /
 // 64 registers (4 / 6 / 7 / 8 CTAs per SM)
@@ -92,6 +103,7 @@ typedef void (*EvKernel)(const EvTables, const EvArgs);
 // translation unit each
 EvKernel pick_track_ce(int minb, bool batch);
 EvKernel pick_track_mg(int minb, bool batch);
+EvKernel pick_track_mgx(int minb, bool batch);
 EvKernel pick_track_all(int minb, bool batch);
 
 }  // namespace ev
@@ -375,7 +387,7 @@ enum { XT = 0, XS = 1, XC = 2 };
 template <int kFl>
 __device__ __forceinline__ bool is_mg(const EvTables &V)
 {
-    return (kFl == FL_MG || kFl == FL_MGB) ? true : (kFl == FL_CE ? false : V.G > 0);
+    return fl_multigroup(kFl) ? true : (kFl == FL_CE ? false : V.G > 0);
 }
 
 // macroscopic cross section of cell material at the particle's energy/group
@@ -623,13 +635,13 @@ __device__ int filter_idx_l(const EvTables &V, int f, const PState &p, float t_o
     }
 }
 
-// kFl == FL_MG: the first bin a history scores is summed in registers
+// fl_lane_bin: the first bin a history scores is summed in registers
 // (cbin / cval) and never goes through the row: short multigroup histories
 // often score one bin only (a leakage or reflection current).
 template <int kFl>
 __device__ __forceinline__ void tally_add(Ctx &C, int hslot, int bin, double val)
 {
-    if constexpr (kFl == FL_MG) {
+    if constexpr (fl_lane_bin(kFl)) {
         if (C.cbin == bin || C.cbin < 0) {
             // most histories score once: no FP64 addition (19 SM cycles a warp)
             if (C.cbin < 0) C.cval = val;
@@ -740,8 +752,8 @@ __device__ void estimator_score(Ctx &C, int e, const PState &p, float t_old, flo
         return;
     }
     if (estimator_score_simple<kFl>(C, e, p, l_in, pre, fixed)) return;
-    if constexpr (kFl != FL_ALL) {
-        atomicCAS(C.s_status, 0, DS_OVERFLOW);   // unreachable: time filters get the FL_ALL kernel
+    if constexpr (!fl_full(kFl)) {
+        atomicCAS(C.s_status, 0, DS_OVERFLOW);   // unreachable: time filters get the full kernels
         return;
     }
     const int f0 = V.est_filt_off[e], nf = V.est_filt_off[e + 1] - f0;
@@ -769,7 +781,7 @@ __device__ void estimator_score(Ctx &C, int e, const PState &p, float t_old, flo
         int idx1 = 0;
         for (int i = 0; i < nf; ++i) idx1 += il[off[i] + idx[i]].bin * fac[i + 1];
         for (int s = 0; s < ns; ++s) {
-            tally_add<FL_ALL>(C, p.hslot, base + idx1, (double)score_value<FL_ALL>(C, s0 + s, p, l));
+            tally_add<kFl>(C, p.hslot, base + idx1, (double)score_value<kFl>(C, s0 + s, p, l));
             idx1 += fac[0];
         }
         for (int i = 0; i < nf; ++i) {
@@ -787,7 +799,7 @@ __device__ void estimator_score(Ctx &C, int e, const PState &p, float t_old, flo
 // The scores of one list of attachments; l_in and fixed as above; x: the flight
 // whose cross sections reaction scores use (kXs).  Nearly all take their bin
 // from the record and at most one filter.  The rest need the general path,
-// which only the FL_ALL kernels carry (EvTables::general): three inlined copies
+// which only the full kernels carry (EvTables::general): three inlined copies
 // were 17 of the continuous-energy kernel's 79 KB, and its loop is bound by
 // instruction fetches; out of line they cost it registers instead.
 template <int kFl, bool kXs>
@@ -805,7 +817,7 @@ __device__ __forceinline__ void score_list(Ctx &C, const EvTables &V, const int4
         const int code = r.y & ATT_CODES;
         int bin = r.x;
         if (code == ATT_GENERAL) {
-            if constexpr (kFl == FL_ALL) estimator_score<kFl>(C, r.z, p, t_old, speed, l_in, bin, fixed);
+            if constexpr (fl_full(kFl)) estimator_score<kFl>(C, r.z, p, t_old, speed, l_in, bin, fixed);
             else atomicCAS(C.s_status, 0, DS_OVERFLOW);   // unreachable
             continue;
         }
@@ -1325,7 +1337,7 @@ __device__ __forceinline__ int event_advance(Ctx &C, const EvTables &V, Rng32 &R
     const float t_old = p.t;
     p.x = fmaf(p.u, l, p.x); p.y = fmaf(p.v, l, p.y); p.z = fmaf(p.w, l, p.z);
     float speed = 0.f;
-    if (kFl == FL_ALL && V.has_time) {
+    if (fl_full(kFl) && V.has_time) {
         speed = speed_of(p.E);
         p.t = t_old + l / speed;
     }
@@ -1354,7 +1366,7 @@ __device__ __forceinline__ int event_collide_begin(Ctx &C, const EvTables &V, Rn
     R.draw = 1u;
     R.cached = 1u;
     const int4 cb = __ldg(V.cell_rec + 2 * p.cell + 1);
-    score_list<kFl, true>(C, V, V.c_rec, cb.y, cb.z, p, p.t, kFl == FL_ALL && V.has_time ? speed_of(p.E) : 0.f, 0.f, 1, &f);
+    score_list<kFl, true>(C, V, V.c_rec, cb.y, cb.z, p, p.t, fl_full(kFl) && V.has_time ? speed_of(p.E) : 0.f, 0.f, 1, &f);
     const float st = f.sig;
     if (is_mg<kFl>(V)) {
         const int row = m * V.G + p.g;
@@ -1442,7 +1454,7 @@ __device__ __forceinline__ bool event_cross(Ctx &C, const EvTables &V, Rng32 &R,
         surface_reflect(V, S, p);
     }
     if (p.wt != 0.f) {   // a vacuum boundary kills first and scores zero (general.cpp:98-111)
-        const float speed = kFl == FL_ALL && V.has_time ? speed_of(p.E) : 0.f;
+        const float speed = fl_full(kFl) && V.has_time ? speed_of(p.E) : 0.f;
         const int2 se = __ldg(V.surf_est_rec + S);
         score_list<kFl, false>(C, V, V.s_rec, se.x, se.y, p, p.t, speed, 0.f, 0, nullptr);
     }
@@ -1891,9 +1903,9 @@ __global__ void __launch_bounds__(kTrackBlock, MinB) k_track(const __grid_consta
     auto seed_of = [&](int prob) -> uint64_t { return kBatch ? A.seeds[prob] : A.seed; };
     if (A.smem_sums) {
         for (int b = threadIdx.x; b < 2 * V0.n_bins; b += blockDim.x) C.T.ssum()[b] = 0.0;
-        if constexpr (kFl == FL_MG) C.T.lane_bin()[threadIdx.x] = -1;
+        if constexpr (fl_lane_bin(kFl)) C.T.lane_bin()[threadIdx.x] = -1;
     }
-    constexpr bool kRinged = kFl == FL_MG;
+    constexpr bool kRinged = fl_lane_bin(kFl);
     __shared__ SrcRing s_ring[kRinged ? kTrackBlock / 32 : 1];
     SrcRing &Q = s_ring[kRinged ? threadIdx.x / 32 : 0];
     if (kRinged && threadIdx.x % 32 == 0) {
@@ -1929,7 +1941,7 @@ __global__ void __launch_bounds__(kTrackBlock, MinB) k_track(const __grid_consta
         return true;
     };
     for (uint32_t it = 1;; ++it) {
-        if constexpr (kFl == FL_ALL) {
+        if constexpr (fl_full(kFl)) {
             // a walk has just ended whenever the stack is non-empty here
             if (!have && sp > 0) {
                 const EvTables &Vc = tab(prob);
@@ -1957,7 +1969,7 @@ __global__ void __launch_bounds__(kTrackBlock, MinB) k_track(const __grid_consta
         const bool refill = __popc(im) >= A.refill_min || __ballot_sync(0xffffffffu, have) == 0u;
         const bool ends = refill && !have && open;
         if (__builtin_expect(refill, 0)) {
-            if constexpr (kFl == FL_MG) {
+            if constexpr (fl_lane_bin(kFl)) {
                 if (ends) fold_first<kBatch>(C, prob);
             }
             if (!C.reg_mask || __any_sync(0xffffffffu, ends && C.tmask != 0ull))
@@ -2055,7 +2067,7 @@ __global__ void __launch_bounds__(kTrackBlock, MinB) k_track(const __grid_consta
         }
         // free-gas target velocities for the whole warp (every lane takes part)
         float Vt = 0.f, mu = 0.f;
-        if constexpr (kFl != FL_MG) {   // multigroup scatters sample no target
+        if constexpr (!fl_multigroup(kFl)) {   // multigroup scatters sample no target
             if (!warp_free_gas<kBatch>(C, cst == 2, R, g, Vt, mu) && cst == 2) {
                 atomicCAS(&s_status, 0, DS_TIMEOUT);
                 cst = 1;
@@ -2082,7 +2094,7 @@ __global__ void __launch_bounds__(kTrackBlock, MinB) k_track(const __grid_consta
         }
     }
 
-    if constexpr (kFl == FL_MG) {
+    if constexpr (fl_lane_bin(kFl)) {
         if (A.smem_sums) {   // the thread's running sums into the CTA's
             const int lb = C.T.lane_bin()[threadIdx.x];
             if (lb >= 0) {

@@ -1,4 +1,4 @@
-// mc_event_mg.cu -- the per-thread kernels (k_track) for multigroup problems without time filters.
+// mc_event_mg.cu -- the per-thread kernels (k_track) for multigroup problems whose estimators all have records.
 // Their Philox refills beyond an event's first block go through one shared
 // out-of-line copy (see Rng32 in mc_event_kernels.cuh): measured faster for
 // these short, cheap events.
