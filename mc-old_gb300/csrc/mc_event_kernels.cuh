@@ -797,7 +797,8 @@ __device__ void estimator_score(Ctx &C, int e, const PState &p, float t_old, flo
 }
 
 // The scores of one list of attachments; l_in and fixed as above; x: the flight
-// whose cross sections reaction scores use (kXs).  Nearly all take their bin
+// whose cross sections reaction scores use (kXs; behind a crossing only a
+// multigroup problem's have a record).  Nearly all take their bin
 // from the record and at most one filter.  The rest need the general path,
 // which only the full kernels carry (EvTables::general): three inlined copies
 // were 17 of the continuous-energy kernel's 79 KB, and its loop is bound by
@@ -832,15 +833,18 @@ __device__ __forceinline__ void score_list(Ctx &C, const EvTables &V, const int4
         if (__builtin_expect(r.y >= ATT_KERNEL, 0)) {   // not a flux by track length
             const int kern = (r.y / ATT_KERNEL) & 3;
             if (kern == K_NEUTRON) val = p.wt;
-            if constexpr (kXs) {
-                // the flight has looked the material up at this energy (a
-                // void's cross sections are zero)
-                if (kern == K_C) val = p.wt / x->sig;
-                const int kind = r.y / ATT_KIND, m = V.cell_mat[p.cell];
+            const int kind = r.y / ATT_KIND;
+            if (kXs || (is_mg<kFl>(V) && (kern == K_C || kind != SC_FLUX))) {
+                // the flight has looked the material up at this energy; behind
+                // a crossing a group's are read here (a void's are zero)
+                const int m = V.cell_mat[p.cell];
+                auto group_xs = [&](const float *tab) { return m >= 0 ? __ldg(tab + m * V.G + p.g) : 0.f; };
+                if (kern == K_C) val = p.wt / (kXs ? x->sig : group_xs(V.mg_total));
                 if (kind != SC_FLUX) {
-                    float xs = kind == SC_TOTAL ? x->sig : (kind == SC_SCATTER ? x->ss : x->sc);
-                    if (is_mg<kFl>(V) && kind != SC_TOTAL && m >= 0)
-                        xs = __ldg((kind == SC_SCATTER ? V.mg_scat_tot : V.mg_capture) + m * V.G + p.g);
+                    float xs;
+                    if (is_mg<kFl>(V) && !(kXs && kind == SC_TOTAL))
+                        xs = group_xs(kind == SC_TOTAL ? V.mg_total : (kind == SC_SCATTER ? V.mg_scat_tot : V.mg_capture));
+                    else xs = kind == SC_TOTAL ? x->sig : (kind == SC_SCATTER ? x->ss : x->sc);
                     val = xs * val;
                 }
                 if (m >= 0) C.cnt[C_XS] += (kern == K_C ? 1u : 0u) + (kind != SC_FLUX ? 1u : 0u);

@@ -137,7 +137,8 @@ bool build_event_tables(const Tables &t, EvHost &h, std::string &err)
     auto bits = [](float x) { int i; std::memcpy(&i, &x, 4); return i; };
     std::vector<int> cell_rec, surf_rec, surf_est_rec, tl_rec, c_rec, s_rec;
     // the records of attachments [first, last) of one cell or surface; `xs`:
-    // the event has the cross sections at hand where it scores them
+    // the event has the cross sections at hand where it scores them (behind a
+    // crossing, a group's are one load away)
     auto attach = [&](std::vector<int> &rec, const std::vector<int32_t> &est, const std::vector<int> &pre, int first,
                       int last, bool xs) {
         const int at = (int)rec.size() / 4;
@@ -177,7 +178,7 @@ bool build_event_tables(const Tables &t, EvHost &h, std::string &err)
             surf_rec.push_back(x);
     }
     for (int sf = 0; sf < t.n_surf(); ++sf) {
-        const auto sl = attach(s_rec, t.surf_est, s_pre, t.surf_est_off[sf], t.surf_est_off[sf + 1], false);
+        const auto sl = attach(s_rec, t.surf_est, s_pre, t.surf_est_off[sf], t.surf_est_off[sf + 1], t.mg_groups > 0);
         surf_est_rec.push_back(sl.first);
         surf_est_rec.push_back(sl.second);
     }
