@@ -239,9 +239,10 @@ mc_status mc_tally_read(const mc_problem *p, uint32_t est, double *mean, double 
     const uint64_t nb = (uint64_t)(b1 - b0);
     if (cap < nb && (mean || sigma || sum || sumsq)) return MC_ERR_ARG;
     std::string err;
-    mc_status st = read_bins(p->dev, (size_t)b0, (size_t)nb, err);
+    std::vector<double> both(2 * nb);
+    mc_status st = read_bins(p->dev, (size_t)b0, (size_t)nb, both.data(), err);
     if (st != MC_OK) { const_cast<mc_problem *>(p)->err = err; return st; }
-    const double *s = reinterpret_cast<const double *>(p->dev.h_stage + kCtlBytes), *q = s + nb;
+    const double *s = both.data(), *q = s + nb;
     // Estimator::end_cycle / end_simulation for one active cycle
     // (Estimator.cpp:347-367) with N = histories folded so far
     const double N = (double)p->dev.histories;

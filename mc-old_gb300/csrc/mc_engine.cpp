@@ -245,11 +245,12 @@ mc_status reset_tallies(DeviceProblem &d, std::string &err)
     return MC_OK;
 }
 
-mc_status read_bins(const DeviceProblem &d, size_t from, size_t count, std::string &err)
+mc_status read_bins(const DeviceProblem &d, size_t from, size_t count, double *out, std::string &err)
 {
     if (count == 0) return MC_OK;
     if (!d.tallies) { err = "read tallies: problem was not loaded"; return MC_ERR_CUDA; }
     const size_t pitch = (size_t)((const char *)d.d_sq - (const char *)d.d_sum), width = count * sizeof(double);
+    std::lock_guard<std::mutex> lk(*d.stage_mu);
     cudaError_t e;
     if ((e = cudaMemcpy2DAsync(d.h_stage + kCtlBytes, width, d.d_sum + from, pitch, width, 2, cudaMemcpyDeviceToHost,
                                d.stream)) != cudaSuccess ||
@@ -257,17 +258,18 @@ mc_status read_bins(const DeviceProblem &d, size_t from, size_t count, std::stri
         err = cuda_msg(e, "read tallies");
         return MC_ERR_CUDA;
     }
+    std::memcpy(out, d.h_stage + kCtlBytes, 2 * width);
     return MC_OK;
 }
 
 mc_status read_sums(const DeviceProblem &d, std::vector<double> &sum, std::vector<double> &sq, std::string &err)
 {
     const size_t nb = (size_t)std::max<long long>(d.dt.n_bins, 1);
-    const mc_status st = read_bins(d, 0, nb, err);
+    std::vector<double> both(2 * nb);
+    const mc_status st = read_bins(d, 0, nb, both.data(), err);
     if (st != MC_OK) return st;
-    const double *h = reinterpret_cast<const double *>(d.h_stage + kCtlBytes);
-    sum.assign(h, h + nb);
-    sq.assign(h + nb, h + 2 * nb);
+    sum.assign(both.begin(), both.begin() + nb);
+    sq.assign(both.begin() + nb, both.end());
     return MC_OK;
 }
 

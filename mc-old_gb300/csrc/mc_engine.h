@@ -4,6 +4,8 @@
 
 #include <stdint.h>
 
+#include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -40,6 +42,8 @@ struct DeviceProblem {
     DevTables dt{};
     // pinned: kCtlBytes for a run's control words, then [2][n_bins] for tallies
     char *h_stage = nullptr;
+    // the stage's tallies are one reader's at a time (a const handle is read by any thread)
+    std::shared_ptr<std::mutex> stage_mu = std::make_shared<std::mutex>();
     void *tallies = nullptr;       // d_sum, d_sq and d_exact, one allocation (cleared as one)
     size_t tally_bytes = 0;
     double *d_sum = nullptr;       // [n_bins] sum of history totals
@@ -71,9 +75,9 @@ cudaError_t upload_tables_async(DeviceProblem &d, cudaStream_t st);
 cudaError_t reset_tallies_async(DeviceProblem &d, cudaStream_t st);
 void tallies_were_reset(DeviceProblem &d);   // the host's side of a reset
 cudaError_t event_tables_upload_async(DeviceProblem &d, cudaStream_t st);
-// bins [from, from + count) of d_sum and d_sq into the handle's pinned stage
-// (sums, then squares); one copy, one wait
-mc_status read_bins(const DeviceProblem &d, size_t from, size_t count, std::string &err);
+// bins [from, from + count) of d_sum and d_sq into out (sums, then squares) by
+// way of the handle's pinned stage; one copy, one wait; from any thread
+mc_status read_bins(const DeviceProblem &d, size_t from, size_t count, double *out, std::string &err);
 mc_status read_sums(const DeviceProblem &d, std::vector<double> &sum, std::vector<double> &sq, std::string &err);
 mc_status run_histories(const Tables &t, DeviceProblem &d, uint64_t first, uint64_t n, uint64_t seed,
                         mc_mode mode, const mc_tune *tune, std::string &err);

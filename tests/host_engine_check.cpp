@@ -1,0 +1,90 @@
+// host_engine_check.cpp -- the host side of the library over a fake CUDA runtime
+// (fake_cudart.h).  argv: the scenario, then a continuous-energy problem's
+// folder, its cross-section folder and a one-group problem's folder.  Prints
+// "ok", or what is wrong.
+#include <cstdio>
+#include <cstring>
+#include <functional>
+#include <string>
+#include <thread>
+#include <vector>
+
+#include "fake_cudart.h"
+#include "mcgpu.h"
+
+static std::string ce, xs, mg, tmp;
+static int bad = 0;
+#define WANT(x)                                                          \
+    do {                                                                 \
+        if (!(x)) { std::printf("line %d: %s\n", __LINE__, #x); ++bad; } \
+    } while (0)
+
+static mc_problem *load(const std::string &d)
+{
+    mc_problem *p = nullptr;
+    if (mc_problem_load_xml(d.c_str(), xs.c_str(), &p) != MC_OK) {
+        std::printf("load: %s\n", mc_last_error(p));
+        std::exit(2);
+    }
+    return p;
+}
+
+// Two threads read different estimators of one handle at the same time, as a
+// const handle allows.
+static void concurrent_reads()
+{
+    mc_problem *p = load(ce);
+    uint32_t ne = 0;
+    mc_tally_count(p, &ne);
+    WANT(ne >= 2);
+    // distinct sums in every bin, by way of a saved state
+    const std::string f = tmp + "/state";
+    WANT(mc_state_save(p, f.c_str()) == MC_OK);
+    std::vector<char> raw;
+    if (FILE *h = std::fopen(f.c_str(), "rb")) {
+        for (int c; (c = std::fgetc(h)) != EOF;) raw.push_back((char)c);
+        std::fclose(h);
+    }
+    const size_t head = 8 + 4 * 8, bins = (raw.size() - head) / 16;
+    for (size_t j = 0; j < 2 * bins; ++j) {
+        const double v = 1.0 + (double)j;
+        std::memcpy(&raw[head + 8 * j], &v, 8);
+    }
+    if (FILE *h = std::fopen(f.c_str(), "wb")) {
+        std::fwrite(raw.data(), 1, raw.size(), h);
+        std::fclose(h);
+    }
+    WANT(mc_state_load(p, f.c_str()) == MC_OK);
+    fake::meet(2, 300);
+    std::vector<double> sum[2], sq[2];
+    std::vector<std::thread> ts;
+    for (uint32_t e = 0; e < 2; ++e)
+        ts.emplace_back([&, e] {
+            uint64_t nb = 0;
+            mc_tally_size(p, e, &nb);
+            sum[e].assign(nb, 0.0);
+            sq[e].assign(nb, 0.0);
+            WANT(mc_tally_read(p, e, nullptr, nullptr, sum[e].data(), sq[e].data(), nb) == MC_OK);
+        });
+    for (auto &t : ts) t.join();
+    fake::meet(0, 0);
+    double want = 1.0;
+    for (int e = 0; e < 2; ++e)
+        for (size_t j = 0; j < sum[e].size(); ++j, want += 1.0) WANT(sum[e][j] == want && sq[e][j] == want + (double)bins);
+    mc_problem_free(p);
+}
+
+int main(int argc, char **argv)
+{
+    if (argc < 6) return 2;
+    ce = argv[2]; xs = argv[3]; mg = argv[4]; tmp = argv[5];
+    const struct { const char *name; void (*run)(); } all[] = {{"concurrent reads", concurrent_reads}};
+    for (const auto &s : all)
+        if (std::strcmp(s.name, argv[1]) == 0) {
+            s.run();
+            if (!bad) std::printf("ok\n");
+            return bad != 0;
+        }
+    std::printf("no such scenario\n");
+    return 2;
+}
