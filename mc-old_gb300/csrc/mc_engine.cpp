@@ -221,6 +221,7 @@ cudaError_t upload_tables_async(DeviceProblem &d, cudaStream_t st)
 
 cudaError_t reset_tallies_async(DeviceProblem &d, cudaStream_t st)
 {
+    if (!d.tallies) return cudaErrorInvalidValue;   // the problem was not loaded (no bytes to clear would be no error)
     const cudaError_t e = cudaMemsetAsync(d.tallies, 0, d.tally_bytes, st);
     if (e != cudaSuccess) return e;
     tallies_were_reset(d);

@@ -74,11 +74,23 @@ static void concurrent_reads()
     mc_problem_free(p);
 }
 
+// A handle whose problem was not loaded has no tallies to clear or to read.
+static void not_loaded()
+{
+    mc_problem *p = nullptr;
+    WANT(mc_problem_load_xml((tmp + "/nowhere").c_str(), xs.c_str(), &p) == MC_ERR_INPUT);
+    WANT(p != nullptr);
+    WANT(mc_reset_tallies(p) != MC_OK);
+    WANT(mc_state_save(p, (tmp + "/none").c_str()) != MC_OK);
+    WANT(mc_run(p, 0, 10, 1, MC_MIXED_EVENT, nullptr) != MC_OK);
+    mc_problem_free(p);
+}
+
 int main(int argc, char **argv)
 {
     if (argc < 6) return 2;
     ce = argv[2]; xs = argv[3]; mg = argv[4]; tmp = argv[5];
-    const struct { const char *name; void (*run)(); } all[] = {{"concurrent reads", concurrent_reads}};
+    const struct { const char *name; void (*run)(); } all[] = {{"concurrent reads", concurrent_reads}, {"not loaded", not_loaded}};
     for (const auto &s : all)
         if (std::strcmp(s.name, argv[1]) == 0) {
             s.run();
