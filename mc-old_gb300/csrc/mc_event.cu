@@ -818,7 +818,8 @@ mc_status batch_run(BatchState *b, int device_sms, uint64_t seed, const mc_tune 
     L.max_events = (tune && tune->max_events) ? tune->max_events : kMaxEvents;
     const bool same_shape = b->have_shape && L.grid == b->shape.grid && L.tile == b->shape.tile &&
                             L.minb == b->shape.minb && L.kernel == b->shape.kernel &&
-                            L.max_events == b->shape.max_events && L.refill == b->shape.refill;
+                            L.max_events == b->shape.max_events && L.refill == b->shape.refill &&
+                            L.ovf_cap == b->shape.ovf_cap;   // (its bank's address is in the graph)
     for (uint32_t i = 0; i < n; ++i) b->h_seeds[i] = batch_problem_seed(seed, i);
     const BatchMeta M = batch_meta(b);
     const EvTables *d_tabs = M.tabs;

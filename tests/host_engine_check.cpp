@@ -86,11 +86,34 @@ static void not_loaded()
     mc_problem_free(p);
 }
 
+// A batch's graph holds the scratch buffers' addresses: a run that makes one of
+// them grow needs another graph.
+static void deeper_stack()
+{
+    mc_problem *ps[2] = {load(mg), load(mg)};
+    const uint64_t n[2] = {5000, 70};
+    mc_batch *b = nullptr;
+    WANT(mc_batch_create(ps, 2, n, &b) == MC_OK);
+    mc_tune t;
+    std::memset(&t, 0, sizeof(t));
+    t.kernel = 2;
+    fake::reset();
+    WANT(mc_batch_run(b, 1, &t) == MC_OK && fake::captures() == 1);
+    WANT(mc_batch_run(b, 2, &t) == MC_OK && fake::captures() == 1);   // the same graph again
+    t.stack_depth = 100;
+    WANT(mc_batch_run(b, 3, &t) == MC_OK && fake::captures() == 2);
+    WANT(mc_batch_run(b, 4, &t) == MC_OK && fake::captures() == 2);
+    t.stack_depth = 3;
+    WANT(mc_batch_run(b, 5, &t) == MC_OK && fake::captures() == 3);   // and another overflow limit
+    mc_batch_free(b);
+    for (mc_problem *p : ps) mc_problem_free(p);
+}
+
 int main(int argc, char **argv)
 {
     if (argc < 6) return 2;
     ce = argv[2]; xs = argv[3]; mg = argv[4]; tmp = argv[5];
-    const struct { const char *name; void (*run)(); } all[] = {{"concurrent reads", concurrent_reads}, {"not loaded", not_loaded}};
+    const struct { const char *name; void (*run)(); } all[] = {{"concurrent reads", concurrent_reads}, {"not loaded", not_loaded}, {"deeper stack", deeper_stack}};
     for (const auto &s : all)
         if (std::strcmp(s.name, argv[1]) == 0) {
             s.run();

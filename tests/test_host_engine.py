@@ -36,6 +36,6 @@ def check(tmp_path_factory):
     return run
 
 
-@pytest.mark.parametrize("scenario", ["concurrent reads", "not loaded"])
+@pytest.mark.parametrize("scenario", ["concurrent reads", "not loaded", "deeper stack"])
 def test_host_engine(check, scenario):
     check(scenario)
