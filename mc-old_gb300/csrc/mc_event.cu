@@ -374,13 +374,11 @@ static mc_status event_launch_shape(const DeviceProblem &d, const mc_tune *tune,
         return MC_ERR_ARG;
     }
     if (R.kernel != k || R.smem != L.smem) {
-        R.per_sm = 0;
+        R = {k, L.smem, 0};
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&R.per_sm, k, L.block, L.smem) != cudaSuccess) {
             cudaGetLastError();
-            R.per_sm = 0;
+            R = {};   // ask again next time
         }
-        R.kernel = k;
-        R.smem = L.smem;
     }
     int per_sm = R.per_sm;
     if (per_sm < 1) { err = "event kernel does not fit on an SM with this tile"; return MC_ERR_ARG; }

@@ -109,11 +109,44 @@ static void deeper_stack()
     for (mc_problem *p : ps) mc_problem_free(p);
 }
 
+static mc_tune tuned(uint32_t kernel, uint32_t chunk = 0, uint32_t digests = 0)
+{
+    mc_tune t;
+    std::memset(&t, 0, sizeof(t));
+    t.kernel = kernel;
+    t.chunk = chunk;
+    t.record_digests = digests;
+    return t;
+}
+
+// A failed query of a kernel's residency is not kept: the next run asks again.
+static void failed_query()
+{
+    int refused = 0;
+    for (long k = 0;; ++k) {
+        mc_problem *p = load(ce);
+        const mc_tune t = tuned(2);
+        fake::reset();
+        fake::fail_call(k);
+        const mc_status st = mc_run(p, 0, 1000, 1, MC_MIXED_EVENT, &t);
+        const bool hit = fake::failed();
+        fake::reset();
+        if (st == MC_ERR_ARG) {
+            ++refused;
+            WANT(mc_run(p, 0, 1000, 1, MC_MIXED_EVENT, &t) == MC_OK);
+        }
+        mc_problem_free(p);
+        if (!hit) break;
+    }
+    WANT(refused > 0);
+}
+
 int main(int argc, char **argv)
 {
     if (argc < 6) return 2;
     ce = argv[2]; xs = argv[3]; mg = argv[4]; tmp = argv[5];
-    const struct { const char *name; void (*run)(); } all[] = {{"concurrent reads", concurrent_reads}, {"not loaded", not_loaded}, {"deeper stack", deeper_stack}};
+    const struct { const char *name; void (*run)(); } all[] = {
+        {"concurrent reads", concurrent_reads}, {"not loaded", not_loaded}, {"deeper stack", deeper_stack}, {"failed query", failed_query}};
     for (const auto &s : all)
         if (std::strcmp(s.name, argv[1]) == 0) {
             s.run();
