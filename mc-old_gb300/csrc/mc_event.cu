@@ -548,19 +548,21 @@ mc_status run_event(const Tables &t, DeviceProblem &d, uint64_t first, uint64_t 
     cudaEventRecord(d.ev[0], d.stream);
     pick_kernel(L.minb, false, L.kernel, L.flavor)<<<L.grid, L.block, L.smem, d.stream>>>(V, A);
     cudaError_t e;
-    if ((e = cudaGetLastError()) != cudaSuccess) {
-        S.rep_dirty = A.n_rep > 0;
+    if ((e = cudaGetLastError()) == cudaSuccess && A.n_rep > 0) {
+        k_batch_reduce<<<(int)std::min<long long>((nb + 255) / 256, 4LL * d.sms), 256, 0, d.stream>>>(A, d_rep_prob);
+        e = cudaGetLastError();
+    }
+    if (e != cudaSuccess) {
+        if (A.n_rep > 0) S.rep_dirty = true;
         err = cuda_msg(e, "event kernel launch");
         return MC_ERR_CUDA;
     }
-    if (A.n_rep > 0)
-        k_batch_reduce<<<(int)std::min<long long>((nb + 255) / 256, 4LL * d.sms), 256, 0, d.stream>>>(A, d_rep_prob);
     cudaEventRecord(d.ev[1], d.stream);
     if ((e = cudaMemcpyAsync(d.h_stage, misc, kCtlBytes, cudaMemcpyDeviceToHost, d.stream)) != cudaSuccess ||
         (e = cudaStreamSynchronize(d.stream)) != cudaSuccess) {
         err = cuda_msg(e, "event kernel");
         S.rows_dirty = true;
-        S.rep_dirty = A.n_rep > 0;
+        if (A.n_rep > 0) S.rep_dirty = true;
         return MC_ERR_CUDA;
     }
     int hs = 0;

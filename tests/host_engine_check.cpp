@@ -141,12 +141,52 @@ static void failed_query()
     WANT(refused > 0);
 }
 
+// A run whose second kernel, the one that adds the replicated sums, could not be
+// launched fails, and its replicas are cleared before the next run folds into
+// them, whatever runs in between.
+static void failed_reduce()
+{
+    mc_problem *p = load(ce);
+    uint32_t ne = 0;
+    size_t bins = 0;
+    mc_tally_count(p, &ne);
+    for (uint32_t e = 0; e < ne; ++e) {
+        uint64_t n = 0;
+        mc_tally_size(p, e, &n);
+        bins += n;
+    }
+    const mc_tune t = tuned(2);
+    auto run = [&](uint64_t n) { return mc_run(p, 0, n, 1, MC_MIXED_EVENT, &t); };
+    auto cleared = [&] {
+        for (const fake::Fill &f : fake::fills())
+            if (f.bytes == 64 * 2 * sizeof(double) * bins) return true;
+        return false;
+    };
+    WANT(run(70000) == MC_OK && cleared());
+    fake::reset();
+    WANT(run(70000) == MC_OK && !cleared());    // the second kernel leaves them clear
+    for (int between = 0; between < 2; ++between) {
+        fake::reset();
+        fake::fail_launch("k_batch_reduce");
+        WANT(run(70000) != MC_OK && fake::failed());
+        if (between) {
+            fake::reset();
+            fake::fail_launch("k_track");
+            WANT(run(1000) != MC_OK && fake::failed());
+        }
+        fake::reset();
+        WANT(run(70000) == MC_OK && cleared());
+    }
+    mc_problem_free(p);
+}
+
 int main(int argc, char **argv)
 {
     if (argc < 6) return 2;
     ce = argv[2]; xs = argv[3]; mg = argv[4]; tmp = argv[5];
     const struct { const char *name; void (*run)(); } all[] = {
-        {"concurrent reads", concurrent_reads}, {"not loaded", not_loaded}, {"deeper stack", deeper_stack}, {"failed query", failed_query}};
+        {"concurrent reads", concurrent_reads}, {"not loaded", not_loaded}, {"deeper stack", deeper_stack}, {"failed query", failed_query},
+        {"failed reduce", failed_reduce}};
     for (const auto &s : all)
         if (std::strcmp(s.name, argv[1]) == 0) {
             s.run();

@@ -36,6 +36,6 @@ def check(tmp_path_factory):
     return run
 
 
-@pytest.mark.parametrize("scenario", ["concurrent reads", "not loaded", "deeper stack", "failed query"])
+@pytest.mark.parametrize("scenario", ["concurrent reads", "not loaded", "deeper stack", "failed query", "failed reduce"])
 def test_host_engine(check, scenario):
     check(scenario)
