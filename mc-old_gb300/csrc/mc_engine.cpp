@@ -9,6 +9,7 @@ namespace mc {
 
 std::string cuda_msg(cudaError_t e, const char *what)
 {
+    cudaGetLastError();   // reported here: a later launch's check must not find it again
     return std::string(what) + ": " + cudaGetErrorString(e);
 }
 
@@ -345,7 +346,10 @@ mc_status run_fp64(const Tables &t, DeviceProblem &d, uint64_t first, uint64_t n
         A.status = d_status;
         A.next = d_next;
         A.lanes = shape.lanes;
-        if (c0 > 0) cudaMemsetAsync(d_next, 0, sizeof(unsigned int), d.stream);
+        if (c0 > 0 && (e = cudaMemsetAsync(d_next, 0, sizeof(unsigned int), d.stream)) != cudaSuccess) {
+            err = cuda_msg(e, "memset");
+            return MC_ERR_CUDA;
+        }
         cudaEventRecord(d.ev[1], d.stream);
         if ((e = launch_history_fp64(d.dt, A, replay, grid, block, d.stream)) != cudaSuccess) {
             err = cuda_msg(e, "history kernel launch");
@@ -370,8 +374,10 @@ mc_status run_fp64(const Tables &t, DeviceProblem &d, uint64_t first, uint64_t n
             ++launches;
         }
         cudaEventRecord(d.ev[3], d.stream);
-        if (want_digest) {
-            cudaMemcpyAsync(d.digests.data() + c0, A.digest, cn * sizeof(uint64_t), cudaMemcpyDeviceToHost, d.stream);
+        if (want_digest && (e = cudaMemcpyAsync(d.digests.data() + c0, A.digest, cn * sizeof(uint64_t),
+                                                cudaMemcpyDeviceToHost, d.stream)) != cudaSuccess) {
+            err = cuda_msg(e, "digests");
+            return MC_ERR_CUDA;
         }
         const bool last = c0 + chunk >= n;
         if (last) {

@@ -420,8 +420,13 @@ static mc_status event_scratch(EventState &S, cudaStream_t st, int grid, int til
         return MC_ERR_NOMEM;
     }
     if (grow || S.rows_dirty) {
-        cudaMemsetAsync(S.acc.ptr, 0, S.acc.bytes, st);
-        cudaMemsetAsync(S.mask.ptr, 0, S.mask.bytes, st);
+        S.rows_dirty = true;
+        cudaError_t e;
+        if ((e = cudaMemsetAsync(S.acc.ptr, 0, S.acc.bytes, st)) != cudaSuccess ||
+            (e = cudaMemsetAsync(S.mask.ptr, 0, S.mask.bytes, st)) != cudaSuccess) {
+            err = cuda_msg(e, "clearing the history rows");
+            return MC_ERR_CUDA;
+        }
         S.rows_dirty = false;
     }
     return MC_OK;
@@ -467,16 +472,24 @@ static mc_status single_replicas(EventState &S, const DeviceProblem &d, long lon
         S.rep_dirty = true;
     }
     char *m = static_cast<char *>(S.rep_meta.ptr);
+    cudaError_t e;
     if (S.rep_dirty || S.rep_sum != d.d_sum || S.rep_sq != d.d_sq) {   // (autotuning folds into scratch sums)
         // the sums' pointers and rep_off = {0, nb} in the first 256 bytes, then rep_prob = 0
         struct { double *ps, *pq; long long off[2]; } h{d.d_sum, d.d_sq, {0, nb}};
-        cudaMemcpyAsync(m, &h, sizeof(h), cudaMemcpyHostToDevice, d.stream);
+        S.rep_sum = nullptr;
+        if ((e = cudaMemcpyAsync(m, &h, sizeof(h), cudaMemcpyHostToDevice, d.stream)) != cudaSuccess) {
+            err = cuda_msg(e, "describing the replicated sums");
+            return MC_ERR_CUDA;
+        }
         S.rep_sum = d.d_sum;
         S.rep_sq = d.d_sq;
     }
     if (S.rep_dirty) {
-        cudaMemsetAsync(m + 256, 0, (size_t)nb * sizeof(int), d.stream);
-        cudaMemsetAsync(S.rep.ptr, 0, rep_bytes, d.stream);
+        if ((e = cudaMemsetAsync(m + 256, 0, (size_t)nb * sizeof(int), d.stream)) != cudaSuccess ||
+            (e = cudaMemsetAsync(S.rep.ptr, 0, rep_bytes, d.stream)) != cudaSuccess) {
+            err = cuda_msg(e, "clearing the replicated sums");
+            return MC_ERR_CUDA;
+        }
         S.rep_dirty = false;
     }
     A.rsum = static_cast<double *>(S.rep.ptr);
@@ -518,7 +531,11 @@ mc_status run_event(const Tables &t, DeviceProblem &d, uint64_t first, uint64_t 
     }
     if ((st = event_scratch(S, d.stream, L.grid, L.tile, L.ovf_cap, nb, err)) != MC_OK) return st;
     char *misc = static_cast<char *>(S.misc.ptr);
-    cudaMemsetAsync(misc, 0, kCtlBytes, d.stream);
+    cudaError_t e;
+    if ((e = cudaMemsetAsync(misc, 0, kCtlBytes, d.stream)) != cudaSuccess) {
+        err = cuda_msg(e, "clearing the control words");
+        return MC_ERR_CUDA;
+    }
     EvArgs A{};
     A.first = first;
     A.n = n;
@@ -547,7 +564,6 @@ mc_status run_event(const Tables &t, DeviceProblem &d, uint64_t first, uint64_t 
     if (!A.rows_shared && (st = single_replicas(S, d, nb, A, d_rep_prob, err)) != MC_OK) return st;
     cudaEventRecord(d.ev[0], d.stream);
     pick_kernel(L.minb, false, L.kernel, L.flavor)<<<L.grid, L.block, L.smem, d.stream>>>(V, A);
-    cudaError_t e;
     if ((e = cudaGetLastError()) == cudaSuccess && A.n_rep > 0) {
         k_batch_reduce<<<(int)std::min<long long>((nb + 255) / 256, 4LL * d.sms), 256, 0, d.stream>>>(A, d_rep_prob);
         e = cudaGetLastError();
@@ -691,6 +707,7 @@ mc_status batch_create(const std::vector<const Tables *> &tabs, const std::vecto
     const size_t rep_bytes = 2 * sizeof(double) * (size_t)b->n_rep * (size_t)b->rep_stride;
     if (!devbuf_reserve(b->meta, sz) || !devbuf_reserve(b->rep, rep_bytes) ||
         cudaHostAlloc(&b->h_seeds, n * 8 + kCtlBytes, cudaHostAllocDefault) != cudaSuccess) {
+        cudaGetLastError();
         batch_state_free(b);
         err = "cannot allocate batch descriptors";
         return MC_ERR_NOMEM;
@@ -814,12 +831,14 @@ mc_status batch_run(BatchState *b, int device_sms, uint64_t seed, const mc_tune 
     EvLaunch L;
     mc_status st = event_launch_shape(shape_dev, tune, tuned, 0, b->total, true, b->flavor, b->comb_teeth, b->scratch.resident, L, err);
     if (st != MC_OK) return st;
-    if ((st = event_scratch(b->scratch, b->stream, L.grid, L.tile, L.ovf_cap, b->row_nb, err)) != MC_OK) return st;
     L.max_events = (tune && tune->max_events) ? tune->max_events : kMaxEvents;
     const bool same_shape = b->have_shape && L.grid == b->shape.grid && L.tile == b->shape.tile &&
                             L.minb == b->shape.minb && L.kernel == b->shape.kernel &&
                             L.max_events == b->shape.max_events && L.refill == b->shape.refill &&
                             L.ovf_cap == b->shape.ovf_cap;   // (its bank's address is in the graph)
+    // until another graph is there, the present one may hold addresses of scratch that has grown
+    b->have_shape = same_shape;
+    if ((st = event_scratch(b->scratch, b->stream, L.grid, L.tile, L.ovf_cap, b->row_nb, err)) != MC_OK) return st;
     for (uint32_t i = 0; i < n; ++i) b->h_seeds[i] = batch_problem_seed(seed, i);
     const BatchMeta M = batch_meta(b);
     const EvTables *d_tabs = M.tabs;
@@ -833,7 +852,11 @@ mc_status batch_run(BatchState *b, int device_sms, uint64_t seed, const mc_tune 
     double *d_rsq = d_rsum + (size_t)b->n_rep * (size_t)b->rep_stride;
     cudaError_t e;
     if (b->rep_dirty) {
-        cudaMemsetAsync(b->rep.ptr, 0, 2 * sizeof(double) * (size_t)b->n_rep * (size_t)b->rep_stride, b->stream);
+        if ((e = cudaMemsetAsync(b->rep.ptr, 0, 2 * sizeof(double) * (size_t)b->n_rep * (size_t)b->rep_stride, b->stream)) !=
+            cudaSuccess) {
+            err = cuda_msg(e, "clearing the replicated sums");
+            return MC_ERR_CUDA;
+        }
         b->rep_dirty = false;
     }
     if (!same_shape) {
@@ -876,18 +899,26 @@ mc_status batch_run(BatchState *b, int device_sms, uint64_t seed, const mc_tune 
             err = cuda_msg(e, "graph capture");
             return MC_ERR_CUDA;
         }
-        cudaMemcpyAsync(d_seeds, b->h_seeds, n * 8, cudaMemcpyHostToDevice, b->stream);
-        cudaMemsetAsync(misc, 0, kCtlBytes, b->stream);
-        pick_kernel(L.minb, true, L.kernel, L.flavor)<<<L.grid, L.block, L.smem, b->stream>>>(V0, A);
-        const int rgrid = (int)std::min<long long>((b->rep_stride + 255) / 256, 4LL * device_sms);
-        k_batch_reduce<<<rgrid, 256, 0, b->stream>>>(A, d_rep_prob);
-        if ((e = cudaStreamEndCapture(b->stream, &g)) != cudaSuccess) {
-            err = cuda_msg(e, "graph capture end");
+        cudaError_t in = cudaMemcpyAsync(d_seeds, b->h_seeds, n * 8, cudaMemcpyHostToDevice, b->stream);
+        if (in == cudaSuccess) in = cudaMemsetAsync(misc, 0, kCtlBytes, b->stream);
+        if (in == cudaSuccess) {
+            pick_kernel(L.minb, true, L.kernel, L.flavor)<<<L.grid, L.block, L.smem, b->stream>>>(V0, A);
+            in = cudaGetLastError();
+        }
+        if (in == cudaSuccess) {
+            const int rgrid = (int)std::min<long long>((b->rep_stride + 255) / 256, 4LL * device_sms);
+            k_batch_reduce<<<rgrid, 256, 0, b->stream>>>(A, d_rep_prob);
+            in = cudaGetLastError();
+        }
+        e = cudaStreamEndCapture(b->stream, &g);   // in any case: the stream must leave the capture
+        if (in != cudaSuccess) e = in;
+        if (e == cudaSuccess) e = cudaGraphInstantiate(&b->exec, g, 0);
+        if (g) cudaGraphDestroy(g);
+        if (e != cudaSuccess) {
+            b->exec = nullptr;
+            err = cuda_msg(e, "batch graph");
             return MC_ERR_CUDA;
         }
-        e = cudaGraphInstantiate(&b->exec, g, 0);
-        cudaGraphDestroy(g);
-        if (e != cudaSuccess) { err = cuda_msg(e, "graph instantiate"); return MC_ERR_CUDA; }
         b->shape = L;
         b->have_shape = true;
     }

@@ -83,8 +83,12 @@ mc_status run_params(mc_problem *p, const double *params, uint64_t n, uint64_t s
     if (!devbuf_reserve(S.tab, mg_bytes + cum.size() * sizeof(double) + 256)) { p->err = "cannot allocate parameter tables"; return MC_ERR_NOMEM; }
     char *tp = static_cast<char *>(S.tab.ptr);
     DevTables T = d.dt;
-    cudaMemcpyAsync(tp, mg.data(), mg_bytes, cudaMemcpyHostToDevice, d.stream);
-    cudaMemcpyAsync(tp + mg_bytes, cum.data(), cum.size() * sizeof(double), cudaMemcpyHostToDevice, d.stream);
+    cudaError_t e;
+    if ((e = cudaMemcpyAsync(tp, mg.data(), mg_bytes, cudaMemcpyHostToDevice, d.stream)) != cudaSuccess ||
+        (e = cudaMemcpyAsync(tp + mg_bytes, cum.data(), cum.size() * sizeof(double), cudaMemcpyHostToDevice, d.stream)) != cudaSuccess) {
+        p->err = cuda_msg(e, "parameter tables");
+        return MC_ERR_CUDA;
+    }
     T.mg = reinterpret_cast<const Mg64 *>(tp);
     T.mg_cum = reinterpret_cast<const double *>(tp + mg_bytes);
 
@@ -110,9 +114,11 @@ mc_status run_params(mc_problem *p, const double *params, uint64_t n, uint64_t s
     unsigned long long *cnt = reinterpret_cast<unsigned long long *>(misc);
     int *status = reinterpret_cast<int *>(misc + kNumCounters * 8);
     unsigned int *next = reinterpret_cast<unsigned int *>(misc + kNumCounters * 8 + 16);
-    cudaMemsetAsync(dsum, 0, 2 * (size_t)row * sizeof(double), d.stream);
-    cudaMemsetAsync(misc, 0, 256 + kNumCounters * sizeof(unsigned long long), d.stream);
-    cudaError_t e;
+    if ((e = cudaMemsetAsync(dsum, 0, 2 * (size_t)row * sizeof(double), d.stream)) != cudaSuccess ||
+        (e = cudaMemsetAsync(misc, 0, 256 + kNumCounters * sizeof(unsigned long long), d.stream)) != cudaSuccess) {
+        p->err = cuda_msg(e, "derivative scratch");
+        return MC_ERR_CUDA;
+    }
     for (uint64_t c0 = 0; c0 < n; c0 += chunk) {
         const uint32_t cn = (uint32_t)std::min<uint64_t>(chunk, n - c0);
         HistoryArgs A;

@@ -180,13 +180,91 @@ static void failed_reduce()
     mc_problem_free(p);
 }
 
+// A handle and what belongs to it, for one attempt.
+struct Attempt {
+    mc_problem *p = nullptr, *q = nullptr;
+    mc_batch *b = nullptr;
+    std::vector<double> out;
+    explicit Attempt(const std::string &d) : p(load(d)), out(4096) {}
+    ~Attempt()
+    {
+        if (b) mc_batch_free(b);
+        if (q) mc_problem_free(q);
+        mc_problem_free(p);
+    }
+};
+
+// Every runtime call of `act` fails once: the status tells, and the same call
+// on the same handle works afterwards.
+static void every_call(const char *name, const std::string &d, const std::function<void(Attempt &)> &setup,
+                       const std::function<mc_status(Attempt &)> &act)
+{
+    for (long k = 0;; ++k) {
+        Attempt a(d);
+        setup(a);
+        fake::reset();
+        fake::fail_call(k);
+        const mc_status st = act(a);
+        if (!fake::failed()) {
+            if (st != MC_OK || k == 0) { std::printf("%s: %d calls, status %d\n", name, (int)k, (int)st); ++bad; }
+            fake::reset();
+            return;
+        }
+        fake::fail_call(-1);
+        if (st == MC_OK) { std::printf("%s: call %d failed and nobody noticed\n", name, (int)k); ++bad; }
+        const mc_status again = act(a);
+        if (again != MC_OK) {
+            std::printf("%s: after call %d failed: status %d, %s\n", name, (int)k, (int)again, mc_last_error(a.p));
+            ++bad;
+        }
+        fake::reset();
+    }
+}
+
+static void failed_calls()
+{
+    auto none = [](Attempt &) {};
+    auto run = [](uint64_t n, mc_mode m, mc_tune t) { return [=](Attempt &a) { return mc_run(a.p, 0, n, 1, m, &t); }; };
+    every_call("mixed, sums in shared memory", ce, none, run(1000, MC_MIXED_EVENT, tuned(2)));
+    every_call("mixed, replicas", ce, none, run(70000, MC_MIXED_EVENT, tuned(2)));
+    every_call("mixed, replicas, second run", ce, [&](Attempt &a) { run(70000, MC_MIXED_EVENT, tuned(2))(a); },
+               run(70000, MC_MIXED_EVENT, tuned(2)));
+    every_call("mixed, multigroup", mg, none, run(300000, MC_MIXED_EVENT, tuned(2)));
+    every_call("mixed, tile kernel", mg, none, run(1000, MC_MIXED_EVENT, tuned(1)));
+    every_call("replay", ce, none, run(1000, MC_FP64_REPLAY, tuned(0)));
+    every_call("replay in chunks, with digests", mg, none, run(1000, MC_FP64_REPLAY, tuned(0, 300, 1)));
+    every_call("plain", mg, none, run(1000, MC_FP64_PLAIN, tuned(0)));
+    every_call("reset", ce, none, [](Attempt &a) { return mc_reset_tallies(a.p); });
+    every_call("read", ce, none, [](Attempt &a) { return mc_tally_read(a.p, 1, a.out.data(), nullptr, nullptr, nullptr, a.out.size()); });
+    every_call("upload", ce, [&](Attempt &a) { run(10, MC_MIXED_EVENT, tuned(2))(a); }, [](Attempt &a) { return mc_problem_upload(a.p); });
+    auto params = [](Attempt &a) { mc_lr_params(a.p, a.out.data(), 128); };
+    every_call("forward", mg, params, [](Attempt &a) { return mc_forward(a.p, a.out.data(), 1000, 1, a.out.data() + 128, a.out.data() + 1024); });
+    every_call("backward", mg, params, [](Attempt &a) { return mc_backward(a.p, a.out.data(), 1000, 1, a.out.data() + 128, a.out.data() + 1024); });
+    every_call("replay without allocation", mg, none,
+               [](Attempt &a) { return mc_run_replay_noalloc(a.p, 0, 1000, 1, a.out.data(), a.out.data() + 1024); });
+    auto batch = [](Attempt &a) {
+        a.q = load(mg);
+        mc_problem *ps[2] = {a.p, a.q};
+        const uint64_t n[2] = {5000, 70};
+        WANT(mc_batch_create(ps, 2, n, &a.b) == MC_OK);
+    };
+    const mc_tune two = tuned(2), one = tuned(1);
+    every_call("batch", mg, batch, [&](Attempt &a) { return mc_batch_run(a.b, 1, &two); });
+    every_call("batch, another shape", mg, [&](Attempt &a) { batch(a); mc_batch_run(a.b, 1, &two); },
+               [&](Attempt &a) { const mc_status st = mc_batch_run(a.b, 1, &one); return st != MC_OK ? st : mc_batch_run(a.b, 1, &two); });
+    every_call("batch reset", mg, batch, [](Attempt &a) { return mc_batch_reset(a.b); });
+    every_call("batch read", mg, batch, [](Attempt &a) {
+        return mc_batch_tally_read(a.b, a.out.data(), nullptr, nullptr, nullptr, a.out.size());
+    });
+}
+
 int main(int argc, char **argv)
 {
     if (argc < 6) return 2;
     ce = argv[2]; xs = argv[3]; mg = argv[4]; tmp = argv[5];
     const struct { const char *name; void (*run)(); } all[] = {
         {"concurrent reads", concurrent_reads}, {"not loaded", not_loaded}, {"deeper stack", deeper_stack}, {"failed query", failed_query},
-        {"failed reduce", failed_reduce}};
+        {"failed reduce", failed_reduce}, {"failed calls", failed_calls}};
     for (const auto &s : all)
         if (std::strcmp(s.name, argv[1]) == 0) {
             s.run();

@@ -36,6 +36,7 @@ def check(tmp_path_factory):
     return run
 
 
-@pytest.mark.parametrize("scenario", ["concurrent reads", "not loaded", "deeper stack", "failed query", "failed reduce"])
+@pytest.mark.parametrize("scenario", ["concurrent reads", "not loaded", "deeper stack", "failed query", "failed reduce",
+                                      "failed calls"])
 def test_host_engine(check, scenario):
     check(scenario)
