@@ -98,6 +98,8 @@ extern "C" mc_status mc_run_replay_noalloc(mc_problem *p, uint64_t first, uint64
     double *hist = reinterpret_cast<double *>(b + kCtrlBytes + stack_bytes);
     // whole groups of 8, the folds' vector width (kMinChunk is one)
     const uint64_t chunk = ((kScratchBytes - kCtrlBytes - stack_bytes) / row_bytes) & ~(uint64_t)7;
+    // the columns' length: every launch clears them, so no more than the run uses
+    const uint64_t ld = hist_rows(std::min(chunk, n));
 
     // the array keeps the previous call's contents: clear what starts at zero
     // (the caller's arrays hold exactly n_bins doubles, none when n_bins is 0)
@@ -115,7 +117,7 @@ extern "C" mc_status mc_run_replay_noalloc(mc_problem *p, uint64_t first, uint64
         A.n = cn;
         A.seed = seed;
         A.hist = hist;
-        A.hist_ld = chunk;
+        A.hist_ld = ld;
         A.stack = stack;
         A.stack_depth = kDepth;
         A.counters = cnt;
@@ -124,7 +126,7 @@ extern "C" mc_status mc_run_replay_noalloc(mc_problem *p, uint64_t first, uint64
         A.next = next;
         if ((e = cudaMemsetAsync(next, 0, sizeof(unsigned int), d.stream)) != cudaSuccess ||
             (e = launch_history_fp64(d.dt, A, true, kThreads / kBlock, kBlock, d.stream)) != cudaSuccess ||
-            (e = launch_fold_ordered(hist, cn, chunk, d.dt.n_bins, d_sum, d_sumsq, d.stream)) != cudaSuccess) {
+            (e = launch_fold_ordered(hist, cn, ld, d.dt.n_bins, d_sum, d_sumsq, d.stream)) != cudaSuccess) {
             p->err = cuda_msg(e, "mc_run_replay_noalloc launch");
             return MC_ERR_CUDA;
         }

@@ -258,13 +258,35 @@ static void failed_calls()
     });
 }
 
+// The replay without allocation clears the rows that it uses, not its scratch.
+static void noalloc_clears()
+{
+    Attempt a(mg);
+    size_t bins = 0;
+    uint32_t ne = 0;
+    mc_tally_count(a.p, &ne);
+    for (uint32_t e = 0; e < ne; ++e) {
+        uint64_t n = 0;
+        mc_tally_size(a.p, e, &n);
+        bins += n;
+    }
+    for (uint64_t n : {1, 8, 9, 1000}) {
+        fake::reset();
+        WANT(mc_run_replay_noalloc(a.p, 0, n, 1, a.out.data(), a.out.data() + 1024) == MC_OK);
+        size_t most = 0;
+        for (const fake::Fill &f : fake::fills()) most = f.bytes > most ? f.bytes : most;
+        WANT(most <= 4096 || most == (n + 7) / 8 * 8 * bins * sizeof(double));
+    }
+}
+
 int main(int argc, char **argv)
 {
     if (argc < 6) return 2;
     ce = argv[2]; xs = argv[3]; mg = argv[4]; tmp = argv[5];
     const struct { const char *name; void (*run)(); } all[] = {
         {"concurrent reads", concurrent_reads}, {"not loaded", not_loaded}, {"deeper stack", deeper_stack}, {"failed query", failed_query},
-        {"failed reduce", failed_reduce}, {"failed calls", failed_calls}};
+        {"failed reduce", failed_reduce}, {"failed calls", failed_calls},
+        {"noalloc clears", noalloc_clears}};
     for (const auto &s : all)
         if (std::strcmp(s.name, argv[1]) == 0) {
             s.run();

@@ -37,6 +37,6 @@ def check(tmp_path_factory):
 
 
 @pytest.mark.parametrize("scenario", ["concurrent reads", "not loaded", "deeper stack", "failed query", "failed reduce",
-                                      "failed calls"])
+                                      "failed calls", "noalloc clears"])
 def test_host_engine(check, scenario):
     check(scenario)
