@@ -117,7 +117,7 @@ cudaError_t launch_exact_normalize(long long *ex, long long n_bins, cudaStream_t
 // Bytes of one FP64 split-stack entry.
 size_t fp64_particle_bytes();
 
-// Launch shape of the FP64 history kernel for n histories on this device.
+// Launch shape of the FP64 history kernel for n histories a launch on this device.
 struct HistoryShape {
     int grid, lanes;
 };

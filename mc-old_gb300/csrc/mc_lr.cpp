@@ -94,11 +94,11 @@ mc_status run_params(mc_problem *p, const double *params, uint64_t n, uint64_t s
 
     const int block = 128;
     const uint32_t depth = 32;
-    const HistoryShape shape = history_fp64_shape(n, true);
-    const int grid = shape.grid;
-    const uint64_t threads = (uint64_t)grid * block;
     uint64_t chunk = (uint64_t)((1ull << 30) / (row * sizeof(double)));
     chunk = std::max<uint64_t>(1, std::min<uint64_t>({chunk, 1u << 22, n}));
+    const HistoryShape shape = history_fp64_shape(chunk, true);
+    const int grid = shape.grid;
+    const uint64_t threads = (uint64_t)grid * block;
     const uint64_t ld = hist_rows(chunk);
     if (!devbuf_reserve(S.rows, (size_t)ld * row * sizeof(double)) ||
         !devbuf_reserve(S.stack, (size_t)threads * depth * fp64_particle_bytes()) ||

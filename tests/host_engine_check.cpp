@@ -1,7 +1,7 @@
 // host_engine_check.cpp -- the host side of the library over a fake CUDA runtime
 // (fake_cudart.h).  argv: the scenario, then a continuous-energy problem's
-// folder, its cross-section folder and a one-group problem's folder.  Prints
-// "ok", or what is wrong.
+// folder, its cross-section folder, a one-group problem's folder, that of one
+// with many bins and a folder to write to.  Prints "ok", or what is wrong.
 #include <cstdio>
 #include <cstring>
 #include <functional>
@@ -12,7 +12,8 @@
 #include "fake_cudart.h"
 #include "mcgpu.h"
 
-static std::string ce, xs, mg, tmp;
+static std::string ce, xs, mg, tmp, wide;
+constexpr size_t kWideBins = 20003;   // of the wide problem (4 layers, one group)
 static int bad = 0;
 #define WANT(x)                                                          \
     do {                                                                 \
@@ -279,14 +280,45 @@ static void noalloc_clears()
     }
 }
 
+// The FP64 kernels' launch shape is that of the histories of one launch, not of
+// the whole run: few of them are spread over all schedulers.
+static void launch_shape()
+{
+    Attempt a(ce);
+    auto grid = [&](uint32_t chunk, uint64_t n, mc_mode m) {
+        const mc_tune t = tuned(0, chunk);
+        fake::reset();
+        WANT(mc_run(a.p, 0, n, 1, m, &t) == MC_OK);
+        unsigned g = 0;
+        for (const fake::Launch &l : fake::launches())
+            if (l.kernel.find("k_history_fp64") != std::string::npos) { WANT(g == 0 || g == l.grid); g = l.grid; }
+        return g;
+    };
+    for (mc_mode m : {MC_FP64_REPLAY, MC_FP64_PLAIN})
+        for (uint32_t chunk : {1u, 61u, 600u, 5000u}) WANT(grid(chunk, 100000, m) == grid(chunk, chunk, m));
+    WANT(grid(61, 100000, MC_FP64_REPLAY) == 16);      // four warps to a CTA, a history to a warp
+    // derivatives of a problem of so many columns that 1 GiB holds few histories
+    Attempt b(wide);
+    std::vector<double> par(128), out((size_t)2 * 4 * kWideBins), sg(out.size());
+    WANT(mc_lr_params(b.p, par.data(), 128) == MC_OK);
+    auto lr_grid = [&](uint64_t n) {
+        fake::reset();
+        WANT(mc_backward(b.p, par.data(), n, 1, out.data(), sg.data()) == MC_OK);
+        for (const fake::Launch &l : fake::launches())
+            if (l.kernel.find("k_history_fp64") != std::string::npos) return l.grid;
+        return 0u;
+    };
+    WANT(lr_grid(3000) == lr_grid((1u << 30) / 8 / 13 / kWideBins));
+}
+
 int main(int argc, char **argv)
 {
-    if (argc < 6) return 2;
-    ce = argv[2]; xs = argv[3]; mg = argv[4]; tmp = argv[5];
+    if (argc < 7) return 2;
+    ce = argv[2]; xs = argv[3]; mg = argv[4]; wide = argv[5]; tmp = argv[6];
     const struct { const char *name; void (*run)(); } all[] = {
         {"concurrent reads", concurrent_reads}, {"not loaded", not_loaded}, {"deeper stack", deeper_stack}, {"failed query", failed_query},
         {"failed reduce", failed_reduce}, {"failed calls", failed_calls},
-        {"noalloc clears", noalloc_clears}};
+        {"noalloc clears", noalloc_clears}, {"launch shape", launch_shape}};
     for (const auto &s : all)
         if (std::strcmp(s.name, argv[1]) == 0) {
             s.run();

@@ -28,15 +28,22 @@ def check(tmp_path_factory):
     assert r.returncode == 0, r.stderr[-3000:]
     ce = W.ce_sphere(str(d / "ce"), n_points=300, n_spectrum=10)
     mg = W.mg_layered_slab(str(d / "mg"), n_regions=4, detectors=True)
+    wide = W.mg_layered_slab(str(d / "wide"), n_regions=4)
+    many = "".join(f'<estimator name="w{i}" scores="flux"><cell name="c{i % 4}"/><filter type="energy" grid_linear="0 1 {k}"/></estimator>'
+                   for i, k in enumerate((10_000, 10_002)))     # with the transmitted current 20,003 bins
+    with open(wide + "/input.xml") as f:
+        s = f.read()
+    with open(wide + "/input.xml", "w") as f:
+        f.write(s.replace("</estimators>", many + "</estimators>"))
 
     def run(scenario):
-        r = subprocess.run([exe, scenario, ce, os.path.join(ce, "xs_library"), mg, str(d)], capture_output=True, text=True,
+        r = subprocess.run([exe, scenario, ce, os.path.join(ce, "xs_library"), mg, wide, str(d)], capture_output=True, text=True,
                            timeout=300)
         assert r.returncode == 0 and r.stdout.strip() == "ok", r.stdout[-3000:] + r.stderr[-1000:]
     return run
 
 
 @pytest.mark.parametrize("scenario", ["concurrent reads", "not loaded", "deeper stack", "failed query", "failed reduce",
-                                      "failed calls", "noalloc clears"])
+                                      "failed calls", "noalloc clears", "launch shape"])
 def test_host_engine(check, scenario):
     check(scenario)
