@@ -92,8 +92,21 @@ cudaError_t launch_history_fp64(const DevTables &T, const HistoryArgs &A, bool r
 
 // Per-history totals are kept column by column, [column][ld]: the folds read
 // a column's histories as contiguous vectors, and neighbouring histories that
-// score the same bin share sectors.  Room of n histories in a column:
-inline uint64_t hist_rows(uint64_t n) { return (n + 7) & ~(uint64_t)7; }
+// score the same bin share sectors.  Room of n histories in a column (whole
+// 16-byte vectors; whole sectors where there are several):
+inline uint64_t hist_rows(uint64_t n) { return n < 8 ? (n + 1) & ~(uint64_t)1 : (n + 7) & ~(uint64_t)7; }
+
+// Histories that one launch of a run of n takes: as many as 1 GiB of `cols`
+// columns holds (two of one history at the least), or as the caller asks for.
+inline uint64_t hist_chunk(uint64_t cols, uint64_t n, uint64_t asked)
+{
+    uint64_t chunk = (1ull << 30) / (cols * sizeof(double));
+    chunk &= ~(uint64_t)(chunk < 8 ? 1 : 7);      // (hist_rows pads)
+    if (asked) chunk = asked;
+    if (chunk > 1u << 22) chunk = 1u << 22;
+    if (chunk > n) chunk = n;
+    return chunk > 0 ? chunk : 1;
+}
 
 // Folds a chunk's per-history totals into sum / sq in history order (the bits
 // of the reference's end_history loop).

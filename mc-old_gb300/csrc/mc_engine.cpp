@@ -294,11 +294,7 @@ mc_status run_fp64(const Tables &t, DeviceProblem &d, uint64_t first, uint64_t n
     if (t.comb_teeth > 0 && !(tune && tune->stack_depth)) depth = std::max<uint32_t>(depth, (uint32_t)t.comb_teeth + 32);
     const bool want_digest = tune && tune->record_digests;
     const long long nb = std::max<long long>(d.dt.n_bins, 1);
-    // chunk: histories whose per-history rows are kept before the fold;
-    // bounded to ~1 GiB of rows
-    uint64_t chunk = (tune && tune->chunk) ? tune->chunk : (uint64_t)((1ull << 30) / (nb * sizeof(double)));
-    chunk = std::max<uint64_t>(1, std::min<uint64_t>(chunk, 1u << 22));
-    chunk = std::min<uint64_t>(chunk, n);
+    const uint64_t chunk = hist_chunk((uint64_t)nb, n, tune ? tune->chunk : 0);
     HistoryShape shape = history_fp64_shape(chunk, t.mg_groups > 0);
     if (tune && tune->grid_blocks) shape = {(int)tune->grid_blocks, 32};
     const int grid = shape.grid;

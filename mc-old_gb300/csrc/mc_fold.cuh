@@ -83,10 +83,10 @@ __device__ __noinline__ FoldMap fold_map(const double (&v)[kFoldValues], int es,
 }
 
 // One chain: block (bin, which), which = 0 the sum of the column's values,
-// 1 the sum of their squares.  hist is [bins][ld], ld a multiple of 8 and at
-// least n, zero from n on.  Adding zero changes nothing, and most histories
-// score few bins, so the column's nonzero values go through a ring in shared
-// memory and every step scans kStep of them.
+// 1 the sum of their squares.  hist is [bins][ld], ld even and at least n, zero
+// from n on.  Adding zero changes nothing, and most histories score few bins,
+// so the column's nonzero values go through a ring in shared memory and every
+// step scans kStep of them.
 __global__ void __launch_bounds__(kFoldThreads) k_fold_ordered(const double *__restrict__ hist, uint32_t n,
                                                                uint64_t ld, double *__restrict__ sum,
                                                                double *__restrict__ sq)
@@ -111,11 +111,11 @@ __global__ void __launch_bounds__(kFoldThreads) k_fold_ordered(const double *__r
     // the column's next values, kFoldAhead blocks of kStep histories ahead
     double nxt[kFoldAhead][kFoldValues];
     auto fetch = [&](double (&to)[kFoldValues], uint64_t at) {
-        const uint64_t h = at + (uint64_t)t * kFoldValues;   // a multiple of 8, as ld
+        const uint64_t h = at + (uint64_t)t * kFoldValues;
         const double2 *p = reinterpret_cast<const double2 *>(col + h);
 #pragma unroll
         for (int j = 0; j < kFoldValues / 2; ++j) {
-            const double2 x = h < n ? p[j] : double2{0.0, 0.0};
+            const double2 x = h + 2 * j < n ? p[j] : double2{0.0, 0.0};   // zero from n to its pair's end
             to[2 * j] = x.x;
             to[2 * j + 1] = x.y;
         }

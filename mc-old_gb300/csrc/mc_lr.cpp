@@ -94,8 +94,7 @@ mc_status run_params(mc_problem *p, const double *params, uint64_t n, uint64_t s
 
     const int block = 128;
     const uint32_t depth = 32;
-    uint64_t chunk = (uint64_t)((1ull << 30) / (row * sizeof(double)));
-    chunk = std::max<uint64_t>(1, std::min<uint64_t>({chunk, 1u << 22, n}));
+    const uint64_t chunk = hist_chunk((uint64_t)row, n, 0);
     const HistoryShape shape = history_fp64_shape(chunk, true);
     const int grid = shape.grid;
     const uint64_t threads = (uint64_t)grid * block;

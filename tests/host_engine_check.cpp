@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "fake_cudart.h"
+#include "mc_device.h"
 #include "mcgpu.h"
 
 static std::string ce, xs, mg, tmp, wide;
@@ -311,6 +312,22 @@ static void launch_shape()
     WANT(lr_grid(3000) == lr_grid((1u << 30) / 8 / 13 / kWideBins));
 }
 
+// The columns of one launch keep within 1 GiB, or two histories.
+static void row_bound()
+{
+    const double GiB = (double)(1u << 30);
+    for (double c = 1.0; c < 4e8; c *= 1.013)
+        for (uint64_t n : {(uint64_t)1, (uint64_t)5, (uint64_t)1000, (uint64_t)1 << 40}) {
+            const uint64_t cols = (uint64_t)c, chunk = mc::hist_chunk(cols, n, 0), rows = mc::hist_rows(chunk);
+            const double bytes = 8.0 * (double)cols * (double)rows;
+            WANT(chunk >= 1 && chunk <= n && rows >= chunk && rows % 2 == 0 && rows < chunk + 8);
+            WANT(bytes <= GiB || rows == 2);
+            // no launch is more than a vector shorter than the bound allows
+            if (chunk < n && chunk < 1u << 22) WANT((double)(chunk + 8) * 8.0 * (double)cols > GiB);
+        }
+    WANT(mc::hist_chunk(10, 1000, 61) == 61 && mc::hist_chunk(10, 50, 61) == 50 && mc::hist_chunk(10, (uint64_t)1 << 40, (uint64_t)1 << 30) == 1u << 22);
+}
+
 int main(int argc, char **argv)
 {
     if (argc < 7) return 2;
@@ -318,7 +335,8 @@ int main(int argc, char **argv)
     const struct { const char *name; void (*run)(); } all[] = {
         {"concurrent reads", concurrent_reads}, {"not loaded", not_loaded}, {"deeper stack", deeper_stack}, {"failed query", failed_query},
         {"failed reduce", failed_reduce}, {"failed calls", failed_calls},
-        {"noalloc clears", noalloc_clears}, {"launch shape", launch_shape}};
+        {"noalloc clears", noalloc_clears}, {"launch shape", launch_shape},
+        {"row bound", row_bound}};
     for (const auto &s : all)
         if (std::strcmp(s.name, argv[1]) == 0) {
             s.run();

@@ -44,6 +44,6 @@ def check(tmp_path_factory):
 
 
 @pytest.mark.parametrize("scenario", ["concurrent reads", "not loaded", "deeper stack", "failed query", "failed reduce",
-                                      "failed calls", "noalloc clears", "launch shape"])
+                                      "failed calls", "noalloc clears", "launch shape", "row bound"])
 def test_host_engine(check, scenario):
     check(scenario)
