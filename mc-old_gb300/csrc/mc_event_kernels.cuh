@@ -463,7 +463,10 @@ __device__ __forceinline__ float quad_root(float a, float h, float c, bool on)
 // The distance's polynomial t^2 + 2 h t + c (c here without compensation) is
 // taken at T, a little beyond l; m bounds, several times over, the rounding of
 // c, of the value at T and of what the root's own rounding amounts to as a
-// change of c (a few 2^-24 (T^2 + |d|^2 + r^2), as |h| <= |d|).  Inside, the
+// change of c: a few 2^-24 (T^2 + |d|^2 + r^2).  (h is the one value that the
+// distance is computed from, and next to a root |h| T is (T^2 + |c|) / 2 at
+// most, next to a tangent h^2 is c; so no term grows with the direction's
+// length, which a source may give other than 1.)  Inside, the
 // sphere is farther if the polynomial is still negative at T; outside, if the
 // flight leads away, passes by, or ends while the polynomial is positive and
 // still falling.  NaN and infinities (a void's flight) answer no.  (Shield of
