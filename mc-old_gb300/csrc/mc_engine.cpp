@@ -86,11 +86,19 @@ struct Packer {
 // order and padding are part of the file format.
 uint64_t table_fingerprint(const Tables &t)
 {
-    std::vector<char> buf;
+    uint64_t h = 0xCBF29CE484222325ULL;
+    size_t at = 0;
+    auto zeros = [&](size_t n) {
+        at += n;
+        while (n--) h *= 0x100000001B3ULL;
+    };
     auto add = [&](const auto &v) {
-        const size_t size = sizeof(v[0]), off = (buf.size() + 255) & ~(size_t)255;
-        buf.resize(off + std::max<size_t>(v.size() * size, 8), 0);
-        if (!v.empty()) std::memcpy(buf.data() + off, v.data(), v.size() * size);
+        zeros((256 - at % 256) % 256);
+        const unsigned char *b = reinterpret_cast<const unsigned char *>(v.data());
+        const size_t bytes = v.size() * sizeof(v[0]);
+        for (size_t i = 0; i < bytes; ++i) h = (h ^ b[i]) * 0x100000001B3ULL;
+        at += bytes;
+        if (bytes < 8) zeros(8 - bytes);      // (an empty table takes eight)
     };
     add(t.surf_type); add(t.surf_bc); add(t.surf_coef); add(t.cell_imp); add(t.cell_mat);
     add(t.cell_surf_off); add(t.cell_surf); add(t.cell_sense); add(t.cell_tl_off); add(t.cell_tl);
@@ -102,8 +110,6 @@ uint64_t table_fingerprint(const Tables &t)
     add(t.filt_grid); add(t.est_factor); add(t.est_factor_off); add(t.est_bin_off); add(t.src_pos);
     add(t.src_dir_par); add(t.src_e_par); add(t.src_cdf); add(t.src_cell); add(t.src_dir_kind);
     add(t.src_e_kind); add(t.src_group);
-    uint64_t h = 0xCBF29CE484222325ULL;
-    for (const char c : buf) h = (h ^ (unsigned char)c) * 0x100000001B3ULL;
     return h;
 }
 

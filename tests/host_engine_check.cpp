@@ -328,6 +328,24 @@ static void row_bound()
     WANT(mc::hist_chunk(10, 1000, 61) == 61 && mc::hist_chunk(10, 50, 61) == 50 && mc::hist_chunk(10, (uint64_t)1 << 40, (uint64_t)1 << 30) == 1u << 22);
 }
 
+// Saved states are found again by later builds: their problems' keys, as the
+// first builds that saved states wrote them.
+static void state_keys()
+{
+    const struct { const std::string &d; uint64_t key; } known[] = {{ce, 0x1FD0E85AACFAC887ull}, {mg, 0xA429E906F037B4E1ull}};
+    for (const auto &k : known) {
+        Attempt a(k.d);
+        const std::string f = tmp + "/keyed";
+        WANT(mc_state_save(a.p, f.c_str()) == MC_OK && mc_state_load(a.p, f.c_str()) == MC_OK);
+        uint64_t head[5] = {};
+        if (FILE *h = std::fopen(f.c_str(), "rb")) {
+            WANT(std::fread(head, 8, 5, h) == 5);
+            std::fclose(h);
+        }
+        WANT(head[4] == k.key);
+    }
+}
+
 int main(int argc, char **argv)
 {
     if (argc < 7) return 2;
@@ -336,7 +354,7 @@ int main(int argc, char **argv)
         {"concurrent reads", concurrent_reads}, {"not loaded", not_loaded}, {"deeper stack", deeper_stack}, {"failed query", failed_query},
         {"failed reduce", failed_reduce}, {"failed calls", failed_calls},
         {"noalloc clears", noalloc_clears}, {"launch shape", launch_shape},
-        {"row bound", row_bound}};
+        {"row bound", row_bound}, {"state keys", state_keys}};
     for (const auto &s : all)
         if (std::strcmp(s.name, argv[1]) == 0) {
             s.run();

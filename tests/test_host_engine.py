@@ -44,6 +44,7 @@ def check(tmp_path_factory):
 
 
 @pytest.mark.parametrize("scenario", ["concurrent reads", "not loaded", "deeper stack", "failed query", "failed reduce",
-                                      "failed calls", "noalloc clears", "launch shape", "row bound"])
+                                      "failed calls", "noalloc clears", "launch shape", "row bound",
+                                      "state keys"])
 def test_host_engine(check, scenario):
     check(scenario)
