@@ -170,7 +170,6 @@ __device__ __forceinline__ void bank_store(const BankArgs &B, const EvTables &V,
 // a dead particle: its slot empties (all lanes call this, for the count of
 // live slots), its history's row is folded when it was the history's last
 // particle
-template <int kFl>
 __device__ __forceinline__ void bank_retire(Ctx &C, const BankArgs &B, bool dies, int s, int hslot)
 {
     const unsigned dm = __ballot_sync(0xffffffffu, dies);
@@ -184,7 +183,7 @@ __device__ __forceinline__ void bank_retire(Ctx &C, const BankArgs &B, bool dies
         if (B.may_split) __threadfence();
         if (atomicSub(&B.hlive[hslot], 1) == 1) {
             if (B.may_split) __threadfence();
-            history_fold<kFl>(C, hslot, 0);
+            history_fold(C, hslot, 0);
         }
     }
 }
@@ -346,7 +345,7 @@ __global__ void __launch_bounds__(kBankBlock) k_bank_collide(const EvTables V, c
                 if (is_mg<kFl>(V)) B.meta[s] = make_int4(p.cell, p.surf, p.g, p.hslot);
             }
         }
-        bank_retire<kFl>(C, B, act && !alive, s, act ? p.hslot : 0);
+        bank_retire(C, B, act && !alive, s, act ? p.hslot : 0);
     }
     bank_flush(B, s_cnt, s_status, &A, sums, V.n_bins);
 }
@@ -406,7 +405,7 @@ __global__ void __launch_bounds__(kBankBlock) k_bank_cross(const EvTables V, con
             alive = event_cross<kFl>(C, V, R, p, f, push);
             if (alive) bank_store(B, V, s, p);
         }
-        bank_retire<kFl>(C, B, act && !alive, s, act ? p.hslot : 0);
+        bank_retire(C, B, act && !alive, s, act ? p.hslot : 0);
     }
     bank_flush(B, s_cnt, s_status, &A, sums, V.n_bins);
     // the last block to finish closes the iteration

@@ -380,28 +380,12 @@ struct Flight {
     int S, sense;   // surface to cross and the cell's sense of it
 };
 
-enum { XT = 0, XS = 1, XC = 2 };
-
 // whether this particle's problem is multigroup, folded at compile time
 // where the flavour decides it
 template <int kFl>
 __device__ __forceinline__ bool is_mg(const EvTables &V)
 {
     return fl_multigroup(kFl) ? true : (kFl == FL_CE ? false : V.G > 0);
-}
-
-// macroscopic cross section of cell material at the particle's energy/group
-template <int kFl>
-__device__ __forceinline__ float macro(Ctx &C, int m, int which, const PState &p)
-{
-    const EvTables &V = *C.V;
-    C.cnt[C_XS]++;
-    if (is_mg<kFl>(V)) {
-        const int i = m * V.G + p.g;
-        return which == XT ? __ldg(V.mg_total + i) : (which == XS ? __ldg(V.mg_scat_tot + i) : __ldg(V.mg_capture + i));
-    }
-    const XsVal x = xs_eval(V, m, p.E);
-    return which == XT ? x.st : (which == XS ? x.ss : x.sc);
 }
 
 // ---------------------------------------------------------------------------
@@ -743,30 +727,19 @@ __device__ __forceinline__ bool estimator_score_simple(Ctx &C, int e, const PSta
 }
 
 
-// Estimator::score (Estimator.cpp:298-336).  pre / fixed as for
-// estimator_score_simple; the general path recomputes every filter.
+// Estimator::score (Estimator.cpp:298-336), for the full kernels.  pre / fixed as
+// for estimator_score_simple; the general path recomputes every filter.  l_in is
+// finite (score_list), or the loop below would never advance.
 template <int kFl>
 __device__ void estimator_score(Ctx &C, int e, const PState &p, float t_old, float speed, float l_in, int pre,
                                 int fixed)
 {
     const EvTables &V = *C.V;
-    if (!(fabsf(l_in) <= FLT_MAX)) {   // non-finite track: the loop below would never advance
-        atomicCAS(C.s_status, 0, DS_NAN);
-        return;
-    }
     if (estimator_score_simple<kFl>(C, e, p, l_in, pre, fixed)) return;
-    if constexpr (!fl_full(kFl)) {
-        atomicCAS(C.s_status, 0, DS_OVERFLOW);   // unreachable: time filters get the full kernels
-        return;
-    }
     const int f0 = V.est_filt_off[e], nf = V.est_filt_off[e + 1] - f0;
     const int s0 = V.est_score_off[e], ns = V.est_score_off[e + 1] - s0;
     const int *fac = V.est_factor + V.est_factor_off[e];
     const int base = V.est_bin_off[e];
-    if (!(fabsf(l_in) <= FLT_MAX)) {   // non-finite track: the loop below would never advance
-        atomicCAS(C.s_status, 0, DS_NAN);
-        return;
-    }
     Il il[kMaxIl];
     int off[kMaxFilt + 1], nil[kMaxFilt], idx[kMaxFilt];
     off[0] = 0;
@@ -922,7 +895,6 @@ __device__ __forceinline__ void fold_first(Ctx &C, int prob)
 
 // Folds a finished history's row into the sums (Estimator.cpp:339-346):
 // the CTA's shared sums, a replica, or the problem's global sums.
-template <int kFl>
 __device__ void history_fold(Ctx &C, int hslot, int prob)
 {
     const size_t row = (size_t)blockIdx.x * C.A->tile + hslot;
@@ -938,8 +910,6 @@ __device__ void history_fold(Ctx &C, int hslot, int prob)
             fold_add<false>(*C.A, C.T.ssum(), C.T.nsum, at, b, row_take(acc + b));
         }
     }
-    C.cbin = -1;
-    C.cval = 0.0;
 }
 
 // The fold of k_track, by the whole warp: the touched sectors of every history
@@ -1016,7 +986,7 @@ __device__ __forceinline__ void particle_dies(Ctx &C, int s, int hslot)
     atomicSub(C.s_nlive, 1);
     if (atomicSub(&C.T.live()[hslot], 1) == 1) {
         __threadfence_block();
-        history_fold<FL_ALL>(C, hslot, C.T.hprob()[hslot]);
+        history_fold(C, hslot, C.T.hprob()[hslot]);
         const int k = atomicAdd(C.s_nhfree, 1);
         C.T.hfree()[k] = hslot;
     }
@@ -1308,7 +1278,8 @@ __device__ __forceinline__ int event_advance(Ctx &C, const EvTables &V, Rng32 &R
     f.xa = XsAt{m, 0, 0.f};
     if (m >= 0) {
         if (is_mg<kFl>(V)) {
-            f.sig = macro<kFl>(C, m, XT, p);
+            f.sig = __ldg(V.mg_total + m * V.G + p.g);
+            C.cnt[C_XS]++;
         } else {
             const XsVal x = xs_eval(V, m, p.E);
             f.xa = x.at;

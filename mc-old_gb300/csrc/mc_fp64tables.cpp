@@ -45,7 +45,6 @@ void build_grid(const double *E, int len, Fp64Tables &f, Grid64 &g)
     const uint64_t lo = bits_of(E[0]), hi = bits_of(E[len - 1]);
     int shift = 52;
     while (shift > 0 && (hi >> (shift - 1)) - (lo >> (shift - 1)) + 1 <= 2 * (uint64_t)len) --shift;
-    if ((hi >> shift) - (lo >> shift) + 1 > 4096 + 2 * (uint64_t)len) { g.fast = 0; return; }
     g.shift = shift;
     g.key0 = lo >> shift;
     g.n_bkt = (int32_t)((hi >> shift) - g.key0 + 1);
