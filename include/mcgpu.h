@@ -122,8 +122,9 @@ typedef struct {
     uint32_t launches;        /* kernels launched by the last mc_run (mixed
                                  mode: 2 where a second kernel adds
                                  replicated sums: a batch, a problem of more
-                                 than 4096 bins, a long run that is not
-                                 multigroup or scores in cells) */
+                                 than 4096 bins, a long continuous-energy
+                                 run, a long multigroup one that scores in
+                                 cells) */
     uint32_t reserved;        /* 0 (pads the struct to 8 bytes) */
 } mc_counters;
 

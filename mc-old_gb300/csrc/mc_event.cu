@@ -265,8 +265,8 @@ static mc_status event_launch_shape(const DeviceProblem &d, const mc_tune *tune,
                                     Residency &R, EvLaunch &L, std::string &err)
 {
     L.flavor = flavor;
-    // measured at 2 / 4 / 8: shield 69.3 / 67.3 / 67.9 ms, deep slab 11.7 /
-    // 11.7 / 11.9 ms, 256 shields 18.3 / 18.1 / 18.6 ms
+    // measured at 2 / 4 / 8: shield 63.7 / 61.8 / 62.3 ms, deep slab 11.9 /
+    // 11.9 / 12.0 ms, 256 shields 18.4 / 18.2 / 18.7 ms
     const int refill_default = 4;
     L.refill = (tune && tune->refill) ? (int)tune->refill : (tuned.refill ? (int)tuned.refill : refill_default);
     if (L.refill < 1 || L.refill > 32) { err = "refill must be 1..32"; return MC_ERR_ARG; }
@@ -309,14 +309,14 @@ static mc_status event_launch_shape(const DeviceProblem &d, const mc_tune *tune,
     const bool own_minb = tune && tune->blocks_per_sm;
     // the per-thread kernel's CTAs per SM: no more than give every history a
     // lane, as fewer CTAs leave a thread more registers (shield of 20,000
-    // histories: 0.70 ms at 4, 0.75 at 6, 0.87 at 8); a full GPU runs 8 for
-    // multigroup problems (deep slab 11.7 against 12.6 ms at 7, a batch of 256
-    // shields 18.1 against 18.6 ms), else 7, as those kernels spill at 8
-    // (shield 67.3 against 68.2 ms, one-group slab 1.67 against 1.77 ms).  The
-    // kernels that carry everything keep 4, their pair lists and spills in
-    // local memory (500,000 duct histories with a time filter 8.9 / 9.5 / 9.7 ms
-    // at 4 / 6 / 7, with the comb 3.3 / 4.1 / 4.5; a slab with two energy
-    // filters 4.9 / 5.3 / 5.9)
+    // histories: 0.65 ms at 4, 0.76 at 6, 0.96 at 8); a full GPU runs 8 for
+    // multigroup problems (deep slab 11.9 against 12.3 ms at 7, a batch of 256
+    // shields 18.2 against 18.5 ms), else 7, as those kernels spill at 8
+    // (shield 61.8 against 64.0 ms, one-group slab 1.55 against 1.59 ms).  The
+    // kernels that carry both physics and everything keep 4, their pair lists
+    // and spills in local memory (500,000 duct histories with a time filter 9.0 /
+    // 8.9 / 9.0 ms at 4 / 6 / 7, with the comb 3.3 / 3.5 / 3.7; a slab with two
+    // energy filters, whose long rows gain from company, 3.5 / 3.1 / 3.0)
     int minb_default = 4;
     if (L.kernel == 2) {
         const uint64_t lanes = (uint64_t)std::max(d.sms, 1) * kTrackBlock;

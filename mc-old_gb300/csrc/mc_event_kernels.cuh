@@ -1803,7 +1803,7 @@ struct __align__(16) SrcSlot {
     int prob;
     unsigned long long hist;
 };
-constexpr int kRing = 32;             // slots per warp: one refill of 32 on top of what is left
+constexpr int kRing = 32;             // slots per warp; a refill fills those that are free
 struct SrcRing {
     SrcSlot slot[kRing];
     unsigned long long last;          // histories handed out when this warp last took some

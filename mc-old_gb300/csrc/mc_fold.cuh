@@ -22,9 +22,9 @@
 // Bound and measure (GB300): the latency of the steps of the densest column
 // (barriers, shuffles, 64-bit shifts) and of its loads, three blocks of which
 // are in flight.  500,000 histories x 19 bins: 61.5 ms as one serial chain per
-// bin, 0.80 ms here; 50,000 x 931 derivative columns, signed and mostly zero:
-// 7.75 -> 0.45 ms, where the slowest column adds 6,700 values serially; 3,001 x
-// 180: 0.47 -> 0.08 ms.  (One block in flight, and squares multiplied in the
+// bin, 0.72 ms here; 50,000 x 931 derivative columns, signed and mostly zero:
+// 7.75 -> 0.44 ms, where the slowest column adds 6,700 values serially; 3,001 x
+// 180: 0.47 -> 0.04 ms.  (One block in flight, and squares multiplied in the
 // serial chain, whose every instruction takes the pipe 64 cycles: 0.87, 0.84
 // and 0.12 ms.)
 #pragma once

@@ -124,8 +124,8 @@ __device__ __forceinline__ double plog_unit(double x, const LnTable &T)
 }
 
 // preduce of x = 2 pi u (or pi/2 u): the quadrant follows from u's bits
-// (round-half-up of x 2/pi is (v + 2^49) >> 50, and v >> 51, for every v:
-// tests/fp64_check.cu), and the products n kPio2_i are constants.
+// (round-half-up of x 2/pi is (v + 2^49) >> 50, and v >> 51: sampled, and at
+// the limits, in tests/fp64_check.cu), and the products n kPio2_i are constants.
 __device__ __forceinline__ double reduce_quadrant(double x, int n)
 {
     if (n == 0) return x;

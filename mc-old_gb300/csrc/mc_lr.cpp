@@ -3,7 +3,7 @@
 // The reference has no derivative capability.  For one-group (multigroup,
 // G = 1) problems the parameters are every material's (Sigma_s, Sigma_a).
 // mc_forward runs the FP64 replay transport with those values; mc_backward
-// runs the likelihood-ratio kernel (k_history_fp64<true, true>), which
+// runs the likelihood-ratio kernel (k_history_fp64<true, F_LR>), which
 // carries each particle's score-function weights S_k = d ln(w x path
 // probability)/d param_k along the history and adds v S_k (plus the direct
 // dependence of a Sigma-weighted score) for every tally contribution v.  The
