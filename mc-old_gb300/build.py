@@ -51,6 +51,7 @@ SOURCES = [
     ("mc_event.cu", "fast"),
     ("mc_event_ce.cu", "fast"),
     ("mc_event_mg.cu", "fast"),
+    ("mc_event_mgs.cu", "fast"),
     ("mc_event_mgx.cu", "fast"),
     ("mc_event_all.cu", "fast"),
     ("mc_bank.cu", "fast"),

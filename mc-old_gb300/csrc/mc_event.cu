@@ -140,12 +140,12 @@ __global__ void k_batch_reduce(const EvArgs A, const int *rep_prob)
 }
 
 // the per-thread kernel's flavour for problems that are all multigroup (mg), all
-// continuous energy (ce) or both; full: one has a time filter, an estimator
-// without records or the comb
-int flavor_of(bool mg, bool ce, bool full)
+// continuous energy (ce) or both; general: one has an estimator without records,
+// full: one has a time filter or the comb
+int flavor_of(bool mg, bool ce, bool general, bool full)
 {
-    if (mg) return full ? FL_MGX : FL_MG;
-    return ce && !full ? FL_CE : FL_ALL;
+    if (mg) return full ? FL_MGX : (general ? FL_MGS : FL_MG);
+    return ce && !full && !general ? FL_CE : FL_ALL;
 }
 
 EvKernel pick_kernel(int minb, bool batch, int kernel, int flavor)
@@ -153,6 +153,7 @@ EvKernel pick_kernel(int minb, bool batch, int kernel, int flavor)
     if (kernel == 2) {
         if (flavor == FL_CE) return pick_track_ce(minb, batch);
         if (flavor == FL_MG) return pick_track_mg(minb, batch);
+        if (flavor == FL_MGS) return pick_track_mgs(minb, batch);
         if (flavor == FL_MGX) return pick_track_mgx(minb, batch);
         return pick_track_all(minb, batch);
     }
@@ -234,7 +235,7 @@ struct EvLaunch {
     int block = 256, tile = 512, minb = 4, grid = 0;
     int kernel = 1;         // 1: tile / event queues (k_event), 2: one particle per thread (k_track)
     int ovf_cap = 0;        // split-copy slots per CTA
-    int flavor = FL_ALL;    // per-thread kernel flavour (FL_ALL / FL_CE / FL_MG / FL_MGX)
+    int flavor = FL_ALL;    // per-thread kernel flavour (FL_ALL / FL_CE / FL_MG / FL_MGS / FL_MGX)
     uint32_t max_events = kMaxEvents;
     int refill = 1;         // k_track: idle lanes a warp gathers before it starts histories
     bool smem_sums = false; // the CTA's tally sums live in shared memory (else in replicas, EvArgs::n_rep)
@@ -266,8 +267,11 @@ static mc_status event_launch_shape(const DeviceProblem &d, const mc_tune *tune,
 {
     L.flavor = flavor;
     // measured at 2 / 4 / 8: shield 63.7 / 61.8 / 62.3 ms, deep slab 11.9 /
-    // 11.9 / 12.0 ms, 256 shields 18.4 / 18.2 / 18.7 ms
-    const int refill_default = 4;
+    // 11.9 / 12.0 ms, 256 shields 18.4 / 18.2 / 18.7 ms; where histories score
+    // in rows through several filters a warp's fold costs more, and is shared
+    // by more of them (4 / 8 / 12: deep slab 2.97 / 2.84 / 2.82 ms, layered slab
+    // 5.37 / 5.17 / 5.32, 256 shields 31.7 / 30.9 / 31.6)
+    const int refill_default = flavor == FL_MGS ? 8 : 4;
     L.refill = (tune && tune->refill) ? (int)tune->refill : (tuned.refill ? (int)tuned.refill : refill_default);
     if (L.refill < 1 || L.refill > 32) { err = "refill must be 1..32"; return MC_ERR_ARG; }
     L.kernel = (tune && tune->kernel) ? (int)tune->kernel : (tuned.kernel ? (int)tuned.kernel : 2);
@@ -312,7 +316,9 @@ static mc_status event_launch_shape(const DeviceProblem &d, const mc_tune *tune,
     // histories: 0.65 ms at 4, 0.76 at 6, 0.96 at 8); a full GPU runs 8 for
     // multigroup problems (deep slab 11.9 against 12.3 ms at 7, a batch of 256
     // shields 18.2 against 18.5 ms), else 7, as those kernels spill at 8
-    // (shield 61.8 against 64.0 ms, one-group slab 1.55 against 1.59 ms).  The
+    // (shield 61.8 against 64.0 ms, one-group slab 1.55 against 1.59 ms), and so
+    // does the multigroup kernel for estimators without records (6 / 7 / 8: deep
+    // slab 3.20 / 2.97 / 3.20 ms, 256 shields 33.6 / 31.7 / 37.1).  The
     // kernels that carry both physics and everything keep 4, their pair lists
     // and spills in local memory (500,000 duct histories with a time filter 9.0 /
     // 8.9 / 9.0 ms at 4 / 6 / 7, with the comb 3.3 / 3.5 / 3.7; a slab with two
@@ -320,7 +326,7 @@ static mc_status event_launch_shape(const DeviceProblem &d, const mc_tune *tune,
     int minb_default = 4;
     if (L.kernel == 2) {
         const uint64_t lanes = (uint64_t)std::max(d.sms, 1) * kTrackBlock;
-        minb_default = n <= 4 * lanes || flavor == FL_ALL ? 4 : (n <= 6 * lanes ? 6 : ((n <= 7 * lanes || !fl_lane_bin(flavor)) ? 7 : 8));
+        minb_default = n <= 4 * lanes || flavor == FL_ALL ? 4 : (n <= 6 * lanes ? 6 : ((n <= 7 * lanes || !fl_lane_bin(flavor) || flavor == FL_MGS) ? 7 : 8));
     }
     L.minb = own_minb ? (int)tune->blocks_per_sm
            : ((tuned.blocks_per_sm && tuned.kernel == (uint32_t)L.kernel) ? (int)tuned.blocks_per_sm : minb_default);
@@ -516,7 +522,7 @@ mc_status run_event(const Tables &t, DeviceProblem &d, uint64_t first, uint64_t 
     const long long nb = std::max<long long>(V.n_bins, 1);
     EvLaunch L;
     const int comb = t.comb_teeth > 0 ? t.comb_teeth : 0;
-    const int flavor = flavor_of(V.G > 0, V.G == 0, V.has_time || V.general || comb);
+    const int flavor = flavor_of(V.G > 0, V.G == 0, V.general, V.has_time || comb);
     mc_status st = event_launch_shape(d, tune, d.tuned, nb, n, false, flavor, comb, S.resident, L, err);
     if (st != MC_OK) return st;
     if (L.kernel == 3) {
@@ -680,14 +686,15 @@ mc_status batch_create(const std::vector<const Tables *> &tabs, const std::vecto
         b->row_nb = std::max<long long>(b->row_nb, views[i].n_bins);
     }
     // one flavour for the launch
-    bool all_mg = true, all_ce = true, any_full = false;
+    bool all_mg = true, all_ce = true, any_general = false, any_full = false;
     for (uint32_t i = 0; i < n; ++i) {
         all_mg = all_mg && views[i].G > 0;
         all_ce = all_ce && views[i].G == 0;
-        any_full = any_full || views[i].has_time || views[i].general || views[i].comb_teeth > 0;
+        any_general = any_general || views[i].general;
+        any_full = any_full || views[i].has_time || views[i].comb_teeth > 0;
         b->comb_teeth = std::max(b->comb_teeth, views[i].comb_teeth);
     }
-    b->flavor = flavor_of(all_mg, all_ce, any_full);
+    b->flavor = flavor_of(all_mg, all_ce, any_general, any_full);
     b->total = prefix[n];
     // replicas of every problem's bins: kBatchReplicas copies, fewer where
     // they would pass kBatchReplicaBytes

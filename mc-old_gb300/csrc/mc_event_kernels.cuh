@@ -2,8 +2,8 @@
 // event functions shared by both kernels, the tile kernel (k_event) and the
 // per-thread kernel (k_track).  Included by mc_event.cu (host side and the
 // tile kernel) and by one translation unit per per-thread kernel flavour
-// (mc_event_ce.cu, mc_event_mg.cu, mc_event_mgx.cu, mc_event_all.cu), so that the flavours
-// compile in parallel.
+// (mc_event_ce.cu, mc_event_mg.cu, mc_event_mgs.cu, mc_event_mgx.cu,
+// mc_event_all.cu), so that the flavours compile in parallel.
 #pragma once
 
 #include <cfloat>
@@ -76,21 +76,29 @@ enum TileArray {
 //           else has no record, EvTables::general) and the particle comb;
 //   FL_CE   continuous energy, records only;
 //   FL_MG   multigroup, records only;
+//   FL_MGS  multigroup, estimators without records too, but no time filter
+//           and no comb: one bin per filter, so no pair list, whose stack
+//           frame and spills a problem with two filters besides the cell paid
+//           for in FL_MGX (FL_MGX / FL_MGS: 10^7 deep-slab histories 3.53 /
+//           2.84 ms, layered slab 5.90 / 5.17; 256 shields 36.7 / 30.9);
 //   FL_MGX  multigroup, with the general scoring path and the comb.  A
 //           multigroup problem loses most of its speed without its sources
 //           from a ring, its first bin in registers and 8 CTAs per SM (FL_ALL /
 //           FL_MGX: 10^7 deep-slab histories with the comb 2.84 / 1.42 ms, with
-//           a time filter 7.3 / 5.2, with two filters besides the cell 5.0 /
-//           3.6; 256 shields, one of them with a time filter, 39.1 / 20.8);
+//           a time filter 7.3 / 5.2; 256 shields, one of them with a time
+//           filter, 39.1 / 20.8);
 //   FL_MGB  multigroup, records only, every tally through the history row
 //           (the event-split kernels: nothing stays in a thread's registers
 //           from one event kernel to the next).
-enum Flavor { FL_ALL = 0, FL_CE = 1, FL_MG = 2, FL_MGB = 3, FL_MGX = 4 };
-__host__ __device__ constexpr bool fl_multigroup(int fl) { return fl == FL_MG || fl == FL_MGB || fl == FL_MGX; }
+enum Flavor { FL_ALL = 0, FL_CE = 1, FL_MG = 2, FL_MGB = 3, FL_MGX = 4, FL_MGS = 5 };
+__host__ __device__ constexpr bool fl_multigroup(int fl)
+{
+    return fl == FL_MG || fl == FL_MGB || fl == FL_MGS || fl == FL_MGX;
+}
 // time filters, estimators without records and the comb
 __host__ __device__ constexpr bool fl_full(int fl) { return fl == FL_ALL || fl == FL_MGX; }
 // sources from a ring, and the first bin of a history in registers
-__host__ __device__ constexpr bool fl_lane_bin(int fl) { return fl == FL_MG || fl == FL_MGX; }
+__host__ __device__ constexpr bool fl_lane_bin(int fl) { return fl == FL_MG || fl == FL_MGS || fl == FL_MGX; }
 
 // 128 threads per CTA lets the register budget step through 128 / 80 / 72 /
 // 64 registers (4 / 6 / 7 / 8 CTAs per SM)
@@ -103,6 +111,7 @@ typedef void (*EvKernel)(const EvTables, const EvArgs);
 // translation unit each
 EvKernel pick_track_ce(int minb, bool batch);
 EvKernel pick_track_mg(int minb, bool batch);
+EvKernel pick_track_mgs(int minb, bool batch);
 EvKernel pick_track_mgx(int minb, bool batch);
 EvKernel pick_track_all(int minb, bool batch);
 
@@ -775,7 +784,8 @@ __device__ void estimator_score(Ctx &C, int e, const PState &p, float t_old, flo
 // The scores of one list of attachments; l_in and fixed as above; x: the flight
 // whose cross sections reaction scores use (kXs; behind a crossing only a
 // multigroup problem's have a record).  Nearly all take their bin
-// from the record and at most one filter.  The rest need the general path,
+// from the record and at most one filter.  The rest need the general path (in
+// FL_MGS, whose estimators have no time filter, its simple form),
 // which only the full kernels carry (EvTables::general): three inlined copies
 // were 17 of the continuous-energy kernel's 79 KB, and its loop is bound by
 // instruction fetches; out of line they cost it registers instead.
@@ -795,6 +805,7 @@ __device__ __forceinline__ void score_list(Ctx &C, const EvTables &V, const int4
         int bin = r.x;
         if (code == ATT_GENERAL) {
             if constexpr (fl_full(kFl)) estimator_score<kFl>(C, r.z, p, t_old, speed, l_in, bin, fixed);
+            else if constexpr (kFl == FL_MGS) estimator_score_simple<kFl>(C, r.z, p, l_in, bin, fixed);
             else atomicCAS(C.s_status, 0, DS_OVERFLOW);   // unreachable
             continue;
         }

@@ -1,5 +1,5 @@
-// mc_event_mgx.cu -- the per-thread kernels (k_track) for multigroup problems with time filters,
-// estimators without records or the particle comb.  Philox refills as in mc_event_mg.cu.
+// mc_event_mgx.cu -- the per-thread kernels (k_track) for multigroup problems with time filters
+// or the particle comb.  Philox refills as in mc_event_mg.cu.
 #define MC_EV_RNG_OUTLINE 1
 #include "mc_event_kernels.cuh"
 

@@ -1,5 +1,5 @@
 """Multigroup problems with a time filter, two filters besides the cell or the
-particle comb run a multigroup kernel too (csrc/mc_event_kernels.cuh, FL_MGX:
+particle comb run a multigroup kernel too (csrc/mc_event_kernels.cuh, FL_MGS and FL_MGX:
 per-CTA sums in shared memory, so one launch below the history count that
 takes replicas): the tile kernel's tallies, and with the comb, which that
 kernel has not, FP64 replay's."""
