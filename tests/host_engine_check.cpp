@@ -161,7 +161,7 @@ static void failed_reduce()
     auto run = [&](uint64_t n) { return mc_run(p, 0, n, 1, MC_MIXED_EVENT, &t); };
     auto cleared = [&] {
         for (const fake::Fill &f : fake::fills())
-            if (f.bytes == 64 * 2 * sizeof(double) * bins) return true;
+            if (f.bytes == 64 * 2 * sizeof(double) * ((bins + 15) & ~(size_t)15)) return true;   // in whole lines
         return false;
     };
     WANT(run(70000) == MC_OK && cleared());
