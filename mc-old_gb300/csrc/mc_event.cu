@@ -239,6 +239,7 @@ struct EvLaunch {
     uint32_t max_events = kMaxEvents;
     int refill = 1;         // k_track: idle lanes a warp gathers before it starts histories
     bool smem_sums = false; // the CTA's tally sums live in shared memory (else in replicas, EvArgs::n_rep)
+    bool rows_shared = false;   // and history rows fold into them (else only a history's first bin does)
     size_t smem = 0;
 };
 
@@ -258,12 +259,17 @@ struct EvLaunch {
 // 0.40, 200,000 0.10 / 0.13; with 30 groups 1.19 / 1.67, 0.31 / 0.39 and 0.12 /
 // 0.12 ms).  Currents alone touch few bins, and gain little (deep slab by
 // groups on every plane, 5,000,000 histories 1.01 / 1.04 ms, 200,000 0.105 /
-// 0.096).
+// 0.096).  Sums that the rows leave alone are worth their shared memory up to
+// kWideSums bins, 16 KB a CTA: from there on they displace CTAs and L1, and the
+// first bin goes to the replicas too (1,000,000 histories, in shared memory /
+// replicas: 432 bins 4.5 / 4.6 ms, 732 0.549 / 0.556, 918 1.58 / 1.53, 1205 1.05 /
+// 1.00, 1983 1.75 / 1.35, 2765 4.54 / 3.26, 3302 1.33 / 1.01).
 constexpr uint64_t kReplicaHistories = 65536, kReplicaHistoriesMg = 1 << 18;
+constexpr long long kWideSums = 1024;
 
 static mc_status event_launch_shape(const DeviceProblem &d, const mc_tune *tune, const mc_tune &tuned,
                                     long long nb, uint64_t n, bool batch, int flavor, int comb_teeth,
-                                    Residency &R, EvLaunch &L, std::string &err)
+                                    bool cell_rows, Residency &R, EvLaunch &L, std::string &err)
 {
     L.flavor = flavor;
     // measured at 2 / 4 / 8: shield 63.7 / 61.8 / 62.3 ms, deep slab 11.9 /
@@ -349,7 +355,9 @@ static mc_status event_launch_shape(const DeviceProblem &d, const mc_tune *tune,
         L.ovf_cap = kTrackBlock * depth;
         // the per-CTA sums, then (multigroup, with them) every thread's
         // running sums of its register bin and that bin
-        L.smem_sums = nb > 0 && nb <= 4096 && (fl_lane_bin(flavor) || n < kReplicaHistories);
+        const bool row_replicas = fl_lane_bin(flavor) ? cell_rows && n >= kReplicaHistoriesMg : n >= kReplicaHistories;
+        L.smem_sums = nb > 0 && nb <= 4096 && (!row_replicas || (fl_lane_bin(flavor) && nb <= kWideSums));
+        L.rows_shared = L.smem_sums && !row_replicas;
         L.smem = sizeof(double) * 2 * (size_t)(L.smem_sums ? nb : 0) + 64;
         if (L.smem_sums && fl_lane_bin(flavor)) L.smem += kTrackBlock * (2 * sizeof(double) + sizeof(int));
     } else {
@@ -367,7 +375,7 @@ static mc_status event_launch_shape(const DeviceProblem &d, const mc_tune *tune,
             err = "stack_depth (the tile kernel's overflow bank) must be 1..2^20";
             return MC_ERR_ARG;
         }
-        L.smem_sums = nb > 0 && nb <= 4096;
+        L.smem_sums = L.rows_shared = nb > 0 && nb <= 4096;
         L.smem = tile_smem_bytes(L.tile, L.smem_sums ? nb : 0);
     }
     EvKernel k = pick_kernel(L.minb, batch, L.kernel, L.flavor);
@@ -523,7 +531,8 @@ mc_status run_event(const Tables &t, DeviceProblem &d, uint64_t first, uint64_t 
     EvLaunch L;
     const int comb = t.comb_teeth > 0 ? t.comb_teeth : 0;
     const int flavor = flavor_of(V.G > 0, V.G == 0, V.general, V.has_time || comb);
-    mc_status st = event_launch_shape(d, tune, d.tuned, nb, n, false, flavor, comb, S.resident, L, err);
+    mc_status st = event_launch_shape(d, tune, d.tuned, nb, n, false, flavor, comb,
+                                      !t.cell_tl.empty() || !t.cell_c.empty(), S.resident, L, err);
     if (st != MC_OK) return st;
     if (L.kernel == 3) {
         mc_tune bt = tune ? *tune : mc_tune{};
@@ -564,9 +573,7 @@ mc_status run_event(const Tables &t, DeviceProblem &d, uint64_t first, uint64_t 
     A.sq = d.d_sq;
     A.tile = L.tile;
     A.smem_sums = L.smem_sums ? 1 : 0;
-    const bool row_replicas = L.kernel == 2 && fl_lane_bin(L.flavor) && n >= kReplicaHistoriesMg &&
-                              t.cell_tl.size() + t.cell_c.size() > 0;
-    A.rows_shared = L.smem_sums && !row_replicas ? 1 : 0;
+    A.rows_shared = L.rows_shared ? 1 : 0;
     A.refill_min = L.refill;
     A.lanes = track_lanes(L.grid, A.n);
     A.n_prob = 0;
@@ -840,7 +847,8 @@ mc_status batch_run(BatchState *b, int device_sms, uint64_t seed, const mc_tune 
     DeviceProblem shape_dev;
     shape_dev.sms = device_sms;
     EvLaunch L;
-    mc_status st = event_launch_shape(shape_dev, tune, tuned, 0, b->total, true, b->flavor, b->comb_teeth, b->scratch.resident, L, err);
+    mc_status st = event_launch_shape(shape_dev, tune, tuned, 0, b->total, true, b->flavor, b->comb_teeth, false,
+                                      b->scratch.resident, L, err);
     if (st != MC_OK) return st;
     L.max_events = (tune && tune->max_events) ? tune->max_events : kMaxEvents;
     const bool same_shape = b->have_shape && L.grid == b->shape.grid && L.tile == b->shape.tile &&
